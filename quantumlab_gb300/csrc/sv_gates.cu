@@ -13,6 +13,7 @@
 // takes k = 2t, 2t+1 and moves them with double2 loads (kVec).  When the
 // partner bit is bit 0 the pair itself is adjacent (kAdj).  Otherwise kScalar.
 #include "df64.cuh"
+#include "fix64.cuh"
 #include "qg_internal.h"
 
 #include <algorithm>
@@ -63,15 +64,62 @@ struct OpMatrix2 {
     }
 };
 
-// QuEST_gpu.cu:783-844: up' = a.up - conj(b).lo ; lo' = b.up + conj(a).lo
-struct OpCompact {
-    double ar, ai, br, bi;
+// The same update in fixed point on the integer pipes (fix64.cuh): the four
+// reals of a pair under the matrix's real 4 x 4 form.  Pairs whose exponents
+// are out of its range (all zero, among others) take the FP64 arithmetic,
+// (OpFixed2: behind a call: inlined, its few FP64 instructions would be predicated, and
+// a predicated-off instruction still takes its slots of the FP64 pipe).
+//
+// With all warps in fixed point the FP64 pipe (whose conversions end each
+// output) is half idle while the integer pipes bound the kernel, so one warp
+// in kFp64Share works in FP64.  One gate at 26 qubits (targets 0, 3, 25):
+// all in FP64 1024 us, all in fixed point 430, 414, 425; shared at 1 in 7
+// 407, 387, 397 (6: 404, 384, 391; 10: 429, 400, 412).  HBM floor 316; at 20
+// qubits 20 us before, 10.3 now.  A warp of 1 in 7 takes turns on the SM's
+// partitions, as a power of two would not.
+constexpr unsigned kFp64Share = 7;
+__device__ __noinline__ double2 real2Rare(double a, double b, double c, double d, double x, double y) {
+    return make_double2(a * x + b * y, c * x + d * y);
+}
+struct OpFixed4 {
+    fx::Map<4> f;
+    OpMatrix2 exact;
     __device__ __forceinline__ void operator()(double& ur, double& ui, double& lr, double& li) const {
-        const double a = ur, b = ui, c = lr, d = li;
-        ur = ar * a - ai * b - br * c - bi * d;
-        ui = ar * b + ai * a - br * d + bi * c;
-        lr = br * a - bi * b + ar * c + ai * d;
-        li = br * b + bi * a + ar * d - ai * c;
+        double* const x[4] = {&ur, &ui, &lr, &li};
+        const unsigned warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+        if (warp % kFp64Share == 0 || !fx::apply<4>(f, x)) exact(ur, ui, lr, li);
+    }
+};
+// A matrix whose real form couples ur only with lr and ui only with li (a
+// real matrix) or, after lr and li change places (launchPair's `cross`), ur
+// only with li and ui only with lr (rotateX): two real 2 x 2 maps, half the
+// products of the general form.  rotateY at 26 qubits: 1024 us in the general
+// FP64 form, 330, 321, 332 in fixed point (HBM-bound); the same two maps in
+// FP64, for matrices that do not fit, take half the general form's time.
+struct OpDirect2 {
+    double a[2][2], b[2][2];
+    __device__ __forceinline__ void operator()(double& ur, double& ui, double& lr, double& li) const {
+        const double x = ur, y = ui;
+        ur = a[0][0] * x + a[0][1] * lr;
+        lr = a[1][0] * x + a[1][1] * lr;
+        ui = b[0][0] * y + b[0][1] * li;
+        li = b[1][0] * y + b[1][1] * li;
+    }
+};
+__device__ __forceinline__ void fixed2(const fx::Map<2>& f, const double (&m)[2][2], double& x, double& y) {
+    double* const p[2] = {&x, &y};
+    if (!fx::apply<2>(f, p)) {
+        const double2 v = real2Rare(m[0][0], m[0][1], m[1][0], m[1][1], x, y);
+        x = v.x;
+        y = v.y;
+    }
+}
+struct OpFixed2 {
+    fx::Map<2> fa, fb;
+    OpDirect2 exact;
+    __device__ __forceinline__ void operator()(double& ur, double& ui, double& lr, double& li) const {
+        fixed2(fa, exact.a, ur, lr);
+        fixed2(fb, exact.b, ui, li);
     }
 };
 
@@ -106,16 +154,6 @@ OpMatrix2DF matrix2DF(const Mat2& m) {
 // 0: exact FP64 (the default); 1: double-float for the general 2 x 2 gates
 int g_plainArith = 0;
 
-// QuEST_gpu.cu:1771-1826
-struct OpHadamard {
-    double f;
-    __device__ __forceinline__ void operator()(double& ur, double& ui, double& lr, double& li) const {
-        const double a = ur, b = ui, c = lr, d = li;
-        ur = f * (a + c); ui = f * (b + d);
-        lr = f * (a - c); li = f * (b - d);
-    }
-};
-
 struct OpSwap {
     __device__ __forceinline__ void operator()(double& ur, double& ui, double& lr, double& li) const {
         double t = ur; ur = lr; lr = t;
@@ -133,21 +171,23 @@ struct OpPauliY {
     }
 };
 
+// lre, lim: the arrays of the partner's parts; the same as re and im, or im
+// and re when the op couples ur with li and ui with lr (`cross`)
 template <class Op>
-__global__ void __launch_bounds__(kThreads) kPairVec(double* __restrict__ re, double* __restrict__ im, InsSpec ins,
+__global__ void __launch_bounds__(kThreads, 6) kPairVec(double* re, double* im, double* lre, double* lim, InsSpec ins,
                                                      uint64_t setMask, uint64_t pmask, uint64_t nThreads, Op op) {
     const uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (t >= nThreads) return;
     const uint64_t i0 = insertZeros(t << 1, ins) | setMask;
     const uint64_t i1 = i0 ^ pmask;
-    double2 ur = ld2(re + i0), ui = ld2(im + i0), lr = ld2(re + i1), li = ld2(im + i1);
+    double2 ur = ld2(re + i0), ui = ld2(im + i0), lr = ld2(lre + i1), li = ld2(lim + i1);
     op(ur.x, ui.x, lr.x, li.x);
     op(ur.y, ui.y, lr.y, li.y);
-    st2(re + i0, ur); st2(im + i0, ui); st2(re + i1, lr); st2(im + i1, li);
+    st2(re + i0, ur); st2(im + i0, ui); st2(lre + i1, lr); st2(lim + i1, li);
 }
 
 // partner bit is bit 0: (re[i0], re[i0+1]) is one pair; two pairs per thread
-template <class Op>
+template <bool CROSS, class Op>
 __global__ void __launch_bounds__(kThreads) kPairAdj(double* __restrict__ re, double* __restrict__ im, InsSpec ins,
                                                      uint64_t setMask, uint64_t nThreads, Op op) {
     const uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
@@ -155,27 +195,27 @@ __global__ void __launch_bounds__(kThreads) kPairAdj(double* __restrict__ re, do
     const uint64_t a0 = insertZeros(t << 1, ins) | setMask;
     const uint64_t a1 = insertZeros((t << 1) | 1ull, ins) | setMask;
     double2 r0 = ld2(re + a0), i0 = ld2(im + a0), r1 = ld2(re + a1), i1 = ld2(im + a1);
-    op(r0.x, i0.x, r0.y, i0.y);
-    op(r1.x, i1.x, r1.y, i1.y);
+    op(r0.x, i0.x, CROSS ? i0.y : r0.y, CROSS ? r0.y : i0.y);
+    op(r1.x, i1.x, CROSS ? i1.y : r1.y, CROSS ? r1.y : i1.y);
     st2(re + a0, r0); st2(im + a0, i0); st2(re + a1, r1); st2(im + a1, i1);
 }
 
 template <class Op>
-__global__ void __launch_bounds__(kThreads) kPairScalar(double* __restrict__ re, double* __restrict__ im, InsSpec ins,
+__global__ void __launch_bounds__(kThreads) kPairScalar(double* re, double* im, double* lre, double* lim, InsSpec ins,
                                                         uint64_t setMask, uint64_t pmask, uint64_t nPairs, Op op) {
     const uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (t >= nPairs) return;
     const uint64_t i0 = insertZeros(t, ins) | setMask;
     const uint64_t i1 = i0 ^ pmask;
-    double ur = re[i0], ui = im[i0], lr = re[i1], li = im[i1];
+    double ur = re[i0], ui = im[i0], lr = lre[i1], li = lim[i1];
     op(ur, ui, lr, li);
-    re[i0] = ur; im[i0] = ui; re[i1] = lr; im[i1] = li;
+    re[i0] = ur; im[i0] = ui; lre[i1] = lr; lim[i1] = li;
 }
 
 // Launch a pair gate: partner = i0 ^ pmask, lowBit = lowest bit of pmask
 // (inserted as 0 in i0), ctrl bits inserted and set according to setMask.
 template <class Op>
-void launchPair(SV s, uint64_t ctrl, uint64_t setMask, uint64_t pmask, const Op& op, const char* caller) {
+void launchPair(SV s, uint64_t ctrl, uint64_t setMask, uint64_t pmask, const Op& op, const char* caller, bool cross = false) {
     const uint64_t lowBit = pmask & (~pmask + 1ull);
     const uint64_t insMask = ctrl | lowBit;
     const InsSpec ins = makeIns(insMask);
@@ -183,12 +223,15 @@ void launchPair(SV s, uint64_t ctrl, uint64_t setMask, uint64_t pmask, const Op&
     if (free < 0) return;
     const uint64_t nPairs = 1ull << free;
     cudaStream_t st = stream();
+    double* const lre = cross ? s.im : s.re;
+    double* const lim = cross ? s.re : s.im;
     if (nPairs >= 2 && !(insMask & 1ull)) {
-        kPairVec<Op><<<blocksFor(nPairs / 2), kThreads, 0, st>>>(s.re, s.im, ins, setMask, pmask, nPairs / 2, op);
+        kPairVec<Op><<<blocksFor(nPairs / 2), kThreads, 0, st>>>(s.re, s.im, lre, lim, ins, setMask, pmask, nPairs / 2, op);
     } else if (nPairs >= 2 && pmask == 1ull) {
-        kPairAdj<Op><<<blocksFor(nPairs / 2), kThreads, 0, st>>>(s.re, s.im, ins, setMask, nPairs / 2, op);
+        if (cross) kPairAdj<true, Op><<<blocksFor(nPairs / 2), kThreads, 0, st>>>(s.re, s.im, ins, setMask, nPairs / 2, op);
+        else kPairAdj<false, Op><<<blocksFor(nPairs / 2), kThreads, 0, st>>>(s.re, s.im, ins, setMask, nPairs / 2, op);
     } else {
-        kPairScalar<Op><<<blocksFor(nPairs), kThreads, 0, st>>>(s.re, s.im, ins, setMask, pmask, nPairs, op);
+        kPairScalar<Op><<<blocksFor(nPairs), kThreads, 0, st>>>(s.re, s.im, lre, lim, ins, setMask, pmask, nPairs, op);
     }
     launchFailed(caller);
 }
@@ -355,43 +398,75 @@ size_t g_matCap = 0;
 }  // namespace
 
 // --------------------------------------------------------------- launchers
+// The plain path of every general 2 x 2 gate.
+static void launchMatrix2(SV s, uint64_t ctrl, uint64_t setMask, uint64_t pmask, const Mat2& u, const char* caller) {
+    if (g_plainArith == 1) {
+        launchPair(s, ctrl, setMask, pmask, matrix2DF(u), caller);
+        return;
+    }
+    const OpMatrix2 exact{u};
+    // the real form, rows and columns in the order (ur, ui, lr, li)
+    double r[4][4];
+    for (int i = 0; i < 2; ++i)
+        for (int j = 0; j < 2; ++j) {
+            r[2 * i][2 * j] = r[2 * i + 1][2 * j + 1] = u.r[i][j];
+            r[2 * i][2 * j + 1] = -u.i[i][j];
+            r[2 * i + 1][2 * j] = u.i[i][j];
+        }
+    OpFixed4 f4;
+    f4.exact = exact;
+    if (fx::mapFits<4>(r, f4.f)) {
+        launchPair(s, ctrl, setMask, pmask, f4, caller);
+        return;
+    }
+    // two real 2 x 2 maps: ur with lr (or li), ui with li (or lr)
+    for (int cross = 0; cross < 2; ++cross) {
+        const int a[2] = {0, cross ? 3 : 2}, b[2] = {1, cross ? 2 : 3};
+        bool apart = true;
+        for (int i = 0; i < 2; ++i)
+            for (int j = 0; j < 2; ++j) apart = apart && r[a[i]][b[j]] == 0 && r[b[i]][a[j]] == 0;
+        if (!apart) continue;
+        OpFixed2 f2;
+        for (int i = 0; i < 2; ++i)
+            for (int j = 0; j < 2; ++j) {
+                f2.exact.a[i][j] = r[a[i]][a[j]];
+                f2.exact.b[i][j] = r[b[i]][b[j]];
+            }
+        if (fx::mapFits<2>(f2.exact.a, f2.fa) && fx::mapFits<2>(f2.exact.b, f2.fb))
+            launchPair(s, ctrl, setMask, pmask, f2, caller, cross);
+        else
+            launchPair(s, ctrl, setMask, pmask, f2.exact, caller, cross);
+        return;
+    }
+    launchPair(s, ctrl, setMask, pmask, exact, caller);
+}
+
 void gateMatrix2(SV s, int target, uint64_t ctrl, uint64_t flip, const Mat2& u) {   // QuEST_gpu.cu:966, 1231, 1299
     if (s.cap) {
         const double ur[4] = {u.r[0][0], u.r[0][1], u.r[1][0], u.r[1][1]}, ui[4] = {u.i[0][0], u.i[0][1], u.i[1][0], u.i[1][1]};
         if (capturePair(s, target, ctrl, flip, ur, ui)) return;
     }
-    if (g_plainArith == 1) launchPair(s, ctrl, ctrl & ~flip, 1ull << target, matrix2DF(u), "unitary");
-    else launchPair(s, ctrl, ctrl & ~flip, 1ull << target, OpMatrix2{u}, "unitary");
+    launchMatrix2(s, ctrl, ctrl & ~flip, 1ull << target, u, "unitary");
 }
 
+// QuEST_gpu.cu:783-844: up' = a.up - conj(b).lo ; lo' = b.up + conj(a).lo
 void gateCompact(SV s, int target, uint64_t ctrl, double ar, double ai, double br, double bi) {   // QuEST_gpu.cu:838, 905
     if (s.cap) {
         const double ur[4] = {ar, -br, br, ar}, ui[4] = {ai, bi, bi, -ai};     // [alpha, -conj(beta); beta, conj(alpha)]
         if (capturePair(s, target, ctrl, 0, ur, ui)) return;
     }
-    if (g_plainArith == 1) {
-        Mat2 m;                                            // [alpha, -conj(beta); beta, conj(alpha)]
-        m.r[0][0] = ar; m.i[0][0] = ai; m.r[0][1] = -br; m.i[0][1] = bi;
-        m.r[1][0] = br; m.i[1][0] = bi; m.r[1][1] = ar; m.i[1][1] = -ai;
-        launchPair(s, ctrl, ctrl, 1ull << target, matrix2DF(m), "compactUnitary");
-        return;
-    }
-    launchPair(s, ctrl, ctrl, 1ull << target, OpCompact{ar, ai, br, bi}, "compactUnitary");
+    const Mat2 m{{{ar, -br}, {br, ar}}, {{ai, bi}, {bi, -ai}}};
+    launchMatrix2(s, ctrl, ctrl, 1ull << target, m, "compactUnitary");
 }
 
-void gateHadamard(SV s, int target) {                                                // QuEST_gpu.cu:1820
+void gateHadamard(SV s, int target) {                                                // QuEST_gpu.cu:1771-1826
+    const double f = 0.70710678118654752440;
     if (s.cap) {
-        const double f = 0.70710678118654752440;
         const double ur[4] = {f, f, f, -f}, ui[4] = {0, 0, 0, 0};
         if (capturePair(s, target, 0, 0, ur, ui)) return;
     }
-    if (g_plainArith == 1) {
-        const double f = 0.70710678118654752440;
-        Mat2 m{{{f, f}, {f, -f}}, {{0, 0}, {0, 0}}};
-        launchPair(s, 0, 0, 1ull << target, matrix2DF(m), "hadamard");
-        return;
-    }
-    launchPair(s, 0, 0, 1ull << target, OpHadamard{0.70710678118654752440}, "hadamard");
+    const Mat2 m{{{f, f}, {f, -f}}, {{0, 0}, {0, 0}}};
+    launchMatrix2(s, 0, 0, 1ull << target, m, "hadamard");
 }
 
 bool setPlainArithmetic(int mode) {
