@@ -229,8 +229,8 @@ void* quest_gb300_swapTestBatchCreate(const double* vectors, const long long* of
                                       int numVectors, const int* idxA, const int* idxB, int numTests);
 int quest_gb300_swapTestBatchRun(void* batch, double* p0Out);
 /* Autotune the batch's kernel: time every pairing of CTAs per SM (2, 3, 4)
- * and shared-memory threshold (states of up to 2^9, 2^11 or 2^13 amplitudes
- * kept in shared memory, larger ones in a global arena), keep the fastest and
+ * and size threshold (states of up to 2^9, 2^11 or 2^13 amplitudes are taken
+ * by one warp each, larger ones by a whole CTA), keep the fastest and
  * capture the graph again with it.  Writes the choice, its time per run and
  * the default's (4 CTAs per SM, 2^13) in ms; returns 0 or -1. */
 int quest_gb300_swapTestBatchTune(void* batch, int* ctasPerSM, int* smemAmps, double* msBest, double* msDefault);

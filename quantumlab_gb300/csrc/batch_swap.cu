@@ -7,24 +7,34 @@
 // Circuit of one test (u, v of length 2^d, qubits: u = 0..d-1, v = d..2d-1,
 // ancilla = 2d):   |0>|v>|u>  ->  H(anc)  ->  prod_i CSWAP(anc; u_i, v_i)
 //                  ->  H(anc)  ->  P(anc = 0).
-// The engine simulates it on an explicit FP32 state vector of 2^(2d+1)
-// amplitudes, with two fused passes:
-//   pass A = state preparation + H(anc): phi(x, a, b) = u_a v_b / sqrt2 for
-//            both ancilla values (a = u-register index, b = v-register index);
-//   pass B = the d controlled swaps (they share the control and commute, so
-//            together they exchange the u and v registers on the anc = 1
-//            half: chi(1, a, b) = phi(1, b, a)) + H(anc) + the probability
-//            P0 = sum_{a,b} |(chi(0,a,b) + chi(1,a,b)) / sqrt2|^2.
-// Small states (2^(2d+1) <= kSmemAmps) live in shared memory; larger ones in
-// a per-CTA slice of a global arena: pass A writes it with 16-byte stores,
-// and in pass B each warp takes 32 x 32 (a, b) tiles, reading the swapped
-// half row by row (coalesced) and transposing it through its own
-// shared-memory tile, so no block-wide barrier is needed inside the pass.
-// Amplitudes are FP32; |omega|^2 terms are summed in FP32 within a thread's
-// share of a tile (at most 32 terms) and in FP64 above that.
+// The engine forms every amplitude of the anc = 0 half of the final state in
+// registers and squares it: preparation + H(anc) gives phi(x, a, b) =
+// u_a v_b / sqrt2 for both ancilla values (a = u-register index, b =
+// v-register index); the d controlled swaps share the control and commute, so
+// together they exchange the registers on the anc = 1 half, chi(1, a, b) =
+// phi(1, b, a); H(anc) makes the amplitude omega(a, b) = (chi(0, a, b) +
+// chi(1, a, b)) / sqrt2 = (u_a v_b + u_b v_a) / 2, and P(anc = 0) =
+// sum_{a,b} |omega|^2.  (The powers of two are applied to the sum.)
 //
-// Scheduling: tests are sorted by size (largest first) and CTAs take the
-// next one from a global ticket (atomicAdd), so uneven sizes balance.
+// Nothing is stored between the gates: a state of 2^(2d+1) amplitudes written
+// to and read back from device memory is what bounded an earlier form of this
+// kernel (6.1 TB/s; 65,536 tests of d = 4..10 took 33.3 ms).  In registers an
+// amplitude costs three FP32 operations (packed in twos) and a share of a
+// shared-memory read, and the FP32 pipes bound it: 16,384 tests of d = 4..10
+// 8.33 -> 0.24 ms, of which the FP32 operations take 0.16.  omega is symmetric, so above d = 6 the
+// amplitudes with a and b in different blocks of 128 are formed once and
+// counted twice.
+//
+// A lane owns NB values of b (u_b, v_b twice in a packed register each) and
+// walks a four at a time, reading u_a, v_a as two broadcast 16-byte words;
+// |omega|^2 is summed in FP32 over at most 8 terms per packed half and
+// accumulator, the accumulators pairwise, and in FP64 above a unit of 16
+// values of a.
+//
+// Scheduling: tests are sorted by size (largest first) and CTAs take the next
+// item from a global ticket (atomicAdd), so uneven sizes balance.  An item is
+// one test for the whole CTA (its units dealt to the warps) or, for small
+// tests, one test per warp.
 #include "qg_internal.h"
 #include "quest_gb300.h"
 
@@ -39,11 +49,10 @@ namespace {
 
 constexpr int kSwapThreads = 256;
 constexpr int kSwapCtasPerSM = 4;        // the most CTAs per SM (launch bounds); the default
-constexpr int kAreaFloats = (kSwapThreads / 32) * 32 * 33;   // 8 transpose tiles (33.8 KB)
-constexpr int kSmemAmps = 8192;          // default: pass A/B in shared memory up to 2^13 amplitudes (d <= 6)
-static_assert(kSmemAmps <= kAreaFloats, "a small state must fit the tile area");
+constexpr int kSmemAmps = 8192;          // default: a warp each for states of up to 2^13 amplitudes (d <= 6)
+constexpr int kBlock = 128;              // values of b that a warp's lanes own together
+constexpr int kUnit = 16;                // values of a per unit of work
 constexpr int kMaxD = 10;
-constexpr double kInvSqrt2 = 0.70710678118654752440;
 
 struct SwapJob {
     long long offA, offB;    // offsets of u and v in the vector pool
@@ -64,92 +73,155 @@ __device__ double blockSum(double v, double* red) {
     return t;
 }
 
+// two FP32 values in one register pair, and their packed operations
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float x, float y) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float sum2(f32x2 a) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(a));
+    return x + y;
+}
+
+// sum of (u_a v_b + u_b v_a)^2 over a = a0, a0 + 4 step, ... (count groups of
+// four consecutive a, at most kUnit / 4) and the lane's NB values of b
+template <int NB>
+__device__ __forceinline__ float unitSum(const float* su, const float* sv, int a0, int count, int step,
+                                         const f32x2 (&ub)[NB], const f32x2 (&vb)[NB]) {
+    f32x2 acc[NB];
+#pragma unroll
+    for (int k = 0; k < NB; ++k) acc[k] = 0ull;
+    for (int i = 0; i < count; ++i) {
+        const ulonglong2 u = *reinterpret_cast<const ulonglong2*>(su + a0 + 4 * i * step);
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(sv + a0 + 4 * i * step);
+#pragma unroll
+        for (int k = 0; k < NB; ++k) {
+            const f32x2 x = fma2(u.x, vb[k], mul2(ub[k], v.x)), y = fma2(u.y, vb[k], mul2(ub[k], v.y));
+            acc[k] = fma2(y, y, fma2(x, x, acc[k]));
+        }
+    }
+    float s[NB];
+#pragma unroll
+    for (int k = 0; k < NB; ++k) s[k] = sum2(acc[k]);
+#pragma unroll
+    for (int w = NB / 2; w > 0; w /= 2)
+#pragma unroll
+        for (int k = 0; k < w; ++k) s[k] += s[k + w];
+    return s[0];
+}
+
+// the lane's values b0 + lane + 32 k
+template <int NB>
+__device__ __forceinline__ void loadB(const float* su, const float* sv, int b, f32x2 (&ub)[NB], f32x2 (&vb)[NB]) {
+#pragma unroll
+    for (int k = 0; k < NB; ++k) {
+        ub[k] = pack2(su[b + 32 * k], su[b + 32 * k]);
+        vb[k] = pack2(sv[b + 32 * k], sv[b + 32 * k]);
+    }
+}
+
+// Units first, first + stride, ... of one test by one warp (D = 2^d values of
+// a and b in su, sv); this lane's share of sum_{a,b} (u_a v_b + u_b v_a)^2.
+template <int NB>
+__device__ double squareUnits(const float* su, const float* sv, int D, int first, int stride, int lane) {
+    f32x2 ub[NB], vb[NB];
+    loadB<NB>(su, sv, lane, ub, vb);
+    double total = 0.0;
+    for (int a0 = first * kUnit; a0 < D; a0 += stride * kUnit) total += (double)unitSum<NB>(su, sv, a0, kUnit / 4, 1, ub, vb);
+    return total;
+}
+__device__ __noinline__ double testUnits(const float* su, const float* sv, int d, int first, int stride, int lane) {
+    const int D = 1 << d;
+    if (d > 6) {
+        // block j of b: the a below it in units counted twice, then the a of
+        // the block itself; units are numbered through all blocks
+        constexpr int kPerBlock = kBlock / kUnit, NB = kBlock / 32;
+        f32x2 ub[NB], vb[NB];
+        double total = 0.0;
+        int unit = first, base = 0;                       // base: units of the blocks before j
+        for (int j = 0; j < D / kBlock; ++j) {
+            const int units = kPerBlock * (j + 1);
+            if (unit < base + units) loadB<NB>(su, sv, j * kBlock + lane, ub, vb);
+            for (; unit < base + units; unit += stride) {
+                const float s = unitSum<NB>(su, sv, (unit - base) * kUnit, kUnit / 4, 1, ub, vb);
+                total += (double)(unit - base < kPerBlock * j ? 2.f * s : s);
+            }
+            base += units;
+        }
+        return total;
+    }
+    if (d == 6) return squareUnits<2>(su, sv, D, first, stride, lane);
+    if (d == 5) return squareUnits<1>(su, sv, D, first, stride, lane);
+    if (first != 0) return 0.0;
+    // D <= 16 values of b: the warp's 32 / D lane groups share the a (four at
+    // a time; for D = 2 the upper half of each four is zero)
+    f32x2 ub[1], vb[1];
+    loadB<1>(su, sv, lane & (D - 1), ub, vb);
+    const int group = lane >> d, groups = 32 >> d;
+    const int fours = D > 4 ? D / 4 : 1;
+    return group < fours ? (double)unitSum<1>(su, sv, 4 * group, (fours - group + groups - 1) / groups, groups, ub, vb) : 0.0;
+}
+
 __global__ void __launch_bounds__(kSwapThreads, kSwapCtasPerSM) kSwapTests(const float* __restrict__ pool,
                                                                            const SwapJob* __restrict__ jobs, int numJobs,
-                                                                           unsigned int* __restrict__ ticket,
-                                                                           float* __restrict__ arena, size_t arenaPerCta,
-                                                                           double* __restrict__ out, int smemAmps) {
+                                                                           int numBig, unsigned int* __restrict__ ticket,
+                                                                           double* __restrict__ out) {
+    constexpr int kWarps = kSwapThreads / 32, kSlice = (1 << kMaxD) / kWarps;   // a warp's own test: d <= 6
+    static_assert(kSlice >= 64, "a warp's test must fit its slice");
     __shared__ __align__(16) float su[1 << kMaxD];
-    __shared__ float sv[1 << kMaxD];
-    // the whole state of a small test, or the warps' 32 x 33 transpose tiles
-    __shared__ __align__(16) float area[kAreaFloats];
-    __shared__ double red[kSwapThreads / 32];
-    __shared__ int sJob;
+    __shared__ __align__(16) float sv[1 << kMaxD];
+    __shared__ double red[kWarps];
+    __shared__ int sItem;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float* myArena = arena + (size_t)blockIdx.x * arenaPerCta;
+    const int numItems = numBig + (numJobs - numBig + kWarps - 1) / kWarps;
     for (;;) {
-        if (threadIdx.x == 0) sJob = (int)atomicAdd(ticket, 1u);
+        if (threadIdx.x == 0) sItem = (int)atomicAdd(ticket, 1u);
         __syncthreads();
-        const int j = sJob;
+        const int item = sItem;
         __syncthreads();
-        if (j >= numJobs) break;
-        const SwapJob job = jobs[j];
-        const int d = job.d;
-        const int D = 1 << d;
-        const uint64_t half = 1ull << (2 * d);          // amplitudes per ancilla value
-        for (int i = threadIdx.x; i < D; i += kSwapThreads) {
-            su[i] = pool[job.offA + i];
-            sv[i] = pool[job.offB + i];
-        }
-        __syncthreads();
-        double total = 0.0;
-        if (2 * half <= (uint64_t)smemAmps) {
-            // ---- small state, in shared memory
-            float* phi = area;
-            for (uint32_t idx = threadIdx.x; idx < half; idx += kSwapThreads) {
-                const float val = su[idx & (D - 1)] * sv[idx >> d] * (float)kInvSqrt2;
-                phi[idx] = val;
-                phi[half + idx] = val;
+        if (item >= numItems) break;
+        if (item < numBig) {
+            const SwapJob job = jobs[item];
+            const int D = 1 << job.d;
+            for (int i = threadIdx.x; i < D; i += kSwapThreads) {
+                su[i] = pool[job.offA + i];
+                sv[i] = pool[job.offB + i];
             }
             __syncthreads();
-            float s = 0.f;
-            for (uint32_t idx = threadIdx.x; idx < half; idx += kSwapThreads) {
-                const uint32_t a = idx & (D - 1), b = idx >> d;
-                const float w = (phi[idx] + phi[half + b + (a << d)]) * (float)kInvSqrt2;
-                s = fmaf(w, w, s);
-            }
-            total = (double)s;
+            const double p = blockSum(testUnits(su, sv, job.d, warp, kWarps, lane), red);
+            if (threadIdx.x == 0) out[job.out] = 0.25 * p;
         } else {
-            // ---- pass A: |0>|v>|u> then H(anc): both halves = u_a v_b / sqrt2,
-            // written as 16-byte vectors (4 consecutive a, one b)
-            float4* phi4 = reinterpret_cast<float4*>(myArena);
-            const uint32_t half4 = (uint32_t)(half >> 2);
-            for (uint32_t i4 = threadIdx.x; i4 < half4; i4 += kSwapThreads) {
-                const uint32_t idx = i4 << 2;
-                const float vb = sv[idx >> d] * (float)kInvSqrt2;
-                const float4 u4 = *reinterpret_cast<const float4*>(su + (idx & (D - 1)));
-                const float4 val = make_float4(u4.x * vb, u4.y * vb, u4.z * vb, u4.w * vb);
-                __stcg(phi4 + i4, val);
-                __stcg(phi4 + half4 + i4, val);
-            }
-            __syncthreads();
-            // ---- pass B: CSWAPs (anc=1 half: u <-> v), H(anc), P(anc = 0),
-            // over 32 x 32 (a, b) tiles, one warp per tile: the swapped half
-            // is read row by row (coalesced) and transposed through the
-            // warp's own shared-memory tile
-            const float* phi = myArena;
-            float(*tile)[33] = reinterpret_cast<float(*)[33]>(area + warp * 32 * 33);
-            const int T = D / 32;
-            for (int t = warp; t < T * T; t += kSwapThreads / 32) {
-                const int a0 = (t % T) * 32, b0 = (t / T) * 32;
-                const float* row1 = phi + half + (uint64_t)(b0 + lane) + ((uint64_t)a0 << d);
-#pragma unroll 8
-                for (int r = 0; r < 32; ++r) tile[r][lane] = __ldcg(row1 + ((uint64_t)r << d));   // phi(1, b0+lane, a0+r)
-                __syncwarp();
-                const float* col0 = phi + (uint64_t)(a0 + lane) + ((uint64_t)b0 << d);
-                float s = 0.f;
-#pragma unroll 8
-                for (int r = 0; r < 32; ++r) {
-                    const float w = (__ldcg(col0 + ((uint64_t)r << d)) + tile[lane][r]) * (float)kInvSqrt2;
-                    s = fmaf(w, w, s);
+            const int j = numBig + (item - numBig) * kWarps + warp;
+            if (j < numJobs) {
+                const SwapJob job = jobs[j];
+                const int D = 1 << job.d;
+                float* const wu = su + warp * kSlice;
+                float* const wv = sv + warp * kSlice;
+                for (int i = lane; i < D || i < 4; i += 32) {
+                    wu[i] = i < D ? pool[job.offA + i] : 0.f;
+                    wv[i] = i < D ? pool[job.offB + i] : 0.f;
                 }
                 __syncwarp();
-                total += (double)s;                      // FP32 within a tile (32 terms), FP64 across tiles
+                double p = testUnits(wu, wv, job.d, 0, 1, lane);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) p += __shfl_down_sync(0xffffffffu, p, o);
+                if (lane == 0) out[job.out] = 0.25 * p;
             }
         }
-        const double p0 = blockSum(total, red);
-        if (threadIdx.x == 0) out[job.out] = p0;
-        __syncthreads();
+        __syncthreads();                                  // su, sv are read no more
     }
 }
 
@@ -158,12 +230,10 @@ struct SwapBatch {
     float* pool = nullptr;
     SwapJob* jobs = nullptr;
     unsigned int* ticket = nullptr;
-    float* arena = nullptr;
-    size_t arenaPerCta = 0;           // floats per CTA of the arena (for up to kSwapCtasPerSM CTAs per SM)
     double* out = nullptr;
-    int maxD = 1;
+    int count[kMaxD + 1] = {};        // tests by d
     int ctasPerSM = kSwapCtasPerSM;   // tunable: 1 .. kSwapCtasPerSM
-    int smemAmps = kSmemAmps;         // tunable: states of at most this many amplitudes stay in shared memory
+    int smemAmps = kSmemAmps;         // tunable: states of at most this many amplitudes take a warp, larger ones a CTA
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     double* hostOut = nullptr;        // pinned
@@ -179,9 +249,11 @@ void dropGraph(SwapBatch* b) {
 // the run's work on `st`: reset the ticket, the persistent kernel, results to
 // pinned host memory
 void queueSwaps(SwapBatch* b, cudaStream_t st) {
+    int numBig = 0;                                       // the jobs are sorted, largest first
+    for (int d = 1; d <= kMaxD; ++d)
+        if (2ll << (2 * d) > b->smemAmps) numBig += b->count[d];
     cudaMemsetAsync(b->ticket, 0, sizeof(unsigned int), st);
-    kSwapTests<<<numSMs() * b->ctasPerSM, kSwapThreads, 0, st>>>(b->pool, b->jobs, b->numTests, b->ticket, b->arena,
-                                                                  b->arenaPerCta, b->out, b->smemAmps);
+    kSwapTests<<<numSMs() * b->ctasPerSM, kSwapThreads, 0, st>>>(b->pool, b->jobs, b->numTests, numBig, b->ticket, b->out);
     cudaMemcpyAsync(b->hostOut, b->out, b->numTests * sizeof(double), cudaMemcpyDeviceToHost, st);
 }
 
@@ -208,7 +280,6 @@ void freeBatch(SwapBatch* b) {
     cudaFree(b->pool);
     cudaFree(b->jobs);
     cudaFree(b->ticket);
-    cudaFree(b->arena);
     cudaFree(b->out);
     cudaFreeHost(b->hostOut);
     delete b;
@@ -238,7 +309,6 @@ void* quest_gb300_swapTestBatchCreate(const double* vectors, const long long* of
         poolLen = std::max(poolLen, offsets[i] + (1ll << dimLog2[i]));
     }
     std::vector<SwapJob> jobs(numTests);
-    int maxD = 1;
     for (int t = 0; t < numTests; ++t) {
         const int a = idxA[t], b = idxB[t];
         if (a < 0 || a >= numVectors || b < 0 || b >= numVectors || dimLog2[a] != dimLog2[b]) {
@@ -246,18 +316,12 @@ void* quest_gb300_swapTestBatchCreate(const double* vectors, const long long* of
             return nullptr;
         }
         jobs[t] = SwapJob{offsets[a], offsets[b], dimLog2[a], t};
-        maxD = std::max(maxD, dimLog2[a]);
     }
     // largest circuits first: dynamic scheduling then balances the tail
     std::stable_sort(jobs.begin(), jobs.end(), [](const SwapJob& x, const SwapJob& y) { return x.d > y.d; });
     SwapBatch* b = new SwapBatch();
     b->numTests = numTests;
-    b->maxD = maxD;
-    // an arena slice per CTA for every state that may leave shared memory
-    // (any state above the smallest tunable threshold)
-    const size_t arenaNeed = (2ull << (2 * maxD)) > 512 ? (2ull << (2 * maxD)) : 0;
-    b->arenaPerCta = arenaNeed;
-    const size_t maxGrid = (size_t)qg::numSMs() * qg::kSwapCtasPerSM;
+    for (const SwapJob& j : jobs) ++b->count[j.d];
     std::vector<float> pool32(poolLen);
     for (long long i = 0; i < poolLen; ++i) pool32[i] = (float)vectors[i];
     cudaStream_t st = qg::stream();
@@ -265,8 +329,7 @@ void* quest_gb300_swapTestBatchCreate(const double* vectors, const long long* of
         QG_CUDA(cudaMalloc(&b->jobs, numTests * sizeof(SwapJob)), fn) ||
         QG_CUDA(cudaMalloc(&b->ticket, sizeof(unsigned int)), fn) ||
         QG_CUDA(cudaMalloc(&b->out, numTests * sizeof(double)), fn) ||
-        QG_CUDA(cudaMallocHost(&b->hostOut, numTests * sizeof(double)), fn) ||
-        (arenaNeed && QG_CUDA(cudaMalloc(&b->arena, arenaNeed * maxGrid * sizeof(float)), fn))) {
+        QG_CUDA(cudaMallocHost(&b->hostOut, numTests * sizeof(double)), fn)) {
         qg::freeBatch(b);
         return nullptr;
     }
@@ -280,9 +343,9 @@ void* quest_gb300_swapTestBatchCreate(const double* vectors, const long long* of
     return b;
 }
 
-// Time the batch with every pairing of CTAs per SM (2, 3, 4) and
-// shared-memory threshold (states of up to 2^9, 2^11 or 2^13 amplitudes stay
-// in shared memory: d <= 4, 5 or 6), two runs each, keep the fastest and
+// Time the batch with every pairing of CTAs per SM (2, 3, 4) and threshold
+// (states of up to 2^9, 2^11 or 2^13 amplitudes, d <= 4, 5 or 6, take a warp
+// each, larger ones a CTA), two runs each, keep the fastest and
 // capture the graph again with it.  Writes the choice, its time and the time
 // of the default (4 CTAs per SM, 2^13) in ms; returns 0 or -1.
 int quest_gb300_swapTestBatchTune(void* batch, int* ctasPerSM, int* smemAmps, double* msBest, double* msDefault) {

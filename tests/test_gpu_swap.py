@@ -98,3 +98,34 @@ def test_swap_batch_tuning_keeps_results(gpulib):
     want = np.array([(1 + np.dot(vecs[a], vecs[b]) ** 2) / 2 for a, b in pairs])
     assert np.max(np.abs(out - want)) < 1e-6
     L.lib.quest_gb300_swapTestBatchDestroy(h)
+
+
+@pytest.mark.parametrize("dims, copies", [((1, 2, 3, 4, 5, 6, 7, 8, 9, 10), 3), ((1,), 5), ((6, 7), 9), ((10,), 2)])
+def test_swap_batch_every_size(gpulib, dims, copies):
+    """Every register size, alone and mixed: partial groups of the small tests
+    that share a CTA, blocks of 128 above and on the diagonal, vectors at odd
+    offsets of the pool.  Bound: inputs, products, their sum and the square
+    rounded to FP32 (2 * 4 half ulps of terms whose squares sum to <= 1), at
+    most 12 more for the FP32 sums: 20 * 2^-24."""
+    L = gpulib
+    rng = np.random.default_rng(17)
+    vecs, offsets, pos = [], [], 1
+    for d in dims:
+        for _ in range(copies):
+            v = rng.normal(size=1 << d)
+            vecs.append(v / np.linalg.norm(v))
+            offsets.append(pos)
+            pos += len(v) + 1
+    pool = np.zeros(pos)
+    for o, v in zip(offsets, vecs):
+        pool[o:o + len(v)] = v
+    dlog = np.array([int(np.log2(len(v))) for v in vecs], dtype=np.int32)
+    pairs = [(a, b) for a in range(len(vecs)) for b in range(len(vecs)) if dlog[a] == dlog[b]]
+    ia = np.array([a for a, _ in pairs], dtype=np.int32)
+    ib = np.array([b for _, b in pairs], dtype=np.int32)
+    h = make_batch(L, pool, np.array(offsets, dtype=np.int64), dlog, ia, ib)
+    out = np.zeros(len(ia))
+    assert L.lib.quest_gb300_swapTestBatchRun(h, out.ctypes.data_as(C.POINTER(C.c_double))) == 0
+    L.lib.quest_gb300_swapTestBatchDestroy(h)
+    want = np.array([(1 + np.dot(vecs[a], vecs[b]) ** 2) / 2 for a, b in pairs])
+    assert np.max(np.abs(out - want)) <= 20 * 2.0 ** -24
