@@ -432,7 +432,7 @@ Qureg allocQureg(int nsv, int isDM, int nrep, const char* caller) {
     }
     double* scratch = nullptr;
     double* slot = nullptr;
-    if (cudaMalloc(&scratch, qg::kScratchDoubles * sizeof(double)) != cudaSuccess ||
+    if (cudaMalloc(&scratch, (qg::kScratchDoubles + qg::kPhaseTableDoubles) * sizeof(double)) != cudaSuccess ||
         cudaMallocHost(&slot, 64 * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
         fail(E_QUREG_NOT_ALLOCATED_ON_GPU, caller);
@@ -1125,28 +1125,28 @@ void multiControlledMultiRotatePauli(Qureg q, int* cs, int nc, int* ts, enum pau
 }
 
 // Trotter (QuEST.c:1079 -> QuEST_common.c:762-844)
-static void expPauliHamil(const Qureg& q, const PauliHamil& h, double fac, int reverse) {
-    int ts[64];
-    for (int i = 0; i < h.numQubits; ++i) ts[i] = i;
-    for (int i = 0; i < h.numSumTerms; ++i) {
-        const int t = reverse ? h.numSumTerms - 1 - i : i;
-        applyPauliRotation(q, 0, ts, h.pauliCodes + (idx_t)t * h.numQubits, h.numQubits, 2 * fac * h.termCoeffs[t]);
+static void expPauliHamil(const std::vector<qg::PauliRotation>& terms, double fac, int reverse,
+                          std::vector<qg::PauliRotation>& out) {
+    for (size_t i = 0; i < terms.size(); ++i) {
+        out.push_back(terms[reverse ? terms.size() - 1 - i : i]);
+        out.back().angle *= 2 * fac;
     }
 }
-static void symTrotter(const Qureg& q, const PauliHamil& h, double time, int order) {
+static void symTrotter(const std::vector<qg::PauliRotation>& terms, double time, int order,
+                       std::vector<qg::PauliRotation>& out) {
     if (order == 1) {
-        expPauliHamil(q, h, time, 0);
+        expPauliHamil(terms, time, 0, out);
     } else if (order == 2) {
-        expPauliHamil(q, h, time / 2., 0);
-        expPauliHamil(q, h, time / 2., 1);
+        expPauliHamil(terms, time / 2., 0, out);
+        expPauliHamil(terms, time / 2., 1, out);
     } else {
         const double p = 1. / (4 - pow(4, 1. / (order - 1)));
         const int lo = order - 2;
-        symTrotter(q, h, p * time, lo);
-        symTrotter(q, h, p * time, lo);
-        symTrotter(q, h, (1 - 4 * p) * time, lo);
-        symTrotter(q, h, p * time, lo);
-        symTrotter(q, h, p * time, lo);
+        symTrotter(terms, p * time, lo, out);
+        symTrotter(terms, p * time, lo, out);
+        symTrotter(terms, (1 - 4 * p) * time, lo, out);
+        symTrotter(terms, p * time, lo, out);
+        symTrotter(terms, p * time, lo, out);
     }
 }
 void applyTrotterCircuit(Qureg q, PauliHamil h, qreal time, int order, int reps) {
@@ -1156,7 +1156,31 @@ void applyTrotterCircuit(Qureg q, PauliHamil h, qreal time, int order, int reps)
     if (!vHamil(h, caller)) return;
     if (!REQUIRE(h.numQubits == q.numQubitsRepresented, E_MISMATCHING_PAULI_HAMIL_QUREG_NUM_QUBITS)) return;
     if (time == 0) return;
-    for (int r = 0; r < reps; ++r) symTrotter(q, h, time / reps, order);
+    // the terms that rotate (identities apply nothing, QuEST_common.c:430-431)
+    std::vector<qg::PauliRotation> terms, seq;
+    std::vector<int> ts(h.numQubits);
+    for (int i = 0; i < h.numQubits; ++i) ts[i] = i;
+    for (int t = 0; t < h.numSumTerms; ++t) {
+        qg::PauliRotation r{0, 0, 0, h.termCoeffs[t], 0};
+        pauliMasks(ts.data(), h.pauliCodes + (idx_t)t * h.numQubits, h.numQubits, &r.x, &r.y, &r.z);
+        if (r.x | r.z) terms.push_back(r);
+    }
+    // The repetitions in runs of some thousand rotations.  A density matrix
+    // gets a run's rotations on its rows, then their conjugates on its
+    // columns: the two act on different qubits.
+    const int s = q.isDensityMatrix ? q.numQubitsRepresented : 0;
+    for (int r = 0; r < reps; ++r) {
+        symTrotter(terms, time / reps, order, seq);
+        if (seq.size() < 4096 && r + 1 < reps) continue;
+        const size_t rows = seq.size();
+        if (q.isDensityMatrix)
+            for (size_t i = 0; i < rows; ++i) {
+                const qg::PauliRotation c = seq[i];
+                seq.push_back(qg::PauliRotation{c.x << s, c.y << s, c.z << s, c.angle, 1});
+            }
+        qg::gatePauliSequence(svg(q), seq, q.firstLevelReduction + qg::kScratchDoubles);
+        seq.clear();
+    }
 }
 
 // ---- measurement (QuEST.c:972-1016, QuEST_common.c:165-180, 361-375) ----

@@ -33,6 +33,9 @@ extern std::atomic<long long> g_launches;
 // Layout (doubles): [partials: 2*kMaxReduceBlocks][result: 64][counter word]
 constexpr int kMaxReduceBlocks = 2048;
 constexpr size_t kScratchDoubles = 2 * kMaxReduceBlocks + 64 + 8;
+// ... and behind it, in a Qureg's, the phase tables of a Pauli rotation
+// sequence (pauli_tile.cu): 4 windows of 2^12 complex factors
+constexpr size_t kPhaseTableDoubles = 4 * 2 * 4096;
 struct Scratch {
     double* partials;          // 2*kMaxReduceBlocks doubles (double2 per block)
     double* result;            // device result slots
@@ -106,6 +109,10 @@ void gateRotateZ(SV s, uint64_t ctrl, uint64_t targ, double angle);
 // exp(-i angle/2 P) with P a Pauli string given by x/y/z masks, where ctrl bits set;
 // conj!=0 applies the elementwise conjugate operator.
 void gatePauliRotation(SV s, uint64_t ctrl, uint64_t xmask, uint64_t ymask, uint64_t zmask, double angle, int conj);
+// the same for a sequence without controls, many rotations per pass
+// (pauli_tile.cu); tables: kPhaseTableDoubles of the register's workspace
+struct PauliRotation { uint64_t x, y, z; double angle; int conj; };
+void gatePauliSequence(SV s, const std::vector<PauliRotation>& seq, double* tables);
 void gateSwap(SV s, int q1, int q2);
 // plain-path arithmetic of the general 2 x 2 gates: 0 FP64, 1 double-float
 bool setPlainArithmetic(int mode);
