@@ -220,8 +220,7 @@ static void flushRecord(Capture* c, double* re, double* im) {
         quest_gb300_planDestroy(plan);
     } else {
         // keep the searched plan as the shape of the next flushes
-        if (plan->device && plan->deviceFree) plan->deviceFree(plan->device);
-        plan->device = nullptr;
+        releaseDevice(*plan);
         plan->passes.clear();
         if (c->shape) quest_gb300_planDestroy(c->shape);
         c->shape = plan;

@@ -9,6 +9,7 @@
 // in fused_tc.cu.  Norms, probabilities and the comparison against an FP64
 // register accumulate in FP64.
 #include "fused_plan.h"
+#include "fused_small.h"
 #include "quest_gb300.h"
 #include "reduce_kernel.cuh"
 
@@ -59,6 +60,7 @@ int tcCheckImageLayouts();
 void tcRoundHalf(const double* v, uint16_t* out, int count);
 int tcCheckHalfImages();
 bool tensorCoresEnabled();
+bool tcDefaultAppliers();
 int tcKernelFor(const FusedPass& pass, int n);
 float* f32re(QuregF32& q) { return q.re; }
 float* f32im(QuregF32& q) { return q.im; }
@@ -510,6 +512,24 @@ static int applyRange(void* h, void* plan, int firstPass, int numPasses, const d
         invalidQuESTInputError("The fusion plan could not be compiled.", "applyPlanF32");
         return -1;
     }
+    const int total = (int)p->passes.size();
+    if (firstPass < 0 || numPasses < 0 || firstPass > total) {
+        invalidQuESTInputError("Pass range outside the plan.", "applyPlanF32");
+        return -1;
+    }
+    const int last = std::min(total, firstPass + numPasses);
+    if (!g_passEvents && qg::smallPlanFits(*p)) {
+        if (!p->small) {
+            p->small = qg::smallPlanUpload(*p);
+            p->smallFree = qg::smallPlanFree;
+        }
+        if (p->small) {
+            qg::tcBeginPlan(p->device, p->passes.size());     // no tensor-core pass of this plan came last
+            const int e = qg::smallPlanApply(p->small, q->re, q->im, firstPass, last);
+            if (e > 0) invalidQuESTInputError("fused passes: timed out on the barrier between passes", "applyPlanF32");
+            return e ? -1 : 0;
+        }
+    }
     if (p->device && !qg::tcImagesFit(p->device)) {      // built for another precision or kernel
         p->deviceFree(p->device);
         p->device = nullptr;
@@ -518,12 +538,6 @@ static int applyRange(void* h, void* plan, int firstPass, int numPasses, const d
         p->device = qg::uploadPlanTC(*p);
         p->deviceFree = qg::freePlanTC;
     }
-    const int total = (int)p->passes.size();
-    if (firstPass < 0 || numPasses < 0 || firstPass > total) {
-        invalidQuESTInputError("Pass range outside the plan.", "applyPlanF32");
-        return -1;
-    }
-    const int last = std::min(total, firstPass + numPasses);
     cudaStream_t st = qg::stream();
     if (firstPass == 0) qg::tcBeginPlan(p->device, p->passes.size());
     qg::tcBeginRange(p->device, entryBound);

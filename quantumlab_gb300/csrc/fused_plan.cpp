@@ -636,7 +636,7 @@ void* quest_gb300_planCreate(int numQubits, int maxFusedQubits) {
 void quest_gb300_planDestroy(void* plan) {
     FusedPlan* p = P(plan);
     if (!p) return;
-    if (p->device && p->deviceFree) p->deviceFree(p->device);
+    qg::releaseDevice(*p);
     delete p;
 }
 
@@ -713,8 +713,7 @@ int quest_gb300_planPassControls(void* plan, int i, int* controls) {
 int quest_gb300_planCompile(void* plan) {
     FusedPlan* p = P(plan);
     if (!p) return -1;
-    if (p->device && p->deviceFree) p->deviceFree(p->device);
-    p->device = nullptr;
+    qg::releaseDevice(*p);
     qg::compilePlan(*p);
     return p->compiled ? (int)p->passes.size() : -1;
 }
@@ -723,8 +722,7 @@ int quest_gb300_planCompileLike(void* plan, void* structure) {
     FusedPlan* p = P(plan);
     const FusedPlan* s = P(structure);
     if (!p || !s || p == s) return -1;
-    if (p->device && p->deviceFree) p->deviceFree(p->device);
-    p->device = nullptr;
+    qg::releaseDevice(*p);
     return qg::compilePlanLike(*p, *s) ? (int)p->passes.size() : -1;
 }
 

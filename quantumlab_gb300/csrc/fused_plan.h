@@ -52,7 +52,16 @@ struct FusedPlan {
     // first use by the FP32 engine; owned by the engine
     void* device = nullptr;
     void (*deviceFree)(void*) = nullptr;
+    // the same for a small register: the plan as one launch (fused_small.cu)
+    void* small = nullptr;
+    void (*smallFree)(void*) = nullptr;
 };
+// give the device copies back (the passes are about to change)
+inline void releaseDevice(FusedPlan& p) {
+    if (p.device && p.deviceFree) p.deviceFree(p.device);
+    if (p.small && p.smallFree) p.smallFree(p.small);
+    p.device = p.small = nullptr;
+}
 
 // Widest pass the FP32 appliers take on registers of n qubits: six qubits
 // need the tensor-core applier (n >= 13: a tile is 2^(6+7) amplitudes), the

@@ -2089,6 +2089,9 @@ bool setTensorCoreStaging(int mode) {
 int tensorCoreStaging() { return g_tcStaging; }
 void setTensorCoreKernel(int version) { g_tcVersion = (version >= 1 && version <= 5) ? version : 0; }
 bool tensorCoresEnabled() { return g_tcEnabled; }
+// the appliers are the library's choice, and in an FP32 form that refuses no
+// state (split-FP16 reports amplitudes out of its range)
+bool tcDefaultAppliers() { return g_tcEnabled && g_tcVersion == 0 && g_tcTrial == 0 && g_tcPrecision != kPrecF16; }
 
 // One pass on `batch` registers of n qubits: register b's planes start
 // b * 2^n floats into re and im, and its operand image imageStride floats

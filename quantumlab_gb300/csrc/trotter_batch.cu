@@ -18,7 +18,11 @@
 //   * each pass is one launch of the tensor-core applier over all the class's
 //     states (the CTAs are shared out among the states, each state's CTAs
 //     load that state's operands); passes narrower than 4 qubits are widened
-//     with identity factors so that every pass runs on the tensor cores;
+//     with identity factors so that every pass runs on the tensor cores.
+//     Classes of small states (2^19 amplitudes at most) run side by side
+//     instead, all their passes in one launch (fused_small.cu): nine 16-qubit
+//     instances in three classes took 3.79 ms one class after the other,
+//     2.26 ms side by side;
 //   * the energies <H_b> are reduced from the FP32 states (FP32 products per
 //     amplitude pair, FP64 sums), one launch per term group over the class's
 //     states, divided by each state's norm, which also removes the norm drift
@@ -27,6 +31,7 @@
 //     passes and reductions, and the copy of the results to pinned host
 //     memory) is one CUDA graph that later runs replay.
 #include "fused_plan.h"
+#include "fused_small.h"
 #include "qg_internal.h"
 #include "quest_gb300.h"
 #include "reduce_kernel.cuh"
@@ -45,6 +50,7 @@ namespace qg {
 size_t tcImageFloats(int k, int parts);
 void tcBuildImage(const FusedPass& pass, float* img, int parts);
 int tcImageParts();
+bool tcDefaultAppliers();
 bool applyPassTCBatch(float* re, float* im, int n, const FusedPass& pass, const float* images, size_t imageStride,
                       int parts, int batch, int* errFlag, cudaStream_t st);
 
@@ -345,6 +351,8 @@ struct TrotterBatch {
     std::vector<Instance> inst;
     bool compiled = false;
     int parts = 0;                                 // operand image parts built (tcImageParts)
+    bool oneLaunch = false;                        // all passes as one program instead
+    SmallProgram small;
     std::vector<TrotterClass> classes;
     std::vector<int> classOf, posOf;               // per instance: its class, its place in it
     float *re = nullptr, *im = nullptr;            // every class's states, class after class
@@ -372,6 +380,9 @@ void freeDevice(TrotterBatch* b) {
     for (void* p : {(void*)b->re, (void*)b->im, (void*)b->images, (void*)b->dInit, (void*)b->dCoef, (void*)b->dResults})
         if (p) cudaFree(p);
     if (b->hResults) cudaFreeHost(b->hResults);
+    smallFree(b->small);
+    b->small = SmallProgram();
+    b->oneLaunch = false;
     b->re = b->im = nullptr;
     b->images = nullptr;
     b->dInit = nullptr;
@@ -605,6 +616,15 @@ bool compileBatch(TrotterBatch* b) {
     size_t stateFloats = 0, imgTotal = 0;
     // the operand image parts the current precision and kernel choice read
     b->parts = tcImageParts();
+    // one program for all classes where each is small (the passes of the
+    // others, and split-FP16's, are launched one by one)
+    b->oneLaunch = tcDefaultAppliers() && C <= kSmallMaxSegs;
+    for (int c = 0; c < C; ++c) {
+        const TrotterClass& cl = b->classes[c];
+        b->oneLaunch = b->oneLaunch && ((uint64_t)cl.members.size() << cl.n) <= 1ull << kSmallMaxQubits;
+        for (const FusedPass& pass : planOf(c, 0).passes)
+            b->oneLaunch = b->oneLaunch && pass.controls.empty() && smallFits(cl.n, pass.targets);
+    }
     int pos = 0, slots = 0;
     std::vector<float> coef;                       // [class][reduction][member][kCoefs]
     for (int c = 0; c < C; ++c) {
@@ -622,7 +642,7 @@ bool compileBatch(TrotterBatch* b) {
             cl.shape.push_back(widenNarrow(planOf(c, 0).passes[p], cl.n));
             cl.imgStride[p] = tcImageFloats((int)cl.shape[p].targets.size(), b->parts);
             cl.imgOffset[p] = imgTotal;
-            imgTotal += cl.imgStride[p] * M;
+            if (!b->oneLaunch) imgTotal += cl.imgStride[p] * M;
         }
         cl.slotBase = slots;
         cl.coefOffset = coef.size();
@@ -630,7 +650,31 @@ bool compileBatch(TrotterBatch* b) {
         slots += (int)(cl.reds.size() * M);
     }
     b->numSlots = slots;
-    // operand images of every (class, pass, member), on host threads
+    // operand images of every (class, pass, member), on host threads; in one
+    // program step p holds pass p of every class that has one
+    std::vector<std::vector<size_t>> matOf(C);     // per class and pass: member 0's matrix
+    if (b->oneLaunch) {
+        size_t steps = 0;
+        uint64_t amps = 0;                         // over all steps
+        for (int c = 0; c < C; ++c) {
+            const TrotterClass& cl = b->classes[c];
+            steps = std::max(steps, cl.shape.size());
+            amps += ((uint64_t)cl.members.size() << cl.n) * cl.shape.size();
+            matOf[c].resize(cl.shape.size());
+        }
+        b->small.groups = smallGroups(amps / std::max<size_t>(steps, 1));
+        b->small.first.push_back(0);
+        for (size_t p = 0; p < steps; ++p) {
+            for (int c = 0; c < C; ++c) {
+                const TrotterClass& cl = b->classes[c];
+                if (p >= cl.shape.size()) continue;
+                matOf[c][p] = imgTotal;
+                imgTotal = smallAddPass(b->small, planOf(c, 0).passes[p], cl.n, cl.stateOffset, (int)cl.members.size(), imgTotal);
+            }
+            b->small.first.push_back((int)b->small.segs.size());
+        }
+        b->oneLaunch = steps > 0;
+    }
     std::vector<float> host(std::max<size_t>(imgTotal, 4));
     std::vector<std::tuple<int, int, int>> imgJobs;            // class, pass, member
     for (int c = 0; c < C; ++c)
@@ -639,6 +683,10 @@ bool compileBatch(TrotterBatch* b) {
     parallelFor(imgJobs.size(), std::min(hw, 16u), [&](size_t j) {
         const int c = std::get<0>(imgJobs[j]), p = std::get<1>(imgJobs[j]), m = std::get<2>(imgJobs[j]);
         const TrotterClass& cl = b->classes[c];
+        if (b->oneLaunch) {
+            smallMatrix(planOf(c, m).passes[p], cl.n, host.data() + matOf[c][p] + m * kSmallMatrixFloats);
+            return;
+        }
         tcBuildImage(widenNarrow(planOf(c, m).passes[p], cl.n), host.data() + cl.imgOffset[p] + m * cl.imgStride[p],
                      b->parts);
     });
@@ -648,14 +696,15 @@ bool compileBatch(TrotterBatch* b) {
     for (int k = 0; k < B; ++k) init[b->classes[b->classOf[k]].posBase + b->posOf[k]] = b->inst[k].init;
     if (QG_CUDA(cudaMalloc(&b->re, stateFloats * sizeof(float)), kFn) ||
         QG_CUDA(cudaMalloc(&b->im, stateFloats * sizeof(float)), kFn) ||
-        QG_CUDA(cudaMalloc(&b->images, host.size() * sizeof(float)), kFn) ||
+        (b->oneLaunch ? !smallUpload(b->small, host.data(), imgTotal, kFn)
+                      : QG_CUDA(cudaMalloc(&b->images, host.size() * sizeof(float)), kFn) ||
+                            QG_CUDA(cudaMemcpyAsync(b->images, host.data(), host.size() * sizeof(float), cudaMemcpyHostToDevice, st), kFn)) ||
         QG_CUDA(cudaMalloc(&b->dInit, B * sizeof(long long)), kFn) ||
         QG_CUDA(cudaMalloc(&b->dCoef, std::max<size_t>(1, coef.size()) * sizeof(float)), kFn) ||
         QG_CUDA(cudaMalloc(&b->dResults, 2 * (size_t)b->numSlots * sizeof(double)), kFn) ||
         QG_CUDA(cudaMallocHost(&b->hResults, 2 * (size_t)b->numSlots * sizeof(double)), kFn))
         return false;
-    if (QG_CUDA(cudaMemcpyAsync(b->images, host.data(), host.size() * sizeof(float), cudaMemcpyHostToDevice, st), kFn) ||
-        QG_CUDA(cudaMemcpyAsync(b->dInit, init.data(), B * sizeof(long long), cudaMemcpyHostToDevice, st), kFn) ||
+    if (QG_CUDA(cudaMemcpyAsync(b->dInit, init.data(), B * sizeof(long long), cudaMemcpyHostToDevice, st), kFn) ||
         QG_CUDA(cudaMemcpyAsync(b->dCoef, coef.data(), coef.size() * sizeof(float), cudaMemcpyHostToDevice, st), kFn) ||
         QG_CUDA(cudaStreamSynchronize(st), kFn))
         return false;
@@ -664,9 +713,10 @@ bool compileBatch(TrotterBatch* b) {
 }
 
 // the run's work, queued on `st` (the library stream, or a capture stream):
-// class after class, its states' initialisation, its passes (one launch each
-// over the class's states) and its reductions (one launch each over the
-// class's states), then one copy of every result to pinned host memory
+// class after class, its states' initialisation and its passes (one launch each
+// over the class's states, or one launch for all passes of all classes), then
+// its reductions (one launch each over the class's states), then one copy of
+// every result to pinned host memory
 bool queueRun(TrotterBatch* b, cudaStream_t st) {
     if (QG_CUDA(cudaMemsetAsync(b->errFlag, 0, sizeof(int), st), kFn)) return false;
     for (const TrotterClass& cl : b->classes) {
@@ -679,12 +729,21 @@ bool queueRun(TrotterBatch* b, cudaStream_t st) {
             return false;
         kBatchClassical<<<(M + 127) / 128, 128, 0, st>>>(re, dim, b->dInit + cl.posBase, M);
         if (launchFailed(kFn)) return false;
-        for (size_t p = 0; p < cl.shape.size(); ++p)
+        for (size_t p = 0; p < cl.shape.size() && !b->oneLaunch; ++p)
             if (!applyPassTCBatch(re, im, cl.n, cl.shape[p], b->images + cl.imgOffset[p], cl.imgStride[p], b->parts, M,
                                   b->errFlag, st)) {
                 invalidQuESTInputError("A pass of the Trotter batch could not be launched on the tensor cores.", kFn);
                 return false;
             }
+    }
+    if (b->oneLaunch &&
+        !smallLaunch(b->small, b->re, b->im, 0, (int)b->small.first.size() - 1, b->errFlag, st, kFn))
+        return false;
+    for (const TrotterClass& cl : b->classes) {
+        const int M = (int)cl.members.size();
+        const uint64_t dim = 1ull << cl.n;
+        const float* re = b->re + cl.stateOffset;
+        const float* im = b->im + cl.stateOffset;
         double* partials = b->partials + (size_t)cl.posBase * kMaxBlocksPerInst;
         unsigned int* counters = b->counters + cl.posBase;
         for (size_t l = 0; l < cl.reds.size(); ++l) {
@@ -834,7 +893,7 @@ int quest_gb300_trotterBatchRun(void* batch, double* energies) {
     TrotterBatch* b = reinterpret_cast<TrotterBatch*>(batch);
     if (!b) return -1;
     // images built for another precision or kernel choice are rebuilt
-    if (b->compiled && (qg::tcImageParts() & ~b->parts) != 0) {
+    if (b->compiled && (((qg::tcImageParts() & ~b->parts) != 0 && !b->oneLaunch) || (b->oneLaunch && !qg::tcDefaultAppliers()))) {
         cudaStreamSynchronize(qg::stream());
         qg::freeDevice(b);
     }
@@ -853,6 +912,7 @@ int quest_gb300_trotterBatchRun(void* batch, double* energies) {
     int err = 0;
     if (QG_CUDA(cudaMemcpy(&err, b->errFlag, sizeof(int), cudaMemcpyDeviceToHost), fn)) return -1;
     if (err) {
+        if (b->oneLaunch) qg::smallReset(b->small);
         invalidQuESTInputError(err == 6 ? "A split-FP16 tensor-core pass of the Trotter batch gave a non-finite output."
                                         : "A tensor-core pass of the Trotter batch timed out waiting on its pipeline.",
                                fn);
