@@ -237,9 +237,12 @@ void launchPair(SV s, uint64_t ctrl, uint64_t setMask, uint64_t pmask, const Op&
 }
 
 // ------------------------------------------------------- elementwise (diagonal)
+// An op is told the parity of idx & targ, which is linear in idx: a kernel
+// works it out once for amplitudes idx, idx + 1.
 struct OpPhase {           // amp *= t
     double tr, ti;
-    __device__ __forceinline__ void operator()(uint64_t, double& r, double& i) const {
+    __device__ __forceinline__ int odd(uint64_t) const { return 0; }
+    __device__ __forceinline__ void operator()(int, double& r, double& i) const {
         const double a = r, b = i;
         r = tr * a - ti * b;
         i = ti * a + tr * b;
@@ -250,11 +253,53 @@ struct OpPhase {           // amp *= t
 struct OpRotZ {
     uint64_t targ;
     double c, s;
-    __device__ __forceinline__ void operator()(uint64_t idx, double& r, double& i) const {
-        const double fs = (__popcll(idx & targ) & 1) ? 1.0 : -1.0;
+    __device__ __forceinline__ int odd(uint64_t idx) const { return __popcll(idx & targ) & 1; }
+    __device__ __forceinline__ void operator()(int one, double& r, double& i) const {
+        const double fs = one ? 1.0 : -1.0;
         const double a = r, b = i;
         r = c * a - fs * s * b;
         i = fs * s * a + c * b;
+    }
+};
+
+// diag(a, d) on a qubit
+struct OpDiag2 {
+    uint64_t targ;
+    double ar, ai, dr, di;
+    __device__ __forceinline__ int odd(uint64_t idx) const { return (idx & targ) != 0; }
+    __device__ __forceinline__ void operator()(int one, double& r, double& i) const {
+        const double tr = one ? dr : ar, ti = one ? di : ai, x = r, y = i;
+        r = tr * x - ti * y;
+        i = ti * x + tr * y;
+    }
+};
+
+// OpRotZ in fixed point (fix64.cuh): [c s; -s c] on (re, im), its inverse for
+// odd parity (the map between two changes of the imaginary part's sign).  Four
+// FP64 operations an amplitude leave HBM half idle; the fixed-point map has
+// two (the conversions at its end), but keeps the integer pipes 76 % busy, so
+// one warp in kTurnFp64Share works in FP64.  rotateZ at 26 qubits (HBM floor
+// 316 us): as a general matrix 1023 us, all in fixed point 362, one warp in 3,
+// 4, 5, 7 in FP64 330, 317, 334, 346.  phaseShift there (floor 158) 203 all in
+// fixed point, 168 so; controlledPhaseShift on a quarter of the amplitudes
+// (floor 79) 133 in FP64, 107-121.
+constexpr unsigned kTurnFp64Share = 4;
+struct OpTurnFixed {
+    uint64_t targ;
+    fx::Map<2> f;
+    double m[2][2];
+    __device__ __forceinline__ int odd(uint64_t idx) const { return __popcll(idx & targ) & 1; }
+    __device__ __forceinline__ void operator()(int one, double& r, double& i) const {
+        const int sign = one << 31;
+        double v = __hiloint2double(__double2hiint(i) ^ sign, __double2loint(i));
+        const unsigned warp = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
+        double* const x[2] = {&r, &v};
+        if (warp % kTurnFp64Share == 0 || !fx::apply<2>(f, x)) {
+            const double2 w = real2Rare(m[0][0], m[0][1], m[1][0], m[1][1], r, v);
+            r = w.x;
+            v = w.y;
+        }
+        i = __hiloint2double(__double2hiint(v) ^ sign, __double2loint(v));
     }
 };
 
@@ -265,8 +310,9 @@ __global__ void __launch_bounds__(kThreads) kDiagVec(double* __restrict__ re, do
     if (t >= nThreads) return;
     const uint64_t i0 = insertZeros(t << 1, ins) | setMask;
     double2 r = ld2(re + i0), m = ld2(im + i0);
-    op(i0, r.x, m.x);
-    op(i0 + 1, r.y, m.y);
+    const int one = op.odd(i0);
+    op(one, r.x, m.x);
+    op(one ^ op.odd(1), r.y, m.y);
     st2(re + i0, r); st2(im + i0, m);
 }
 
@@ -277,7 +323,7 @@ __global__ void __launch_bounds__(kThreads) kDiagScalar(double* __restrict__ re,
     if (t >= nAmps) return;
     const uint64_t i = insertZeros(t, ins) | setMask;
     double r = re[i], m = im[i];
-    op(i, r, m);
+    op(op.odd(i), r, m);
     re[i] = r; im[i] = m;
 }
 
@@ -293,6 +339,15 @@ void launchDiag(SV s, uint64_t fixedMask, uint64_t setMask, const Op& op, const 
     else
         kDiagScalar<Op><<<blocksFor(nAmps), kThreads, 0, st>>>(s.re, s.im, ins, setMask, nAmps, op);
     launchFailed(caller);
+}
+
+// amp *= c - i s where idx & targ has even parity, c + i s where it has odd:
+// in fixed point unless c or s is small, else in FP64
+template <class Op>
+void launchTurn(SV s, uint64_t fixedMask, uint64_t setMask, uint64_t targ, double c, double sn, const Op& exact, const char* caller) {
+    OpTurnFixed f{targ, {}, {{c, sn}, {-sn, c}}};
+    if (fx::mapFits<2>(f.m, f.f)) launchDiag(s, fixedMask, setMask, f, caller);
+    else launchDiag(s, fixedMask, setMask, exact, caller);
 }
 
 // ------------------------------------------------------- Pauli-string rotation
@@ -404,6 +459,14 @@ static void launchMatrix2(SV s, uint64_t ctrl, uint64_t setMask, uint64_t pmask,
         launchPair(s, ctrl, setMask, pmask, matrix2DF(u), caller);
         return;
     }
+    // a diagonal matrix (rotateZ, controlledRotateZ) pairs no amplitudes: 120
+    // us at 23 qubits as a general one, 45 so
+    if (u.r[0][1] == 0 && u.i[0][1] == 0 && u.r[1][0] == 0 && u.i[1][0] == 0) {
+        const OpDiag2 d{pmask, u.r[0][0], u.i[0][0], u.r[1][1], u.i[1][1]};
+        if (d.dr == d.ar && d.di == -d.ai) launchTurn(s, ctrl, setMask, pmask, d.ar, -d.ai, d, caller);
+        else launchDiag(s, ctrl, setMask, d, caller);
+        return;
+    }
     const OpMatrix2 exact{u};
     // the real form, rows and columns in the order (ur, ui, lr, li)
     double r[4][4];
@@ -491,12 +554,13 @@ void gatePauliY(SV s, int target, uint64_t ctrl, double conjFac) {              
 
 void gatePhase(SV s, uint64_t mask, double tr, double ti) {                          // QuEST_gpu.cu:1485, 1521, 1552, 1702
     if (s.cap && capturePhase(s, mask, tr, ti)) return;
-    launchDiag(s, mask, mask, OpPhase{tr, ti}, "phaseShift");
+    launchTurn(s, mask, mask, 0, tr, -ti, OpPhase{tr, ti}, "phaseShift");
 }
 
 void gateRotateZ(SV s, uint64_t ctrl, uint64_t targ, double angle) {                 // QuEST_gpu.cu:1582, 1615
     if (s.cap && captureRotateZ(s, ctrl, targ, angle)) return;
-    launchDiag(s, ctrl, ctrl, OpRotZ{targ, cos(angle / 2), sin(angle / 2)}, "multiRotateZ");
+    const double c = cos(angle / 2), sn = sin(angle / 2);
+    launchTurn(s, ctrl, ctrl, targ, c, sn, OpRotZ{targ, c, sn}, "multiRotateZ");
 }
 
 void gatePauliRotation(SV s, uint64_t ctrl, uint64_t xmask, uint64_t ymask, uint64_t zmask, double angle, int conj) {
