@@ -19,6 +19,7 @@
 //     exp(-i sum +-phi) and an amplitude takes the product of its entries.
 // Second-order step of an 11-site Fermi-Hubbard chain (22 qubits, 146
 // rotations): 8.17 ms one launch a term, 0.64 ms here in 5 passes.
+#include "chain_launch.cuh"
 #include "qg_internal.h"
 
 #include <algorithm>
@@ -76,6 +77,7 @@ struct TableSpec {
 // Tables (1 + grow) exp(-i sum_k (-1)^popc(index & mask_k) phi_k); the sum is
 // compensated (TwoSum), so an entry is as good as one sincos of the exact sum.
 __global__ void __launch_bounds__(kThreads) kPhaseTables(const __grid_constant__ TableSpec ts, double2* __restrict__ tab) {
+    chainStart();
     const int w = blockIdx.y;
     const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= 1u << ts.bits[w]) return;
@@ -119,6 +121,7 @@ __global__ void __launch_bounds__(kThreads) kPauliTile(double* __restrict__ re, 
         for (int k = kLow; k < b; ++k) a |= (uint64_t)((h >> (k - kLow)) & 1u) << p.pos[k];
         high[h] = a;
     }
+    chainStart();
     __syncthreads();
     for (uint32_t l = 2 * threadIdx.x; l < size; l += 2 * kThreads) {
         const uint64_t a = high[l >> kLow] | (l & ((1u << kLow) - 1u));
@@ -550,11 +553,11 @@ void gatePauliSequence(SV s, const std::vector<PauliRotation>& seq, double* tabl
         if (ts.numWindows) {
             int bits = 0;
             for (int w = 0; w < ts.numWindows; ++w) bits = std::max(bits, ts.bits[w]);
-            kPhaseTables<<<dim3(((1u << bits) + kThreads - 1) / kThreads, ts.numWindows), kThreads, 0, st>>>(
-                ts, reinterpret_cast<double2*>(tables));
+            chain(kPhaseTables, dim3(((1u << bits) + kThreads - 1) / kThreads, ts.numWindows), kThreads, 0, st, ts,
+                  reinterpret_cast<double2*>(tables));
             if (launchFailed(caller)) return;
         }
-        kPauliTile<<<(unsigned)(1ull << (s.n - b)), kThreads, smem, st>>>(s.re, s.im, p, reinterpret_cast<const double2*>(tables));
+        chain(kPauliTile, (unsigned)(1ull << (s.n - b)), kThreads, smem, st, s.re, s.im, p, reinterpret_cast<const double2*>(tables));
         if (launchFailed(caller)) return;
     }
 }

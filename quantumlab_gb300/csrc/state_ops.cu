@@ -7,6 +7,7 @@
 // each channel is one pass over groups of the four entries
 // {rho[.0..0.], rho[.0..1.], rho[.1..0.], rho[.1..1.]} (row bit t, column bit
 // t+N), with the same per-entry arithmetic.
+#include "chain_launch.cuh"
 #include "qg_internal.h"
 
 #include <type_traits>
@@ -193,6 +194,7 @@ __global__ void __launch_bounds__(kThreads) kChannelVec(double* __restrict__ re,
     if (k >= nThreads) return;
     const uint64_t rb = 1ull << t, cb = 1ull << (t + N);
     const uint64_t b = ins2(k << 1, t, t + N);
+    chainStart();
     double2 r00 = ld2(re + b), i00 = ld2(im + b);
     double2 r01 = ld2(re + (b | rb)), i01 = ld2(im + (b | rb));
     double2 r10 = ld2(re + (b | cb)), i10 = ld2(im + (b | cb));
@@ -213,6 +215,7 @@ __global__ void __launch_bounds__(kThreads) kChannelT0(double* __restrict__ re, 
     if (k >= nGroups) return;
     const uint64_t cb = 1ull << N;
     const uint64_t b = ins2(k, 0, N);
+    chainStart();
     double2 rA = ld2(re + b), iA = ld2(im + b), rB = ld2(re + (b | cb)), iB = ld2(im + (b | cb));
     op(rA.x, iA.x, rA.y, iA.y, rB.x, iB.x, rB.y, iB.y);
     st2(re + b, rA); st2(im + b, iA); st2(re + (b | cb), rB); st2(im + (b | cb), iB);
@@ -222,9 +225,9 @@ template <class Op>
 void launchChannel(SV s, int t, int N, const Op& op, const char* caller) {
     const uint64_t nGroups = 1ull << (s.n - 2);
     if (t >= 1 && nGroups >= 2)
-        kChannelVec<Op><<<blocksFor(nGroups / 2), kThreads, 0, stream()>>>(s.re, s.im, t, N, nGroups / 2, op);
+        chain(kChannelVec<Op>, blocksFor(nGroups / 2), kThreads, 0, stream(), s.re, s.im, t, N, nGroups / 2, op);
     else
-        kChannelT0<Op><<<blocksFor(nGroups), kThreads, 0, stream()>>>(s.re, s.im, N, nGroups, op);
+        chain(kChannelT0<Op>, blocksFor(nGroups), kThreads, 0, stream(), s.re, s.im, N, nGroups, op);
     launchFailed(caller);
 }
 
@@ -256,6 +259,7 @@ __global__ void __launch_bounds__(kThreads) kTwoQubitChannel(double* __restrict_
         for (int i = 0; i < 4; ++i) o |= (uint64_t)((j >> i) & 1) << tb.b[i];
         return o;
     };
+    chainStart();
     if (MIX) {
         const int dj[4] = {0, 5, 10, 15};
         vec r[4], m[4];
@@ -307,10 +311,10 @@ void launchTwoQubitChannel(SV s, int q1, int q2, int N, double retain, double di
     const TwoQubitBits tb{{q1, q2, q1 + N, q2 + N}};
     const uint64_t nGroups = 1ull << (s.n - 4);
     if (q1 >= 1)
-        kTwoQubitChannel<2, MIX><<<blocksFor(nGroups / 2), kThreads, 0, stream()>>>(s.re, s.im, tb, nGroups / 2,
+        chain(kTwoQubitChannel<2, MIX>, blocksFor(nGroups / 2), kThreads, 0, stream(), s.re, s.im, tb, nGroups / 2,
                                                                                   retain, diagRetain, mix);
     else
-        kTwoQubitChannel<1, MIX><<<blocksFor(nGroups), kThreads, 0, stream()>>>(s.re, s.im, tb, nGroups, retain,
+        chain(kTwoQubitChannel<1, MIX>, blocksFor(nGroups), kThreads, 0, stream(), s.re, s.im, tb, nGroups, retain,
                                                                                diagRetain, mix);
     launchFailed(caller);
 }

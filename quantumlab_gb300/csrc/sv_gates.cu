@@ -12,6 +12,7 @@
 // inserted bit is bit 0, consecutive k give consecutive i0, so one thread
 // takes k = 2t, 2t+1 and moves them with double2 loads (kVec).  When the
 // partner bit is bit 0 the pair itself is adjacent (kAdj).  Otherwise kScalar.
+#include "chain_launch.cuh"
 #include "df64.cuh"
 #include "fix64.cuh"
 #include "qg_internal.h"
@@ -180,6 +181,7 @@ __global__ void __launch_bounds__(kThreads, 6) kPairVec(double* re, double* im, 
     if (t >= nThreads) return;
     const uint64_t i0 = insertZeros(t << 1, ins) | setMask;
     const uint64_t i1 = i0 ^ pmask;
+    chainStart();
     double2 ur = ld2(re + i0), ui = ld2(im + i0), lr = ld2(lre + i1), li = ld2(lim + i1);
     op(ur.x, ui.x, lr.x, li.x);
     op(ur.y, ui.y, lr.y, li.y);
@@ -194,6 +196,7 @@ __global__ void __launch_bounds__(kThreads) kPairAdj(double* __restrict__ re, do
     if (t >= nThreads) return;
     const uint64_t a0 = insertZeros(t << 1, ins) | setMask;
     const uint64_t a1 = insertZeros((t << 1) | 1ull, ins) | setMask;
+    chainStart();
     double2 r0 = ld2(re + a0), i0 = ld2(im + a0), r1 = ld2(re + a1), i1 = ld2(im + a1);
     op(r0.x, i0.x, CROSS ? i0.y : r0.y, CROSS ? r0.y : i0.y);
     op(r1.x, i1.x, CROSS ? i1.y : r1.y, CROSS ? r1.y : i1.y);
@@ -207,6 +210,7 @@ __global__ void __launch_bounds__(kThreads) kPairScalar(double* re, double* im, 
     if (t >= nPairs) return;
     const uint64_t i0 = insertZeros(t, ins) | setMask;
     const uint64_t i1 = i0 ^ pmask;
+    chainStart();
     double ur = re[i0], ui = im[i0], lr = lre[i1], li = lim[i1];
     op(ur, ui, lr, li);
     re[i0] = ur; im[i0] = ui; lre[i1] = lr; lim[i1] = li;
@@ -226,12 +230,12 @@ void launchPair(SV s, uint64_t ctrl, uint64_t setMask, uint64_t pmask, const Op&
     double* const lre = cross ? s.im : s.re;
     double* const lim = cross ? s.re : s.im;
     if (nPairs >= 2 && !(insMask & 1ull)) {
-        kPairVec<Op><<<blocksFor(nPairs / 2), kThreads, 0, st>>>(s.re, s.im, lre, lim, ins, setMask, pmask, nPairs / 2, op);
+        chain(kPairVec<Op>, blocksFor(nPairs / 2), kThreads, 0, st, s.re, s.im, lre, lim, ins, setMask, pmask, nPairs / 2, op);
     } else if (nPairs >= 2 && pmask == 1ull) {
-        if (cross) kPairAdj<true, Op><<<blocksFor(nPairs / 2), kThreads, 0, st>>>(s.re, s.im, ins, setMask, nPairs / 2, op);
-        else kPairAdj<false, Op><<<blocksFor(nPairs / 2), kThreads, 0, st>>>(s.re, s.im, ins, setMask, nPairs / 2, op);
+        if (cross) chain(kPairAdj<true, Op>, blocksFor(nPairs / 2), kThreads, 0, st, s.re, s.im, ins, setMask, nPairs / 2, op);
+        else chain(kPairAdj<false, Op>, blocksFor(nPairs / 2), kThreads, 0, st, s.re, s.im, ins, setMask, nPairs / 2, op);
     } else {
-        kPairScalar<Op><<<blocksFor(nPairs), kThreads, 0, st>>>(s.re, s.im, lre, lim, ins, setMask, pmask, nPairs, op);
+        chain(kPairScalar<Op>, blocksFor(nPairs), kThreads, 0, st, s.re, s.im, lre, lim, ins, setMask, pmask, nPairs, op);
     }
     launchFailed(caller);
 }
@@ -309,6 +313,7 @@ __global__ void __launch_bounds__(kThreads) kDiagVec(double* __restrict__ re, do
     const uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (t >= nThreads) return;
     const uint64_t i0 = insertZeros(t << 1, ins) | setMask;
+    chainStart();
     double2 r = ld2(re + i0), m = ld2(im + i0);
     const int one = op.odd(i0);
     op(one, r.x, m.x);
@@ -322,6 +327,7 @@ __global__ void __launch_bounds__(kThreads) kDiagScalar(double* __restrict__ re,
     const uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (t >= nAmps) return;
     const uint64_t i = insertZeros(t, ins) | setMask;
+    chainStart();
     double r = re[i], m = im[i];
     op(op.odd(i), r, m);
     re[i] = r; im[i] = m;
@@ -335,9 +341,9 @@ void launchDiag(SV s, uint64_t fixedMask, uint64_t setMask, const Op& op, const 
     const uint64_t nAmps = 1ull << free;
     cudaStream_t st = stream();
     if (nAmps >= 2 && !(fixedMask & 1ull))
-        kDiagVec<Op><<<blocksFor(nAmps / 2), kThreads, 0, st>>>(s.re, s.im, ins, setMask, nAmps / 2, op);
+        chain(kDiagVec<Op>, blocksFor(nAmps / 2), kThreads, 0, st, s.re, s.im, ins, setMask, nAmps / 2, op);
     else
-        kDiagScalar<Op><<<blocksFor(nAmps), kThreads, 0, st>>>(s.re, s.im, ins, setMask, nAmps, op);
+        chain(kDiagScalar<Op>, blocksFor(nAmps), kThreads, 0, st, s.re, s.im, ins, setMask, nAmps, op);
     launchFailed(caller);
 }
 
@@ -378,6 +384,7 @@ __global__ void __launch_bounds__(kThreads) kPauliRotVec(double* __restrict__ re
     if (t >= nThreads) return;
     const uint64_t j0 = insertZeros(t << 1, ins) | setMask;
     const uint64_t k0 = j0 ^ p.xmask;
+    chainStart();
     double2 jr = ld2(re + j0), ji = ld2(im + j0), kr = ld2(re + k0), ki = ld2(im + k0);
     pauliPair(p, j0, jr.x, ji.x, kr.x, ki.x);
     pauliPair(p, j0 + 1, jr.y, ji.y, kr.y, ki.y);
@@ -390,6 +397,7 @@ __global__ void __launch_bounds__(kThreads) kPauliRotScalar(double* __restrict__
     if (t >= nPairs) return;
     const uint64_t j = insertZeros(t, ins) | setMask;
     const uint64_t k = j ^ p.xmask;
+    chainStart();
     double jr = re[j], ji = im[j], kr = re[k], ki = im[k];
     pauliPair(p, j, jr, ji, kr, ki);
     re[j] = jr; im[j] = ji; re[k] = kr; im[k] = ki;
@@ -402,6 +410,7 @@ __global__ void __launch_bounds__(kThreads) kSwap(double* __restrict__ re, doubl
     if (t >= n) return;
     const uint64_t base = insertZeros(t, ins);
     const uint64_t a = base | b1, b = base | b2;
+    chainStart();
     const double r = re[a], m = im[a];
     re[a] = re[b]; im[a] = im[b];
     re[b] = r; im[b] = m;
@@ -588,9 +597,9 @@ void gatePauliRotation(SV s, uint64_t ctrl, uint64_t xmask, uint64_t ymask, uint
     const uint64_t nPairs = 1ull << free;
     cudaStream_t st = stream();
     if (nPairs >= 2 && !(insMask & 1ull) && !(xmask & 1ull))
-        kPauliRotVec<<<blocksFor(nPairs / 2), kThreads, 0, st>>>(s.re, s.im, ins, ctrl, nPairs / 2, p);
+        chain(kPauliRotVec, blocksFor(nPairs / 2), kThreads, 0, st, s.re, s.im, ins, ctrl, nPairs / 2, p);
     else
-        kPauliRotScalar<<<blocksFor(nPairs), kThreads, 0, st>>>(s.re, s.im, ins, ctrl, nPairs, p);
+        chain(kPauliRotScalar, blocksFor(nPairs), kThreads, 0, st, s.re, s.im, ins, ctrl, nPairs, p);
     launchFailed("multiRotatePauli");
 }
 
@@ -598,7 +607,7 @@ void gateSwap(SV s, int q1, int q2) {
     if (s.cap && captureSwap(s, q1, q2)) return;
     const InsSpec ins = makeIns((1ull << q1) | (1ull << q2));
     const uint64_t n = 1ull << (s.n - 2);
-    kSwap<<<blocksFor(n), kThreads, 0, stream()>>>(s.re, s.im, ins, 1ull << q1, 1ull << q2, n);
+    chain(kSwap, blocksFor(n), kThreads, 0, stream(), s.re, s.im, ins, 1ull << q1, 1ull << q2, n);
     launchFailed("swapGate");
 }
 
