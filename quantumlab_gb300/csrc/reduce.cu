@@ -10,6 +10,8 @@
 // ticket counter in the register's scratch) adds the per-block partials in a
 // fixed order.  The partial layout depends only on the problem size, so
 // results are deterministic run to run.  One scalar pair is copied back.
+#include "fixed_sum.cuh"
+#include "pauli_expec.h"
 #include "reduce_kernel.cuh"
 
 #include <algorithm>
@@ -20,11 +22,28 @@ namespace {
 using namespace red;
 
 // ------------------------------------------------------------------ functors
-struct NormSq2 {          // two consecutive amplitudes per item
+// Sums of squares, four amplitudes an item on the integer pipes (fixed_sum.cuh).
+// First amplitudes of the pairs i, i + 1 and j, j + 1.
+struct Squares {
     const double *re, *im;
-    __device__ __forceinline__ double2 operator()(uint64_t i) const {
-        const double2 r = ld2(re + 2 * i), m = ld2(im + 2 * i);
-        return make_double2(r.x * r.x + m.x * m.x + r.y * r.y + m.y * m.y, 0.0);
+    __device__ __forceinline__ double pairs(double acc, uint64_t i, uint64_t j) const {
+        return fsum::addSquares(acc, ld2(re + i), ld2(re + j), ld2(im + i), ld2(im + j));
+    }
+};
+struct NormSq4 : Squares {
+    __device__ __forceinline__ double operator()(double acc, uint64_t k) const { return pairs(acc, 4 * k, 4 * k + 2); }
+};
+struct ProbZero4 : Squares {       // target >= 1: the amplitudes with bit t clear
+    int t;
+    __device__ __forceinline__ double operator()(double acc, uint64_t k) const {
+        return pairs(acc, ins0(4 * k, t), ins0(4 * k + 2, t));
+    }
+};
+struct ProbZeroEven : Squares {    // target 0
+    __device__ __forceinline__ double operator()(double acc, uint64_t k) const {
+        const double *r = re + 8 * k, *m = im + 8 * k;
+        const double2 a = ld2(r), b = ld2(r + 2), c = ld2(r + 4), d = ld2(r + 6), e = ld2(m), f = ld2(m + 2), g = ld2(m + 4), h = ld2(m + 6);
+        return fsum::addSquares(acc, make_double2(a.x, b.x), make_double2(c.x, d.x), make_double2(e.x, f.x), make_double2(g.x, h.x));
     }
 };
 struct NormSq1 {
@@ -39,20 +58,12 @@ struct DiagSum {          // sum of Re rho_rr
     uint64_t step;        // D + 1
     __device__ __forceinline__ double2 operator()(uint64_t r) const { return make_double2(re[r * step], 0.0); }
 };
-struct ProbZeroVec {      // target >= 1: amps i with bit t = 0, two per item
+struct ProbZeroFew {      // registers of one or two qubits
     const double *re, *im;
     int t;
     __device__ __forceinline__ double2 operator()(uint64_t k) const {
-        const uint64_t i = ins0(2 * k, t);
-        const double2 r = ld2(re + i), m = ld2(im + i);
-        return make_double2(r.x * r.x + m.x * m.x + r.y * r.y + m.y * m.y, 0.0);
-    }
-};
-struct ProbZeroT0 {       // target 0: even amps
-    const double *re, *im;
-    __device__ __forceinline__ double2 operator()(uint64_t k) const {
-        const double2 r = ld2(re + 2 * k), m = ld2(im + 2 * k);
-        return make_double2(r.x * r.x + m.x * m.x, 0.0);
+        const uint64_t i = ins0(k, t);
+        return make_double2(re[i] * re[i] + im[i] * im[i], 0.0);
     }
 };
 struct ProbZeroDiag {     // diagonal entries rho_rr with bit t of r = 0
@@ -61,11 +72,32 @@ struct ProbZeroDiag {     // diagonal entries rho_rr with bit t of r = 0
     int t;
     __device__ __forceinline__ double2 operator()(uint64_t k) const { return make_double2(re[ins0(k, t) * step], 0.0); }
 };
-struct Inner2 {           // sum conj(bra) ket, two amps per item
+// sum conj(bra) ket, two amplitudes an item on the integer pipes
+__device__ __noinline__ double2 innerFp64(double2 a, double2 b, double2 c, double2 d) {
+    return make_double2(a.x * c.x + b.x * d.x + a.y * c.y + b.y * d.y, a.x * d.x - b.x * c.x + a.y * d.y - b.y * c.y);
+}
+struct Inner2 {
     const double *br, *bi, *kr, *ki;
-    __device__ __forceinline__ double2 operator()(uint64_t i) const {
+    __device__ __forceinline__ double2 operator()(double2 acc, uint64_t i) const {
         const double2 a = ld2(br + 2 * i), b = ld2(bi + 2 * i), c = ld2(kr + 2 * i), d = ld2(ki + 2 * i);
-        return make_double2(a.x * c.x + b.x * d.x + a.y * c.y + b.y * d.y, a.x * d.x - b.x * c.x + a.y * d.y - b.y * c.y);
+        using namespace fsum;
+        const uint32_t wb = max(max(magnitude(a.x), magnitude(a.y)), max(magnitude(b.x), magnitude(b.y)));
+        const uint32_t wk = max(max(magnitude(c.x), magnitude(c.y)), max(magnitude(d.x), magnitude(d.y)));
+        const int E = (int)(wb >> 20), F = (int)(wk >> 20);
+        // (a zero factor adds nothing, unless the other is infinite or NaN)
+        if ((wb == 0 && allZero(a, b) && F < 0x7FF) || (wk == 0 && allZero(c, d) && E < 0x7FF)) return acc;
+        if (!unitFits(E, F)) {
+            const double2 v = innerFp64(a, b, c, d);
+            return make_double2(acc.x + v.x, acc.y + v.y);
+        }
+        const int2 ax = digits(a.x, E), ay = digits(a.y, E), bx = digits(b.x, E), by = digits(b.y, E);
+        const int2 cx = digits(c.x, F), cy = digits(c.y, F), dx = digits(d.x, F), dy = digits(d.y, F);
+        const int2 nx = make_int2(-bx.x, -bx.y), ny = make_int2(-by.x, -by.y);
+        Sums r{0, 0, 0}, m{0, 0, 0};
+        r.add(ax, cx); r.add(bx, dx); r.add(ay, cy); r.add(by, dy);
+        m.add(ax, dx); m.add(nx, cx); m.add(ay, dy); m.add(ny, cy);
+        const double u = unit(E, F);
+        return make_double2(fma(u, r.few(), acc.x), fma(u, m.few(), acc.y));
     }
 };
 struct Inner1 {
@@ -106,11 +138,8 @@ struct FidelityDM {
 //     2 c_q s_q(j) (+-Re w or +-Im w) when tau_q fits the phase, else 0.  An
 //     item costs wr A(j) + wi B(j) with A, B = sums of +-c over the terms;
 //   * DM, Tr(P rho) = sum_r s(r) Re((-i)^ph rho[r ^ x, r]) = er A(r) + ei B(r);
-//   * a diagonal group (x = 0, SV): an item is 8 consecutive amplitudes.  A
-//     Walsh-Hadamard transform of their |psi|^2 over the 3 low bits gives
-//     Q[m] = sum_l p_l (-1)^popc(l & m); each term then adds
-//     c (-1)^popc(base & z_high) Q[z & 7].  Terms are bucketed by z & 7 on the
-//     host, so an amplitude costs ~6 FP64 operations plus terms / 8.
+//   * state vectors of 8 qubits or more go by tiles (expec_tile.cu), except
+//     masks of more X/Y qubits than a tile has.
 // Reference semantics: QuEST_common.c:506-533 (calcExpecPauliSum: clone,
 // apply the Pauli string, inner product, per term).
 constexpr int kMaxGroupTerms = 32;
@@ -156,46 +185,7 @@ struct ExpecDM {
         return make_double2(pairValue(r, re[idx], im[idx], g), 0.0);
     }
 };
-constexpr int kDiagLow = 3;                      // low bits transformed per item
-constexpr int kDiagItem = 1 << kDiagLow;
-constexpr int kMaxDiagTerms = 64;
-struct PauliDiagGroup {
-    int off[kDiagItem + 1];                      // terms of bucket m (z & 7 = m): [off[m], off[m + 1])
-    uint64_t zh[kMaxDiagTerms];                  // z with the low bits cleared
-    double c[kMaxDiagTerms];
-};
-struct ExpecDiag {                               // SV, x = 0: 8 amplitudes per item (n >= 3)
-    const double *re, *im;
-    PauliDiagGroup g;
-    __device__ __forceinline__ double2 operator()(uint64_t i) const {
-        const uint64_t base = i << kDiagLow;
-        double p[kDiagItem];
-#pragma unroll
-        for (int h = 0; h < kDiagItem / 2; ++h) {
-            const double2 r = ld2(re + base + 2 * h), m = ld2(im + base + 2 * h);
-            p[2 * h] = r.x * r.x + m.x * m.x;
-            p[2 * h + 1] = r.y * r.y + m.y * m.y;
-        }
-#pragma unroll
-        for (int sb = 1; sb < kDiagItem; sb <<= 1)
-#pragma unroll
-            for (int l = 0; l < kDiagItem; ++l)
-                if (!(l & sb)) {
-                    const double a = p[l], b = p[l | sb];
-                    p[l] = a + b;
-                    p[l | sb] = a - b;
-                }
-        double acc = 0.0;
-#pragma unroll
-        for (int m = 0; m < kDiagItem; ++m) {
-            double gm = 0.0;
-            for (int t = g.off[m]; t < g.off[m + 1]; ++t) gm += (__popcll(base & g.zh[t]) & 1) ? -g.c[t] : g.c[t];
-            acc = fma(gm, p[m], acc);
-        }
-        return make_double2(acc, 0.0);
-    }
-};
-struct ExpecDiag1 {                              // SV, x = 0, one amplitude per item (n < 3)
+struct ExpecDiag1 {                              // SV, x = 0, one amplitude per item (n < 8)
     const double *re, *im;
     PauliPairGroup g;
     __device__ __forceinline__ double2 operator()(uint64_t j) const {
@@ -203,29 +193,81 @@ struct ExpecDiag1 {                              // SV, x = 0, one amplitude per
     }
 };
 
-// ---- calcProbOfAllOutcomes: shared-memory histogram, FP64 atomics --------
-__global__ void kOutcomeHist(const double* __restrict__ re, const double* __restrict__ im, uint64_t nItems,
-                             uint64_t step, int nq, const int* __restrict__ qs, double* __restrict__ out, int useShared) {
-    extern __shared__ double hist[];
-    const int nOut = 1 << nq;
-    if (useShared) {
-        for (int b = threadIdx.x; b < nOut; b += blockDim.x) hist[b] = 0.0;
+// ---- calcProbOfAllOutcomes ------------------------------------------------
+// The amplitude index is 8 low qubits, one per thread of a block, and the
+// rest, the items: (values of the measured high qubits, values of the others),
+// the others fastest.  A block takes a run of items; a thread sums its
+// amplitudes while the measured high qubits stay, four at a time on the
+// integer pipes, and the block then adds its threads of equal outcome and
+// gives the sums to out.  An atomic addition in shared memory per amplitude,
+// as before, took 119 us at 24 qubits and 10 measured ones; 46 us so.
+constexpr int kLowQubits = 8;
+struct OutcomeSpec {
+    int low, high;                 // low qubits (8, or all of fewer), the other ones
+    uint64_t measured;             // high qubits that are measured (bit 0: qubit `low`)
+    int highBit[64];               // the outcome's bit of each measured high qubit, ascending
+    uint32_t lowMask;              // low qubits that are measured
+    int lowBit[kLowQubits];        // the outcome's bit of each low qubit
+};
+template <bool DM>
+__global__ void __launch_bounds__(1 << kLowQubits) kOutcomes(const double* __restrict__ re, const double* __restrict__ im,
+                                                             uint64_t step, const __grid_constant__ OutcomeSpec s,
+                                                             double* __restrict__ out) {
+    __shared__ double part[1 << kLowQubits];
+    const uint32_t tid = threadIdx.x;
+    const bool live = tid < 1u << s.low;
+    const uint64_t others = ((1ull << s.high) - 1) & ~s.measured;
+    const int fast = __popcll(others);
+    const uint64_t items = 1ull << s.high;
+    const uint64_t each = items / gridDim.x, more = items % gridDim.x;
+    uint64_t k = each * blockIdx.x + min((uint64_t)blockIdx.x, more);
+    const uint64_t end = k + each + (blockIdx.x < more ? 1 : 0);
+    uint32_t own = 0;
+    for (int q = 0; q < s.low; ++q)
+        if (s.lowMask >> q & 1u) own |= ((tid >> q) & 1u) << s.lowBit[q];
+    while (k < end) {
+        // a run with the same measured high qubits
+        const uint64_t stop = min(end, ((k >> fast) + 1) << fast);
+        uint64_t set = 0, h = 0, v = k >> fast, r = k & ((1ull << fast) - 1);
+        uint32_t o = own;
+        for (int q = 0, m = 0; q < s.high; ++q) {
+            if (s.measured >> q & 1) {
+                set |= (v & 1) << q;
+                o |= (uint32_t)(v & 1) << s.highBit[m++];
+                v >>= 1;
+            } else {
+                h |= (r & 1) << q;
+                r >>= 1;
+            }
+        }
+        double acc = 0.0;
+        for (; k < stop; k += 4) {
+            double x[4] = {0, 0, 0, 0}, y[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (live && k + u < stop) {
+                    const uint64_t i = (((set | h) << s.low) | tid) * step;
+                    x[u] = re[i];
+                    if (!DM) y[u] = im[i];
+                }
+                h = ((h | ~others) + 1) & others;
+            }
+            if (DM) acc += (x[0] + x[1]) + (x[2] + x[3]);
+            else acc = fsum::addSquares(acc, make_double2(x[0], x[1]), make_double2(x[2], x[3]), make_double2(y[0], y[1]), make_double2(y[2], y[3]));
+        }
+        k = stop;
+        // the threads that differ in unmeasured low qubits only: lanes, then warps
+#pragma unroll
+        for (int q = 0; q < 5; ++q)
+            if (!(s.lowMask >> q & 1u)) acc += __shfl_xor_sync(0xffffffffu, acc, 1 << q);
         __syncthreads();
-    }
-    int q[32];
-    for (int b = 0; b < nq; ++b) q[b] = qs[b];
-    for (uint64_t it = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; it < nItems; it += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t i = it * step;                 // step = 1 (SV) or D + 1 (DM diagonal)
-        const double p = step == 1 ? re[i] * re[i] + im[i] * im[i] : re[i];
-        int o = 0;                                    // outcome bits of the amplitude (row) index
-        for (int b = 0; b < nq; ++b) o |= (int)((it >> q[b]) & 1ull) << b;
-        if (useShared) atomicAdd(hist + o, p);
-        else atomicAdd(out + o, p);
-    }
-    if (useShared) {
+        part[tid] = acc;
         __syncthreads();
-        for (int b = threadIdx.x; b < nOut; b += blockDim.x)
-            if (hist[b] != 0.0) atomicAdd(out + b, hist[b]);
+        const uint32_t skip = ~s.lowMask & ((1u << kLowQubits) - 1u);          // (qubits a small register lacks too)
+        if (tid & skip) continue;
+        for (uint32_t w = 1; w < 8; ++w)
+            if (((w << 5) & ~skip) == 0) acc += part[tid | (w << 5)];
+        atomicAdd(out + o, acc);
     }
 }
 
@@ -235,7 +277,7 @@ __global__ void kOutcomeHist(const double* __restrict__ re, const double* __rest
 double reduceTotalProbSV(SV s, const Scratch& w) {                 // replaces QuEST_gpu.cu:1649-1679
     double v = 0;
     const uint64_t n = 1ull << s.n;
-    if (n >= 2) runReduce(NormSq2{s.re, s.im}, n / 2, w, &v, nullptr, "calcTotalProb");
+    if (n >= 4) runSum<double>(NormSq4{{s.re, s.im}}, n / 4, w, &v, nullptr, "calcTotalProb");
     else runReduce(NormSq1{s.re, s.im}, n, w, &v, nullptr, "calcTotalProb");
     return v;
 }
@@ -251,9 +293,9 @@ double reduceTotalProbDM(SV s, int N, const Scratch& w) {          // replaces Q
 double reduceProbZeroSV(SV s, int t, const Scratch& w) {           // QuEST_gpu.cu:1992-2161
     double v = 0;
     const uint64_t half = 1ull << (s.n - 1);
-    if (t >= 1 && half >= 2) runReduce(ProbZeroVec{s.re, s.im, t}, half / 2, w, &v, nullptr, "calcProbOfOutcome");
-    else if (t == 0 && half >= 1 && s.n >= 1) runReduce(ProbZeroT0{s.re, s.im}, half, w, &v, nullptr, "calcProbOfOutcome");
-    else runReduce(ProbZeroDiag{s.re, 1, t}, half, w, &v, nullptr, "calcProbOfOutcome");
+    if (half < 4) runReduce(ProbZeroFew{s.re, s.im, t}, half, w, &v, nullptr, "calcProbOfOutcome");
+    else if (t >= 1) runSum<double>(ProbZero4{{s.re, s.im}, t}, half / 4, w, &v, nullptr, "calcProbOfOutcome");
+    else runSum<double>(ProbZeroEven{{s.re, s.im}}, half / 4, w, &v, nullptr, "calcProbOfOutcome");
     return v;
 }
 
@@ -265,7 +307,7 @@ double reduceProbZeroDM(SV s, int t, int N, const Scratch& w) {    // QuEST_gpu.
 
 void reduceInnerProduct(SV bra, SV ket, const Scratch& w, double* outRe, double* outIm) {   // QuEST_gpu.cu:2368-2483
     const uint64_t n = 1ull << bra.n;
-    if (n >= 2) runReduce(Inner2{bra.re, bra.im, ket.re, ket.im}, n / 2, w, outRe, outIm, "calcInnerProduct");
+    if (n >= 2) runSum<double2>(Inner2{bra.re, bra.im, ket.re, ket.im}, n / 2, w, outRe, outIm, "calcInnerProduct");
     else runReduce(Inner1{bra.re, bra.im, ket.re, ket.im}, n, w, outRe, outIm, "calcInnerProduct");
 }
 
@@ -323,28 +365,16 @@ double reduceExpecPauliGroups(SV s, int isDM, int N, const std::vector<PauliTerm
         ++used;
         return true;
     };
-    for (const PauliTermGroup& grp : groups) {
+    // state vectors go by tiles, except masks wider than a tile
+    std::vector<PauliTermGroup> tiled, rest;
+    for (const PauliTermGroup& grp : groups) (!isDM && expecTileTakes(s.n, grp.xmask) ? tiled : rest).push_back(grp);
+    const bool queued = queueExpecTiles(s, tiled, w, [&]() -> double* {
+        if (used == kSlots && !drain()) return nullptr;
+        return w.result + 2 * used++;
+    }, caller);
+    if (!queued) return total;
+    for (const PauliTermGroup& grp : rest) {
         const uint64_t x = grp.xmask;
-        const int nt = (int)grp.terms.size();
-        if (!isDM && x == 0 && s.n >= kDiagLow) {
-            // diagonal group: terms bucketed by their low bits
-            for (int b0 = 0; b0 < nt; b0 += kMaxDiagTerms) {
-                const int cnt = std::min(kMaxDiagTerms, nt - b0);
-                PauliDiagGroup g{};
-                int k = 0;
-                for (int m = 0; m < kDiagItem; ++m) {
-                    g.off[m] = k;
-                    for (int t = b0; t < b0 + cnt; ++t)
-                        if ((int)(grp.terms[t].yz & (kDiagItem - 1)) == m) {
-                            g.zh[k] = grp.terms[t].yz & ~(uint64_t)(kDiagItem - 1);
-                            g.c[k++] = grp.terms[t].coeff;    // x = 0: no Y, phase 0
-                        }
-                }
-                g.off[kDiagItem] = k;
-                if (!queue(ExpecDiag{s.re, s.im, g}, 1ull << (s.n - kDiagLow))) return total;
-            }
-            continue;
-        }
         // pairs / DM entries: each term goes to the Re (A) or Im (B) list
         std::vector<std::pair<uint64_t, double>> A, B;
         if (isDM) {
@@ -352,7 +382,7 @@ double reduceExpecPauliGroups(SV s, int isDM, int N, const std::vector<PauliTerm
                 const int ph = t.nY & 3;
                 (ph % 2 == 0 ? A : B).push_back({t.yz, ph < 2 ? t.coeff : -t.coeff});
             }
-        } else if (x == 0) {                     // n < 3 diagonal group: |psi_j|^2 terms
+        } else if (x == 0) {                     // n < 8 diagonal group: |psi_j|^2 terms
             for (const PauliTerm& t : grp.terms) A.push_back({t.yz, t.coeff});
         } else {
             pauliPairTerms(x, grp.terms, A, B);
@@ -383,7 +413,7 @@ double reduceExpecPauliGroups(SV s, int isDM, int N, const std::vector<PauliTerm
 void reduceProbAllOutcomes(SV s, int isDM, int N, const int* qubits, int nq, double* hostOut, const Scratch& w) {
     (void)w;
     const int nOut = 1 << nq;
-    const size_t bytes = (size_t)nOut * sizeof(double) + 32 * sizeof(int);
+    const size_t bytes = (size_t)nOut * sizeof(double);
     static double* dOut = nullptr;
     static size_t cap = 0;
     if (bytes > cap) {
@@ -394,17 +424,25 @@ void reduceProbAllOutcomes(SV s, int isDM, int N, const int* qubits, int nq, dou
         cap = bytes;
     }
     cudaStream_t st = stream();
-    int qs[32];
-    for (int b = 0; b < nq; ++b) qs[b] = qubits[b];
-    int* dQ = reinterpret_cast<int*>(dOut + nOut);
     if (QG_CUDA(cudaMemsetAsync(dOut, 0, (size_t)nOut * sizeof(double), st), "calcProbOfAllOutcomes")) return;
-    if (QG_CUDA(cudaMemcpyAsync(dQ, qs, nq * sizeof(int), cudaMemcpyHostToDevice, st), "calcProbOfAllOutcomes")) return;
-    const uint64_t nItems = isDM ? (1ull << N) : (1ull << s.n);
-    const uint64_t step = isDM ? (1ull << N) + 1 : 1;
-    const int useShared = nq <= 12;
-    const size_t smem = useShared ? (size_t)nOut * sizeof(double) : 0;
-    const int grid = (int)std::max<uint64_t>(1, std::min<uint64_t>((nItems + 255) / 256, (uint64_t)numSMs() * 4));
-    kOutcomeHist<<<grid, 256, smem, st>>>(s.re, s.im, nItems, step, nq, dQ, dOut, useShared);
+    const int n = isDM ? N : s.n;
+    OutcomeSpec sp{};
+    sp.low = std::min(n, kLowQubits);
+    sp.high = n - sp.low;
+    for (int q = 0, m = 0; q < n; ++q)
+        for (int b = 0; b < nq; ++b) {
+            if (qubits[b] != q) continue;
+            if (q < sp.low) {
+                sp.lowMask |= 1u << q;
+                sp.lowBit[q] = b;
+            } else {
+                sp.measured |= 1ull << (q - sp.low);
+                sp.highBit[m++] = b;
+            }
+        }
+    const unsigned grid = (unsigned)std::min<uint64_t>(1ull << sp.high, 8ull * (uint64_t)numSMs());
+    if (isDM) kOutcomes<true><<<grid, 1 << kLowQubits, 0, st>>>(s.re, s.im, (1ull << N) + 1, sp, dOut);
+    else kOutcomes<false><<<grid, 1 << kLowQubits, 0, st>>>(s.re, s.im, 1, sp, dOut);
     if (launchFailed("calcProbOfAllOutcomes")) return;
     QG_CUDA(cudaMemcpyAsync(hostOut, dOut, (size_t)nOut * sizeof(double), cudaMemcpyDeviceToHost, st), "calcProbOfAllOutcomes");
     QG_CUDA(cudaStreamSynchronize(st), "calcProbOfAllOutcomes");

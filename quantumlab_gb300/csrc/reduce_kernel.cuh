@@ -40,26 +40,14 @@ __device__ __forceinline__ double warpSum(double v) {
     return v;
 }
 
-// f(i) -> double2 contribution of item i.  4 items are loaded per iteration
-// so every thread keeps several loads in flight.
-template <class F>
-__global__ void __launch_bounds__(kThreads) kReduce(F f, uint64_t nItems, double* __restrict__ partials,
-                                                    unsigned int* __restrict__ counter, double* __restrict__ result) {
+// Sum of the blocks' (x, y) into result, which may be page-locked host memory
+// (each thread passes its own part).
+__device__ __forceinline__ void gridSum(double x, double y, double* __restrict__ partials, unsigned int* __restrict__ counter,
+                                        double* __restrict__ result) {
     __shared__ double sx[kWarps], sy[kWarps];
     __shared__ bool amLast;
-    Acc ax, ay;
-    const uint64_t stride = (uint64_t)gridDim.x * kThreads;
-    uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-    for (; i + 3 * stride < nItems; i += 4 * stride) {
-        const double2 v0 = f(i), v1 = f(i + stride), v2 = f(i + 2 * stride), v3 = f(i + 3 * stride);
-        ax.add2(v0.x + v2.x, v1.x + v3.x);
-        ay.add2(v0.y + v2.y, v1.y + v3.y);
-    }
-    for (; i < nItems; i += stride) {
-        const double2 v = f(i);
-        ax.add(v.x); ay.add(v.y);
-    }
-    double x = warpSum(ax.value()), y = warpSum(ay.value());
+    x = warpSum(x);
+    y = warpSum(y);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     if (lane == 0) { sx[w] = x; sy[w] = y; }
     __syncthreads();
@@ -94,6 +82,46 @@ __global__ void __launch_bounds__(kThreads) kReduce(F f, uint64_t nItems, double
     }
 }
 
+// f(i) -> double2 contribution of item i.  4 items are loaded per iteration
+// so every thread keeps several loads in flight.
+template <class F>
+__global__ void __launch_bounds__(kThreads) kReduce(F f, uint64_t nItems, double* __restrict__ partials,
+                                                    unsigned int* __restrict__ counter, double* __restrict__ result) {
+    Acc ax, ay;
+    const uint64_t stride = (uint64_t)gridDim.x * kThreads;
+    uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+    for (; i + 3 * stride < nItems; i += 4 * stride) {
+        const double2 v0 = f(i), v1 = f(i + stride), v2 = f(i + 2 * stride), v3 = f(i + 3 * stride);
+        ax.add2(v0.x + v2.x, v1.x + v3.x);
+        ay.add2(v0.y + v2.y, v1.y + v3.y);
+    }
+    for (; i < nItems; i += stride) {
+        const double2 v = f(i);
+        ax.add(v.x); ay.add(v.y);
+    }
+    gridSum(ax.value(), ay.value(), partials, counter, result);
+}
+
+// f(acc, i) -> acc plus item i, T double or double2 (functors whose item is
+// worth several FP64 operations saved)
+__device__ __forceinline__ double first(double v) { return v; }
+__device__ __forceinline__ double first(double2 v) { return v.x; }
+__device__ __forceinline__ double second(double) { return 0.0; }
+__device__ __forceinline__ double second(double2 v) { return v.y; }
+template <class T, class F>
+__global__ void __launch_bounds__(kThreads) kSum(F f, uint64_t nItems, double* __restrict__ partials,
+                                                 unsigned int* __restrict__ counter, double* __restrict__ result) {
+    T a{}, b{};
+    const uint64_t stride = (uint64_t)gridDim.x * kThreads;
+    uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
+    for (; i + stride < nItems; i += 2 * stride) {
+        a = f(a, i);
+        b = f(b, i + stride);
+    }
+    if (i < nItems) a = f(a, i);
+    gridSum(first(a) + first(b), second(a) + second(b), partials, counter, result);
+}
+
 inline int reduceGrid(uint64_t nItems) {
     // one full wave: 256-thread blocks, 8 resident per SM (the kernel needs
     // well under 32 registers per thread)
@@ -102,17 +130,25 @@ inline int reduceGrid(uint64_t nItems) {
     return (int)std::max<uint64_t>(1, std::min<uint64_t>(want, std::min<uint64_t>(resident, kMaxReduceBlocks)));
 }
 
-template <class F>
-inline bool runReduce(const F& f, uint64_t nItems, const Scratch& w, double* out0, double* out1, const char* caller) {
-    cudaStream_t st = stream();
-    const int grid = reduceGrid(nItems);
-    kReduce<F><<<grid, kThreads, 0, st>>>(f, nItems, w.partials, w.counter, w.result);
+// The kernels write the result to the register's page-locked slot themselves.
+inline bool takeResult(const Scratch& w, double* out0, double* out1, const char* caller) {
     if (launchFailed(caller)) return false;
-    if (QG_CUDA(cudaMemcpyAsync(w.host, w.result, 2 * sizeof(double), cudaMemcpyDeviceToHost, st), caller)) return false;
-    if (QG_CUDA(cudaStreamSynchronize(st), caller)) return false;
+    if (QG_CUDA(cudaStreamSynchronize(stream()), caller)) return false;
     if (out0) *out0 = w.host[0];
     if (out1) *out1 = w.host[1];
     return true;
+}
+template <class F>
+inline bool runReduce(const F& f, uint64_t nItems, const Scratch& w, double* out0, double* out1, const char* caller) {
+    kReduce<F><<<reduceGrid(nItems), kThreads, 0, stream()>>>(f, nItems, w.partials, w.counter, w.host);
+    return takeResult(w, out0, out1, caller);
+}
+template <class T, class F>
+inline bool runSum(const F& f, uint64_t nItems, const Scratch& w, double* out0, double* out1, const char* caller) {
+    // six blocks an SM are resident (40 registers): one wave
+    const unsigned grid = (unsigned)std::min<uint64_t>(reduceGrid(nItems), 6ull * (uint64_t)numSMs());
+    kSum<T, F><<<grid, kThreads, 0, stream()>>>(f, nItems, w.partials, w.counter, w.host);
+    return takeResult(w, out0, out1, caller);
 }
 
 }  // namespace red
