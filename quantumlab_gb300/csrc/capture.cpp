@@ -16,6 +16,7 @@
 // on for every register created afterwards, quest_gb300_setCapture per
 // register.  A gate on more than 6 qubits flushes the queue and runs directly.
 #include "fused_plan.h"
+#include "fused_small.h"
 #include "qg_internal.h"
 #include "quest_gb300.h"
 
@@ -32,12 +33,18 @@
 
 namespace qg {
 
+bool tensorCoresEnabled();       // fused_tc.cu
+bool tcDefaultAppliers();
+void freePlanTC(void* devicePlan);
+
 struct Capture {
     int n = 0;
     int dmQubits = 0;             // N of a density matrix, 0 for a state vector
     bool tracePreserving = true;  // every queued op is a unitary gate or a channel
     std::vector<FusedGate> gates;
     void* q32 = nullptr;          // FP32 scratch register of the flushes (kept between flushes)
+    // device memory of the last flush's plan, for the next one's
+    void *spare = nullptr, *smallSpare = nullptr;
     long long flushes = 0, gatesApplied = 0, passesApplied = 0;
     double compileMs = 0.0;       // host time spent planning the flushes
     // The last searched plan (gates and passes, no device copy).  A flush of
@@ -185,6 +192,11 @@ static void flushRecord(Capture* c, double* re, double* im) {
     plan->maxControls = defaultMaxControls(c->n);
     const bool tuned = g_capMaxFused == 0;
     plan->maxFused = tuned && c->shape ? c->shape->maxFused : capWidest(c->n);
+    // the device forms the products of a plan that runs at once
+    if (!tuned && tensorCoresEnabled() && plan->maxControls == 0)
+        plan->deferProducts = c->n <= kSmallMaxQubits && tcDefaultAppliers() ? 2 : c->n >= 13 ? 1 : 0;
+    plan->spare = c->spare;
+    plan->smallSpare = c->smallSpare;
     plan->gates.swap(c->gates);
     const auto t0 = std::chrono::steady_clock::now();
     // No lookahead: it takes 2-3x the search time for ~2 % fewer passes (12 %
@@ -212,6 +224,9 @@ static void flushRecord(Capture* c, double* re, double* im) {
     else quest_gb300_applyPlanF32(c->q32, plan);
     if (keepTrace) copyToQuregTraceKept(c->q32, view, c->dmQubits);
     else copyToQuregAfterPlan(c->q32, view, plan);
+    c->spare = plan->device ? plan->device : plan->spare;
+    c->smallSpare = plan->small ? plan->small : plan->smallSpare;
+    plan->device = plan->small = plan->spare = plan->smallSpare = nullptr;
     c->gatesApplied += (long long)plan->gates.size();
     c->passesApplied += (long long)plan->passes.size();
     c->flushes += 1;
@@ -260,6 +275,8 @@ void captureDrop(const double* re) {
         if (c->better.joinable()) c->better.join();
         if (c->betterPlan) quest_gb300_planDestroy(c->betterPlan);
         if (c->q32) quest_gb300_destroyQuregF32(c->q32);
+        freePlanTC(c->spare);
+        smallPlanFree(c->smallSpare);
         if (c->shape) quest_gb300_planDestroy(c->shape);
         delete c;
     }

@@ -40,14 +40,14 @@ struct QuregF32 {
 
 // tensor-core applier (fused_tc.cu): 1 applied, 0 not a tensor-core pass, -1 launch failed
 int applyPassTCIndexed(QuregF32& q, const FusedPass& p, const void* devPlan, size_t index, cudaStream_t st);
-void* uploadPlanTC(const FusedPlan& plan);
+void* uploadPlanTC(const FusedPlan& plan, void* reuse);
 bool tcImagesFit(const void* devPlan);
 void freePlanTC(void* d);
 int tcErrorFlag(const void* devPlan);
 int tcPassNorms(const void* devPlan, size_t index, double* out3);
 bool tcFinalNorms(const void* devPlan, const double** target, const double** out);
 void tcBeginPlan(void* devPlan, size_t numPasses);
-void tcBeginRange(void* devPlan, const double* entryBound);
+void tcBeginRange(void* devPlan, const double* entryBound, size_t first, size_t last);
 void tcNoteSimtPass(void* devPlan, size_t index);
 void setTensorCoresEnabled(bool on);
 void setTensorCoreKernel(int version);
@@ -520,7 +520,8 @@ static int applyRange(void* h, void* plan, int firstPass, int numPasses, const d
     const int last = std::min(total, firstPass + numPasses);
     if (!g_passEvents && qg::smallPlanFits(*p)) {
         if (!p->small) {
-            p->small = qg::smallPlanUpload(*p);
+            p->small = qg::smallPlanUpload(*p, p->smallSpare);
+            p->smallSpare = nullptr;
             p->smallFree = qg::smallPlanFree;
         }
         if (p->small) {
@@ -535,12 +536,13 @@ static int applyRange(void* h, void* plan, int firstPass, int numPasses, const d
         p->device = nullptr;
     }
     if (!p->device) {
-        p->device = qg::uploadPlanTC(*p);
+        p->device = qg::uploadPlanTC(*p, p->spare);
+        p->spare = nullptr;
         p->deviceFree = qg::freePlanTC;
     }
     cudaStream_t st = qg::stream();
     if (firstPass == 0) qg::tcBeginPlan(p->device, p->passes.size());
-    qg::tcBeginRange(p->device, entryBound);
+    qg::tcBeginRange(p->device, entryBound, firstPass, std::max(firstPass, last));
     bool usedTC = false;
     if (g_passEvents) {
         while ((int)g_passEv.size() < 2 * total) {
@@ -561,6 +563,7 @@ static int applyRange(void* h, void* plan, int firstPass, int numPasses, const d
                 invalidQuESTInputError("fused pass with control qubits needs the tensor-core applier", "applyPlanF32");
                 return -1;
             }
+            if (pass.m.empty()) qg::buildProduct(*p, i);
             if (!qg::applyPassSimt(*q, pass, st)) {
                 invalidQuESTInputError("fused pass on more than 5 qubits needs the tensor-core applier", "applyPlanF32");
                 return -1;

@@ -44,6 +44,7 @@
 // The inner loop runs over the D matrix columns.  Once the search has fixed
 // the passes, their products are independent and are shared among up to 16
 // host threads.
+#include "fused_build.h"
 #include "fused_plan.h"
 #include "quest_gb300.h"
 
@@ -448,14 +449,19 @@ FusedGate controlBlock(const FusedGate& g, uint64_t ctl, uint32_t val) {
 
 // products of the absorbed gates of one pass on its qubit set S, one per
 // value of its control qubits `ctl`
-void buildPass(const FusedPlan& plan, uint64_t S, uint64_t ctl, const std::vector<int>& absorbed, FusedPass& p) {
+void buildPass(const FusedPlan& plan, uint64_t S, uint64_t ctl, const std::vector<int>& absorbed, FusedPass& p, int defer) {
     p.targets.clear();
     p.controls.clear();
     for (int q = 0; q < 64; ++q) {
         if (S >> q & 1) p.targets.push_back(q);
         if (ctl >> q & 1) p.controls.push_back(q);
     }
+    p.numGates = (int)absorbed.size();
+    p.unitary = true;
+    for (int i : absorbed) p.unitary = p.unitary && plan.gates[i].unitary;
+    p.m.clear();
     const int k = (int)p.targets.size(), D = 1 << k;
+    if (defer && (k >= 4 || defer == 2) && buildsOnDevice(plan, p, absorbed)) return;
     const uint32_t nv = 1u << p.controls.size();
     int posOf[64];
     for (int b = 0; b < k; ++b) posOf[p.targets[b]] = b;
@@ -478,9 +484,34 @@ void buildPass(const FusedPlan& plan, uint64_t S, uint64_t ctl, const std::vecto
         cplx* blk = p.m.data() + (size_t)v * D * D;
         for (size_t e = 0; e < (size_t)D * D; ++e) blk[e] = cplx(Mr[e], Mi[e]);
     }
-    p.numGates = (int)absorbed.size();
-    p.unitary = true;
-    for (int i : absorbed) p.unitary = p.unitary && plan.gates[i].unitary;
+}
+
+void buildProduct(FusedPlan& plan, size_t i) {
+    buildPass(plan, plan.passSets[i], plan.passControls[i], plan.passMembers[i], plan.passes[i], 0);
+}
+
+// the passes of plan.passSets, their products shared among a few host threads
+static void buildPasses(FusedPlan& plan) {
+    const size_t np = plan.passSets.size();
+    plan.passes.resize(np);
+    std::atomic<size_t> nextPass{0};
+    auto work = [&]() {
+        for (size_t i; (i = nextPass.fetch_add(1)) < np;)
+            buildPass(plan, plan.passSets[i], plan.passControls[i], plan.passMembers[i], plan.passes[i], plan.deferProducts);
+    };
+    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+    unsigned nt = (unsigned)std::min<size_t>({(size_t)std::min(hw, 16u), np, 1 + plan.gates.size() / 64});
+    if (plan.deferProducts) nt = 1;                  // little is left to do
+    std::vector<std::thread> pool;
+    for (unsigned t = 1; t < nt; ++t) {
+        try {
+            pool.emplace_back(work);
+        } catch (...) {                     // fewer threads: the work items are shared
+            break;
+        }
+    }
+    work();
+    for (auto& t : pool) t.join();
 }
 
 void compilePlan(FusedPlan& plan) {
@@ -508,25 +539,7 @@ void compilePlan(FusedPlan& plan) {
         plan.compiled = true;                 // a structure for compilePlanLike
         return;
     }
-    // the pass products are independent: a few host threads share them
-    const size_t np = sets.size();
-    plan.passes.resize(np);
-    std::atomic<size_t> nextPass{0};
-    auto work = [&]() {
-        for (size_t i; (i = nextPass.fetch_add(1)) < np;) buildPass(plan, sets[i], ctls[i], members[i], plan.passes[i]);
-    };
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const unsigned nt = (unsigned)std::min<size_t>({(size_t)std::min(hw, 16u), np, 1 + plan.gates.size() / 64});
-    std::vector<std::thread> pool;
-    for (unsigned t = 1; t < nt; ++t) {
-        try {
-            pool.emplace_back(work);
-        } catch (...) {                     // fewer threads: the work items are shared
-            break;
-        }
-    }
-    work();
-    for (auto& t : pool) t.join();
+    buildPasses(plan);
     plan.compiled = true;
 }
 
@@ -544,25 +557,7 @@ bool compilePlanLike(FusedPlan& plan, const FusedPlan& structure) {
     plan.passSets = structure.passSets;
     plan.passControls = structure.passControls;
     plan.passMembers = structure.passMembers;
-    const size_t np = plan.passSets.size();
-    plan.passes.resize(np);
-    std::atomic<size_t> nextPass{0};
-    auto work = [&]() {
-        for (size_t i; (i = nextPass.fetch_add(1)) < np;)
-            buildPass(plan, plan.passSets[i], plan.passControls[i], plan.passMembers[i], plan.passes[i]);
-    };
-    const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-    const unsigned nt = (unsigned)std::min<size_t>({(size_t)std::min(hw, 16u), np, 1 + plan.gates.size() / 64});
-    std::vector<std::thread> pool;
-    for (unsigned t = 1; t < nt; ++t) {
-        try {
-            pool.emplace_back(work);
-        } catch (...) {                     // fewer threads: the work items are shared
-            break;
-        }
-    }
-    work();
-    for (auto& t : pool) t.join();
+    buildPasses(plan);
     plan.compiled = true;
     return true;
 }

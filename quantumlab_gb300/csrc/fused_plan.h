@@ -28,7 +28,9 @@ struct FusedPass {
     // diagonal.  The pass applies, to each amplitude, the matrix of the value
     // c of its control bits (bit j of c <-> controls[j]).
     std::vector<int> controls;
-    std::vector<cplx> m;       // 2^controls.size() row-major D x D blocks (block c), D = 2^targets.size()
+    // 2^controls.size() row-major D x D blocks (block c), D = 2^targets.size();
+    // empty while the product is left to the device (FusedPlan::deferProducts)
+    std::vector<cplx> m;
     int numGates = 0;
     bool unitary = false;      // every absorbed gate is unitary
 };
@@ -40,6 +42,9 @@ struct FusedPlan {
     int maxControls = 0;        // control qubits a pass may use (0..3; see FusedPass)
     int lookahead = 4;          // candidate sets tried one pass ahead (0: the best set at once)
     bool searchOnly = false;    // compilePlan finds the passes (passSets...) without their products
+    // Passes whose products the device may form as it uploads the plan
+    // (fused_build.cu): 0 none, 1 those on four qubits or more, 2 all.
+    int deferProducts = 0;
     std::vector<FusedGate> gates;
     std::vector<FusedPass> passes;
     // the search's result: per pass its qubit set and the indices of the
@@ -55,6 +60,8 @@ struct FusedPlan {
     // the same for a small register: the plan as one launch (fused_small.cu)
     void* small = nullptr;
     void (*smallFree)(void*) = nullptr;
+    // device copies of an earlier plan whose memory the next upload takes over
+    void *spare = nullptr, *smallSpare = nullptr;
 };
 // give the device copies back (the passes are about to change)
 inline void releaseDevice(FusedPlan& p) {
@@ -88,6 +95,9 @@ void compilePlan(FusedPlan& plan);
 // structure's reordering stays valid).  Gates of the same circuit with other
 // angles qualify.  Returns false (plan not compiled) otherwise.
 bool compilePlanLike(FusedPlan& plan, const FusedPlan& structure);
+
+// the product of a pass that was left to the device, on the host after all
+void buildProduct(FusedPlan& plan, size_t pass);
 
 // exp(-i angle/2 P) as a dense gate on the qubits of the Pauli string with
 // X/Y/Z masks x, y, z (Y bits also in x); the operator QuEST's

@@ -23,6 +23,7 @@
 //
 // Every wait on the barrier is bounded: a block that gives up sets the error
 // flag and ends.
+#include "fused_build.h"
 #include "fused_small.h"
 #include "qg_internal.h"
 
@@ -323,11 +324,16 @@ bool smallFits(int n, const std::vector<int>& targets) {
     return n >= 10 && n <= 30 && !targets.empty() && targets.size() <= 6;
 }
 
-size_t smallAddPass(SmallProgram& p, const FusedPass& pass, int n, size_t stateOffset, int registers, size_t mat) {
-    std::vector<int> t = pass.targets;
+// a pass's qubits, filled up to six with the lowest others
+static std::vector<int> widened(std::vector<int> t, int n) {
     for (int q = 0; q < n && (int)t.size() < 6; ++q)
         if (std::find(t.begin(), t.end(), q) == t.end()) t.push_back(q);
     std::sort(t.begin(), t.end());
+    return t;
+}
+
+size_t smallAddPass(SmallProgram& p, const FusedPass& pass, int n, size_t stateOffset, int registers, size_t mat) {
+    const std::vector<int> t = widened(pass.targets, n);
     std::vector<int> all = t;
     const int bits = p.groups == 32 ? 11 : p.groups == 16 ? 10 : 9;
     for (int q = 0; (int)all.size() < bits; ++q)
@@ -350,11 +356,8 @@ size_t smallAddPass(SmallProgram& p, const FusedPass& pass, int n, size_t stateO
 }
 
 void smallMatrix(const FusedPass& pass, int n, float* out) {
-    std::vector<int> t = pass.targets;
-    const int k = (int)t.size(), Dk = 1 << k;
-    for (int q = 0; q < n && (int)t.size() < 6; ++q)
-        if (std::find(t.begin(), t.end(), q) == t.end()) t.push_back(q);
-    std::sort(t.begin(), t.end());
+    const std::vector<int> t = widened(pass.targets, n);
+    const int Dk = 1 << pass.targets.size();
     int old[kD], rest[kD];                    // a 6-qubit index's bits on the pass's own qubits, and the others
     for (int i = 0; i < kD; ++i) {
         old[i] = rest[i] = 0;
@@ -414,13 +417,17 @@ bool smallUpload(SmallProgram& p, const float* mats, size_t matFloats, const cha
     }
     const size_t segBytes = segs.size() * sizeof(SmallSeg), segAt = matFloats * sizeof(float);
     const size_t countersAt = segAt + (segBytes + 31) / 32 * 32, counterBytes = 2 * sizeof(unsigned);
-    if (QG_CUDA(cudaMalloc(&p.buffer, countersAt + counterBytes), caller)) return false;
+    if (p.bytes < countersAt + counterBytes) {
+        smallFree(p);
+        if (QG_CUDA(cudaMalloc(&p.buffer, countersAt + counterBytes), caller)) return false;
+        p.bytes = countersAt + counterBytes;
+    }
     char* b = reinterpret_cast<char*>(p.buffer);
     p.dMats = reinterpret_cast<float*>(b);
     p.dSegs = b + segAt;
     p.counters = reinterpret_cast<unsigned*>(b + countersAt);
     // pageable sources: a copy returns once its source is staged
-    return !QG_CUDA(cudaMemcpyAsync(p.dMats, mats, segAt, cudaMemcpyHostToDevice, stream()), caller) &&
+    return (!mats || !QG_CUDA(cudaMemcpyAsync(p.dMats, mats, segAt, cudaMemcpyHostToDevice, stream()), caller)) &&
            !QG_CUDA(cudaMemcpyAsync(p.dSegs, segs.data(), segBytes, cudaMemcpyHostToDevice, stream()), caller) &&
            !QG_CUDA(cudaMemsetAsync(p.counters, 0, counterBytes, stream()), caller);
 }
@@ -431,12 +438,14 @@ void smallReset(SmallProgram& p) { cudaMemsetAsync(p.counters, 0, 2 * sizeof(uns
 void smallFree(SmallProgram& p) {
     if (p.buffer) cudaFree(p.buffer);
     p.buffer = nullptr;
+    p.bytes = 0;
 }
 
 // ------------------------------------------------------------ a plan on one register
 namespace {
 struct PlanProgram {
     SmallProgram p;
+    BuildScratch scratch;                     // of products formed on the device
     int* errFlag = nullptr;                   // page-locked: a kernel writes it only when it gives up
 };
 }  // namespace
@@ -448,9 +457,12 @@ bool smallPlanFits(const FusedPlan& plan) {
     return true;
 }
 
-void* smallPlanUpload(const FusedPlan& plan) {
-    PlanProgram* pp = new PlanProgram();
+void* smallPlanUpload(const FusedPlan& plan, void* reuse) {
+    PlanProgram* pp = reinterpret_cast<PlanProgram*>(reuse);
+    if (!pp) pp = new PlanProgram();
     const int n = plan.numQubits;
+    pp->p.segs.clear();
+    pp->p.first.clear();
     pp->p.groups = smallGroups((uint64_t)1 << n);
     size_t at = 0;
     pp->p.first.push_back(0);
@@ -458,10 +470,28 @@ void* smallPlanUpload(const FusedPlan& plan) {
         at = smallAddPass(pp->p, pass, n, 0, 1, at);
         pp->p.first.push_back((int)pp->p.segs.size());
     }
-    std::vector<float> mats(at);
-    for (size_t i = 0; i < plan.passes.size(); ++i) smallMatrix(plan.passes[i], n, mats.data() + i * 2 * kD * kD);
-    if (QG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&pp->errFlag), sizeof(int), cudaHostAllocMapped), "applyPlanF32") ||
-        !smallUpload(pp->p, mats.data(), at, "applyPlanF32")) {
+    std::vector<float> mats;
+    std::vector<int> deferred;
+    std::vector<BuildOutput> outputs;
+    for (size_t i = 0; i < plan.passes.size(); ++i) {
+        const FusedPass& pass = plan.passes[i];
+        if (pass.m.empty()) {
+            BuildOutput o;
+            o.small = i * 2 * kD * kD;
+            const std::vector<int> t = widened(pass.targets, n);
+            for (int b = 0; b < 6; ++b)
+                if (std::binary_search(pass.targets.begin(), pass.targets.end(), t[b])) o.smallMask |= 1 << b;
+            deferred.push_back((int)i);
+            outputs.push_back(o);
+            continue;
+        }
+        mats.resize(at);
+        smallMatrix(pass, n, mats.data() + i * 2 * kD * kD);
+    }
+    const char* caller = "applyPlanF32";
+    if ((!pp->errFlag && QG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&pp->errFlag), sizeof(int), cudaHostAllocMapped), caller)) ||
+        !smallUpload(pp->p, mats.empty() ? nullptr : mats.data(), at, caller) ||
+        !queueBuild(plan, deferred, outputs, pp->p.dMats, pp->scratch, stream(), caller)) {
         smallPlanFree(pp);
         return nullptr;
     }
@@ -474,6 +504,7 @@ void smallPlanFree(void* h) {
     if (!pp) return;
     cudaStreamSynchronize(stream());
     smallFree(pp->p);
+    freeBuildScratch(pp->scratch);
     if (pp->errFlag) cudaFreeHost(pp->errFlag);
     delete pp;
 }

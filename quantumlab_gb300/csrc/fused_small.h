@@ -27,6 +27,7 @@ struct SmallProgram {
     unsigned grid = 1;
     std::vector<SmallSeg> segs;
     std::vector<int> first;
+    size_t bytes = 0;                        // room in buffer
     void* buffer = nullptr;                  // device: matrices, segments, barrier counters
     float* dMats = nullptr;
     void* dSegs = nullptr;
@@ -44,6 +45,7 @@ bool smallFits(int n, const std::vector<int>& targets);
 size_t smallAddPass(SmallProgram& p, const FusedPass& pass, int n, size_t stateOffset, int registers, size_t mat);
 // the pass's matrix as the kernel reads it (2 x 64 x 64 floats)
 void smallMatrix(const FusedPass& pass, int n, float* out);
+// mats null: the caller fills p.dMats
 bool smallUpload(SmallProgram& p, const float* mats, size_t matFloats, const char* caller);
 bool smallLaunch(const SmallProgram& p, float* re, float* im, int step0, int step1, int* errFlag, cudaStream_t st,
                  const char* caller);
@@ -57,7 +59,8 @@ void smallFree(SmallProgram& p);
 // (14.5), 19 9.3 (14.7); 20 qubits 16.0 (13.9).
 constexpr int kSmallMaxQubits = 19;
 bool smallPlanFits(const FusedPlan& plan);
-void* smallPlanUpload(const FusedPlan& plan);
+// reuse: an earlier program, whose memory is taken over; null when it failed
+void* smallPlanUpload(const FusedPlan& plan, void* reuse);
 void smallPlanFree(void* program);
 int smallPlanApply(void* program, float* re, float* im, int first, int last);
 

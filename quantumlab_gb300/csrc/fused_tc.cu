@@ -39,6 +39,8 @@
 // Every wait is bounded: on timeout the CTA records an error code in a
 // device flag, skips the rest of its tiles, frees its TMEM and returns; the
 // host reads the flag after the pass.
+#include "chain_launch.cuh"
+#include "fused_build.h"
 #include "fused_plan.h"
 #include "qg_internal.h"
 
@@ -691,9 +693,6 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
                                                                   const __grid_constant__ TC2Params<KQ> p) {
     using S = TC2Shape<KQ, LG, EG, LS, PR>;
     constexpr bool BF = (PR == kPrecBF16), F16 = (PR == kPrecF16), H16 = BF || F16;
-    // split-FP16: X's scale 2^xe before the split (the epilogue undoes it)
-    const int xe = F16 ? f16XExp(nl) : 0;
-    const float kXs = __int_as_float((127 + xe) << 23);
     // this CTA's register of a batch and control value, and its place among
     // the CTAs of that pair
     const uint32_t cta = blockIdx.x % p.ctasPerInst, ncta = p.ctasPerInst;
@@ -755,6 +754,10 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
     fenceBefore();
     __syncthreads();
     fenceAfter();
+    chainStart();                                        // the state, norms and images are the grids' before
+    // split-FP16: X's scale 2^xe before the split (the epilogue undoes it)
+    const int xe = F16 ? f16XExp(nl) : 0;
+    const float kXs = __int_as_float((127 + xe) << 23);
     const uint32_t tmem = tmemBase;
     const int rw = warp & 3;                             // warp within its role = TMEM lane quarter
     const uint32_t laneSel = (uint32_t)(32 * rw) << 16;
@@ -1153,6 +1156,8 @@ struct DevicePlan {
     // unitary pass is corrected; a non-unitary pass changes the norm on purpose.
     std::vector<char> unitary;
     int parts = 0;          // the image parts built (kPart*)
+    size_t imageFloats = 0, normPasses = 0;          // room in imageBuf, norms
+    BuildScratch scratch;                            // of products formed on the device
 };
 
 // Canonical no-swizzle K-major image of an N x K operand (rows r, K index j):
@@ -1453,7 +1458,7 @@ bool launchTC2(float* re, float* im, int n, const FusedPass& pass, const float* 
             return false;
         configured = true;
     }
-    kApplyTC2<KQ, LG, EG, LS, PR, CV, ST><<<(unsigned)grid, (4 * (LG + EG) + 1) * 32, smem, st>>>(re, im, img, numTiles, errFlag, nl, p);
+    chain(kApplyTC2<KQ, LG, EG, LS, PR, CV, ST>, (unsigned)grid, (4 * (LG + EG) + 1) * 32, smem, st, re, im, img, numTiles, errFlag, nl, p);
     return !launchFailed("applyPlanF32");
 }
 
@@ -1592,20 +1597,34 @@ size_t g_stageFloats = 0;
 // and one copy.  A 6-qubit block holds 96 KB in split-TF32 (72 KB in
 // split-BF16); with every part it held 300 KB, whose building and pageable
 // copy took ~9 ms of each flush of the 30-qubit circuit.
-void* uploadPlanTC(const FusedPlan& plan) {
-    DevicePlan* dp = new DevicePlan();
+// Passes without a product (deferProducts) get product and image on the
+// device.  `reuse`: an earlier plan's copy, whose memory is taken over.
+void* uploadPlanTC(const FusedPlan& plan, void* reuse) {
+    DevicePlan* dp = reinterpret_cast<DevicePlan*>(reuse);
+    if (!dp) dp = new DevicePlan();
     dp->parts = currentParts();
-    if (cudaMalloc(&dp->errFlag, sizeof(int)) != cudaSuccess) {
+    dp->unitary.clear();
+    dp->inNorm.clear();
+    dp->target.clear();
+    dp->lastTC = -1;
+    dp->chain = false;
+    dp->entryBound = nullptr;
+    if (!dp->errFlag && cudaMalloc(&dp->errFlag, sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
         delete dp;
         return nullptr;
     }
     cudaMemsetAsync(dp->errFlag, 0, sizeof(int), stream());
-    if (cudaMalloc(&dp->norms, 3 * std::max<size_t>(1, plan.passes.size()) * sizeof(double)) != cudaSuccess) {
-        cudaGetLastError();
-        dp->norms = nullptr;
-    }
     const size_t np = plan.passes.size();
+    if (dp->normPasses < std::max<size_t>(1, np)) {
+        if (dp->norms) cudaFree(dp->norms);
+        dp->normPasses = std::max<size_t>(1, np);
+        if (cudaMalloc(&dp->norms, 3 * dp->normPasses * sizeof(double)) != cudaSuccess) {
+            cudaGetLastError();
+            dp->norms = nullptr;
+            dp->normPasses = 0;
+        }
+    }
     std::vector<size_t> offset(np + 1, 0);
     for (size_t i = 0; i < np; ++i) {
         const FusedPass& pass = plan.passes[i];
@@ -1616,11 +1635,43 @@ void* uploadPlanTC(const FusedPlan& plan) {
     }
     dp->images.assign(np, nullptr);
     if (offset[np] == 0) return dp;
-    if (cudaMalloc(&dp->imageBuf, offset[np] * sizeof(float)) != cudaSuccess) {
-        cudaGetLastError();
-        dp->imageBuf = nullptr;
-        return dp;                                   // every pass then runs on the SIMT applier
+    if (dp->imageFloats < offset[np]) {
+        if (dp->imageBuf) cudaFree(dp->imageBuf);
+        dp->imageFloats = 0;
+        if (cudaMalloc(&dp->imageBuf, offset[np] * sizeof(float)) != cudaSuccess) {
+            cudaGetLastError();
+            dp->imageBuf = nullptr;
+            return dp;                               // every pass then runs on the SIMT applier
+        }
+        dp->imageFloats = offset[np];
     }
+    std::vector<int> deferred;
+    std::vector<BuildOutput> outputs;
+    size_t onHost = 0;
+    for (size_t i = 0; i < np; ++i) {
+        if (offset[i + 1] == offset[i]) continue;
+        const FusedPass& pass = plan.passes[i];
+        if (!pass.m.empty()) {
+            ++onHost;
+            continue;
+        }
+        const ImageLayout lay = imageLayout((int)pass.targets.size(), dp->parts);
+        auto at = [&](size_t part) { return part == kNoPart ? kNoPart : offset[i] + part; };
+        BuildOutput o;
+        o.full = at(lay.full);
+        o.bf16 = at(lay.bf16);
+        o.compact = at(lay.compact);
+        o.f16 = at(lay.f16);
+        deferred.push_back((int)i);
+        outputs.push_back(o);
+    }
+    auto finish = [&]() {
+        if (!queueBuild(plan, deferred, outputs, dp->imageBuf, dp->scratch, stream(), "applyPlanF32")) return dp;
+        for (size_t i = 0; i < np; ++i)
+            if (offset[i + 1] > offset[i]) dp->images[i] = dp->imageBuf + offset[i];
+        return dp;
+    };
+    if (!onHost) return finish();
     // built in a page-locked staging buffer kept for the process (a captured
     // 30-qubit circuit re-uploads ~50 MB at every flush), else in pageable memory
     std::lock_guard<std::mutex> lk(g_stageMutex);
@@ -1645,7 +1696,7 @@ void* uploadPlanTC(const FusedPlan& plan) {
     std::atomic<size_t> next{0};
     auto work = [&]() {
         for (size_t i; (i = next.fetch_add(1)) < np;)
-            if (offset[i + 1] > offset[i]) buildImage(plan.passes[i], host + offset[i], dp->parts);
+            if (offset[i + 1] > offset[i] && !plan.passes[i].m.empty()) buildImage(plan.passes[i], host + offset[i], dp->parts);
     };
     const unsigned nt = (unsigned)std::min<size_t>({(size_t)16, (size_t)std::max(1u, std::thread::hardware_concurrency()), np});
     std::vector<std::thread> pool;
@@ -1659,9 +1710,7 @@ void* uploadPlanTC(const FusedPlan& plan) {
     work();
     for (auto& t : pool) t.join();
     cudaMemcpy(dp->imageBuf, host, offset[np] * sizeof(float), cudaMemcpyHostToDevice);
-    for (size_t i = 0; i < np; ++i)
-        if (offset[i + 1] > offset[i]) dp->images[i] = dp->imageBuf + offset[i];
-    return dp;
+    return finish();
 }
 
 // The tensor-core operands of one pass holding `parts`, as uploadPlanTC lays
@@ -1735,6 +1784,7 @@ void freePlanTC(void* h) {
     if (dp->imageBuf) cudaFree(dp->imageBuf);
     if (dp->errFlag) cudaFree(dp->errFlag);
     if (dp->norms) cudaFree(dp->norms);
+    freeBuildScratch(dp->scratch);
     delete dp;
 }
 
@@ -1750,12 +1800,14 @@ void tcBeginPlan(void* devPlan, size_t numPasses) {
 
 // start of every applyPlanF32Range call: the caller may have changed the
 // state since the last call, so the next tensor-core pass measures its input;
-// entryBound: sum |x|^2 of the state now, on the device, or null
-void tcBeginRange(void* devPlan, const double* entryBound) {
+// entryBound: sum |x|^2 of the state now, on the device, or null; the norm
+// records of passes [first, last) are cleared
+void tcBeginRange(void* devPlan, const double* entryBound, size_t first, size_t last) {
     DevicePlan* dp = reinterpret_cast<DevicePlan*>(devPlan);
     if (!dp) return;
     dp->chain = false;
     dp->entryBound = entryBound;
+    if (dp->norms && last > first) cudaMemsetAsync(dp->norms + 3 * first, 0, 3 * (last - first) * sizeof(double), stream());
 }
 
 // a pass ran on the SIMT applier: a non-unitary one changes the norm
@@ -2015,7 +2067,6 @@ int applyPassTCIndexed(QuregF32& q, const FusedPass& pass, const void* devPlan, 
         if (dp->inNorm.size() != dp->images.size()) dp->inNorm.assign(dp->images.size(), nullptr);
         if (dp->target.size() != dp->images.size()) dp->target.assign(dp->images.size(), nullptr);
         double* mine = dp->norms + 3 * index;            // in, out, scale^2
-        cudaMemsetAsync(mine, 0, 3 * sizeof(double), st);
         nl.out = mine + 1;
         nl.scaleSq = mine + 2;
         const bool chained = dp->chain && dp->lastTC >= 0;
