@@ -8,6 +8,7 @@
 // {rho[.0..0.], rho[.0..1.], rho[.1..0.], rho[.1..1.]} (row bit t, column bit
 // t+N), with the same per-entry arithmetic.
 #include "chain_launch.cuh"
+#include "scale_int.cuh"
 #include "qg_internal.h"
 
 #include <type_traits>
@@ -138,32 +139,42 @@ __global__ void kCollapseDM(double* __restrict__ re, double* __restrict__ im, ui
 // ---------------------------------------------------------------- channels
 // The four entries of one group: e00 = base, e01 = base|row, e10 = base|col,
 // e11 = base|row|col.  Off-diagonal-in-t entries are e01, e10.
+//
+// Scalings run on the integer pipes (scale_int.cuh), with the FP64 product's
+// bits: two FP64 operations an entry and more bound these kernels (12 qubits,
+// 268 MB: HBM 79 us, dephasing, which changes half the entries, 40).
+// mixDepolarising there 102 -> 82 us, mixDephasing 64 -> 50; mixDamping 79
+// before and after.
 struct Dephase {
-    double retain;
+    static constexpr bool kOffOnly = true;
+    ScaleInt retain;
     __device__ __forceinline__ void operator()(double&, double&, double& r01, double& i01, double& r10, double& i10,
                                                double&, double&) const {
-        r01 *= retain; i01 *= retain; r10 *= retain; i10 *= retain;
+        r01 = retain(r01); i01 = retain(i01); r10 = retain(r10); i10 = retain(i10);
     }
 };
 // QuEST_gpu.cu:2980-3004 (after the 1-level dephase): both diagonal entries
-// become (1-l) x + l (x+y)/2
+// become (1-l) x + l (x+y)/2 = x + l/2 (y-x)
 struct Depolarise {
-    double level;
+    static constexpr bool kOffOnly = false;
+    ScaleInt retain;
+    double half;                                 // l / 2
     __device__ __forceinline__ void operator()(double& r00, double& i00, double& r01, double& i01, double& r10,
                                                double& i10, double& r11, double& i11) const {
-        const double retain = 1 - level;
-        r01 *= retain; i01 *= retain; r10 *= retain; i10 *= retain;
-        const double avr = level * 0.5 * (r00 + r11), avi = level * 0.5 * (i00 + i11);
-        r00 = r00 * retain + avr; i00 = i00 * retain + avi;
-        r11 = r11 * retain + avr; i11 = i11 * retain + avi;
+        r01 = retain(r01); i01 = retain(i01); r10 = retain(r10); i10 = retain(i10);
+        const double dr = r11 - r00, di = i11 - i00;
+        r00 = fma(half, dr, r00); i00 = fma(half, di, i00);
+        r11 = fma(-half, dr, r11); i11 = fma(-half, di, i11);
     }
 };
 // QuEST_gpu.cu:3006-3078: off-diagonals * sqrt(1-p); rho00 += p rho11; rho11 *= 1-p
 struct Damp {
-    double p, dephase;
+    static constexpr bool kOffOnly = false;
+    double p;
+    ScaleInt dephase;
     __device__ __forceinline__ void operator()(double& r00, double& i00, double& r01, double& i01, double& r10,
                                                double& i10, double& r11, double& i11) const {
-        r01 *= dephase; i01 *= dephase; r10 *= dephase; i10 *= dephase;
+        r01 = dephase(r01); i01 = dephase(i01); r10 = dephase(r10); i10 = dephase(i10);
         const double tr = p * r11, ti = p * i11;
         r11 *= 1 - p; i11 *= 1 - p;
         r00 += tr; i00 += ti;
@@ -175,6 +186,7 @@ struct Damp {
 // superoperator of those four operators): the diagonal pair exchanges weight
 // pX + pY, the off-diagonal pair keeps 1 - pX - pY - 2 pZ and exchanges pX - pY.
 struct PauliMix {
+    static constexpr bool kOffOnly = false;
     double diagKeep, diagSwap, offKeep, offSwap;
     __device__ __forceinline__ void operator()(double& r00, double& i00, double& r01, double& i01, double& r10,
                                                double& i10, double& r11, double& i11) const {
@@ -195,16 +207,21 @@ __global__ void __launch_bounds__(kThreads) kChannelVec(double* __restrict__ re,
     const uint64_t rb = 1ull << t, cb = 1ull << (t + N);
     const uint64_t b = ins2(k << 1, t, t + N);
     chainStart();
-    double2 r00 = ld2(re + b), i00 = ld2(im + b);
+    double2 r00{}, i00{}, r11{}, i11{};
+    if (!Op::kOffOnly) {
+        r00 = ld2(re + b); i00 = ld2(im + b);
+        r11 = ld2(re + (b | rb | cb)); i11 = ld2(im + (b | rb | cb));
+    }
     double2 r01 = ld2(re + (b | rb)), i01 = ld2(im + (b | rb));
     double2 r10 = ld2(re + (b | cb)), i10 = ld2(im + (b | cb));
-    double2 r11 = ld2(re + (b | rb | cb)), i11 = ld2(im + (b | rb | cb));
     op(r00.x, i00.x, r01.x, i01.x, r10.x, i10.x, r11.x, i11.x);
     op(r00.y, i00.y, r01.y, i01.y, r10.y, i10.y, r11.y, i11.y);
-    st2(re + b, r00); st2(im + b, i00);
+    if (!Op::kOffOnly) {
+        st2(re + b, r00); st2(im + b, i00);
+        st2(re + (b | rb | cb), r11); st2(im + (b | rb | cb), i11);
+    }
     st2(re + (b | rb), r01); st2(im + (b | rb), i01);
     st2(re + (b | cb), r10); st2(im + (b | cb), i10);
-    st2(re + (b | rb | cb), r11); st2(im + (b | rb | cb), i11);
 }
 
 // row bit t == 0: (e00, e01) and (e10, e11) are adjacent pairs
@@ -441,13 +458,13 @@ void collapseDM(SV s, int target, int nRep, int outcome, double renorm) {
 void dmDephase(SV s, int t, int N, double retain) {
     const double S[16] = {1, 0, 0, 0, 0, retain, 0, 0, 0, 0, retain, 0, 0, 0, 0, 1};
     if (s.cap && captureChannel(s, t, N, S)) return;
-    launchChannel(s, t, N, Dephase{retain}, "mixDephasing");
+    launchChannel(s, t, N, Dephase{ScaleInt(retain)}, "mixDephasing");
 }
 void dmDepolarise(SV s, int t, int N, double level) {
     const double d = 1 - level / 2, x = level / 2, o = 1 - level;
     const double S[16] = {d, 0, 0, x, 0, o, 0, 0, 0, 0, o, 0, x, 0, 0, d};
     if (s.cap && captureChannel(s, t, N, S)) return;
-    launchChannel(s, t, N, Depolarise{level}, "mixDepolarising");
+    launchChannel(s, t, N, Depolarise{ScaleInt(1 - level), level / 2}, "mixDepolarising");
 }
 void dmPauli(SV s, int t, int N, double pX, double pY, double pZ) {
     const PauliMix op{1 - pX - pY, pX + pY, 1 - pX - pY - 2 * pZ, pX - pY};
@@ -477,7 +494,7 @@ void dmDamp(SV s, int t, int N, double p) {
     const double o = sqrt(1 - p);
     const double S[16] = {1, 0, 0, p, 0, o, 0, 0, 0, 0, o, 0, 0, 0, 0, 1 - p};
     if (s.cap && captureChannel(s, t, N, S)) return;
-    launchChannel(s, t, N, Damp{p, o}, "mixDamping");
+    launchChannel(s, t, N, Damp{p, ScaleInt(o)}, "mixDamping");
 }
 
 }  // namespace qg
