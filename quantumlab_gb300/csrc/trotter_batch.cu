@@ -74,10 +74,11 @@ __device__ __forceinline__ float signedSumF(uint64_t j, const uint64_t* m, const
 }
 // Re(conj(psi_j) psi_k) A(j) + Im(conj(psi_j) psi_k) B(j), in FP32, for
 // instance b (A's coefficients at coef[b * kCoefs], B's kMaxTerms later)
+template <class Shape = PairShape>
 struct PairsF32 {
     const float *re, *im;
     uint64_t dim;
-    PairShape g;
+    Shape g;                         // the shape, or a reference to it
     const float* coef;
     __device__ __forceinline__ double operator()(int b, uint64_t t) const {
         const float* r = re + (uint64_t)b * dim;
@@ -94,10 +95,11 @@ struct PairsF32 {
 // of sixteen 4-byte ones, one FP64 addition per four pairs.  The scalar form
 // was bound by load latency and FP64 work (one conversion and addition per
 // pair, GB300's FP64 pipe 55 % busy).
+template <class Shape = PairShape>
 struct PairsF32x4 {
     const float *re, *im;
     uint64_t dim;
-    PairShape g;
+    Shape g;                         // the shape, or a reference to it
     const float* coef;
     __device__ __forceinline__ double operator()(int b, uint64_t i) const {
         const float* r = re + (uint64_t)b * dim;
@@ -125,10 +127,11 @@ struct DiagShape {                   // x = 0: terms bucketed by their 4 low mas
 // sum over 16 amplitudes of |psi|^2 sum_t c_t (-1)^popc(j & z_t), through the
 // Walsh-Hadamard transform of the 16 probabilities (as in reduce.cu, which
 // takes 8), in FP32: a term then costs one signed addition per 16 amplitudes
+template <class Shape = DiagShape>
 struct DiagF32 {
     const float *re, *im;
     uint64_t dim;
-    DiagShape g;
+    Shape g;
     const float* coef;
     __device__ __forceinline__ double operator()(int b, uint64_t i) const {
         const uint64_t base = i * kDiagItem;
@@ -179,17 +182,21 @@ struct NormF32b {                    // 8 amplitudes per item
     }
 };
 
-// One reduction for every instance of the batch: block (x, b) sums items of
-// instance b; the last block of instance b (its ticket in counters[b]) adds
-// the instance's block partials in a fixed order into results[2 b].
+// The energy reductions of one class, over its instances.
+struct Red {
+    int kind;                                      // 0 pairs, 3 pairs by four, 1 diagonal, 2 norm
+    PairShape ps;
+    DiagShape ds;
+};
+
+// Sum of f(b, i) over nItems by the blocks x of instance b; the last block to
+// finish (its ticket) adds the block partials in a fixed order into result.
 constexpr int kMaxBlocksPerInst = 2048;
 template <class F>
-__global__ void __launch_bounds__(red::kThreads) kReduceBatch(F f, uint64_t nItems, double* __restrict__ partials,
-                                                              unsigned int* __restrict__ counters,
-                                                              double* __restrict__ results) {
+__device__ __forceinline__ void reduceInst(const F& f, int b, uint64_t nItems, double* __restrict__ part,
+                                           unsigned int* __restrict__ ticket, double* __restrict__ result) {
     __shared__ double sx[red::kWarps];
     __shared__ bool amLast;
-    const int b = blockIdx.y;
     const uint64_t stride = (uint64_t)gridDim.x * red::kThreads;
     uint64_t i = (uint64_t)blockIdx.x * red::kThreads + threadIdx.x;
     double a0 = 0.0, a1 = 0.0;
@@ -202,13 +209,12 @@ __global__ void __launch_bounds__(red::kThreads) kReduceBatch(F f, uint64_t nIte
     double x = red::warpSum(a0 + a1);
     if (lane == 0) sx[w] = x;
     __syncthreads();
-    double* part = partials + (size_t)b * kMaxBlocksPerInst;
     if (threadIdx.x == 0) {
         double t = 0.0;
         for (int k = 0; k < red::kWarps; ++k) t += sx[k];
         part[blockIdx.x] = t;
         __threadfence();
-        amLast = atomicAdd(counters + b, 1u) == gridDim.x - 1;
+        amLast = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
     if (!amLast) return;
@@ -221,10 +227,45 @@ __global__ void __launch_bounds__(red::kThreads) kReduceBatch(F f, uint64_t nIte
     if (threadIdx.x == 0) {
         double t = 0.0;
         for (int k = 0; k < red::kWarps; ++k) t += sx[k];
-        results[2 * b] = t;
-        results[2 * b + 1] = 0.0;
-        counters[b] = 0u;
+        result[0] = t;
+        result[1] = 0.0;
+        *ticket = 0u;
     }
+}
+// one reduction for every instance of a class (blockIdx.y)
+template <class F>
+__global__ void __launch_bounds__(red::kThreads) kReduceBatch(F f, uint64_t nItems, double* __restrict__ partials,
+                                                              unsigned int* __restrict__ counters,
+                                                              double* __restrict__ results) {
+    const int b = blockIdx.y;
+    reduceInst(f, b, nItems, partials + (size_t)b * kMaxBlocksPerInst, counters + b, results + 2 * b);
+}
+// items of a reduction over dim amplitudes: a pair (kind 0), four pairs or 8
+// amplitudes (kinds 3, 2), kDiagItem amplitudes (kind 1)
+__host__ __device__ inline uint64_t reduceItems(int kind, uint64_t dim) {
+    return kind == 0 ? dim / 2 : kind == 1 ? dim / kDiagItem : dim / 8;
+}
+// All reductions (blockIdx.z) of a class of small states, in one launch: 15
+// launches of about 5 us a class were 0.28 of the 2.25 ms of nine 16-qubit
+// instances, 0.08 in 3.
+__global__ void __launch_bounds__(red::kThreads) kReduceAll(const float* re, const float* im, uint64_t dim,
+                                                            const Red* __restrict__ reds, const float* __restrict__ coef,
+                                                            double* __restrict__ partials, unsigned int* __restrict__ tickets,
+                                                            double* __restrict__ results) {
+    __shared__ Red r;
+    const int b = blockIdx.y, M = gridDim.y, l = blockIdx.z;
+    for (int i = threadIdx.x; i < (int)(sizeof(Red) / 4); i += red::kThreads)
+        reinterpret_cast<uint32_t*>(&r)[i] = reinterpret_cast<const uint32_t*>(reds + l)[i];
+    __syncthreads();
+    coef += (size_t)l * M * kCoefs;
+    double* part = partials + (size_t)b * kMaxBlocksPerInst + l * gridDim.x;
+    unsigned int* ticket = tickets + l * M + b;
+    double* out = results + 2 * (l * M + b);
+    const uint64_t items = reduceItems(r.kind, dim);
+    if (r.kind == 0) reduceInst(PairsF32<const PairShape&>{re, im, dim, r.ps, coef}, b, items, part, ticket, out);
+    else if (r.kind == 3) reduceInst(PairsF32x4<const PairShape&>{re, im, dim, r.ps, coef}, b, items, part, ticket, out);
+    else if (r.kind == 1) reduceInst(DiagF32<const DiagShape&>{re, im, dim, r.ds, coef}, b, items, part, ticket, out);
+    else reduceInst(NormF32b{re, im, dim}, b, items, part, ticket, out);
 }
 
 __global__ void kBatchClassical(float* re, uint64_t stride, const long long* idx, int B) {
@@ -318,14 +359,6 @@ FusedPass widenNarrow(const FusedPass& p, int n) {
     return w;
 }
 
-// The energy reductions of one class: one launch each over the class's
-// instances (blockIdx.y = instance).
-struct Red {
-    int kind;                                      // 0 pairs, 3 pairs by four, 1 diagonal, 2 norm
-    PairShape ps;
-    DiagShape ds;
-};
-
 // Instances that share register size, Pauli strings, order and repetitions:
 // one fusion plan, one launch per pass over all of them.
 struct TrotterClass {
@@ -335,6 +368,7 @@ struct TrotterClass {
     int posBase = 0;                               // first row of partials / counters / dInit
     int slotBase = 0;                              // first result slot
     size_t coefOffset = 0;                         // floats into dCoef
+    size_t redOffset = 0;                          // its first reduction in dReds
     std::vector<FusedPass> shape;                  // per pass: the targets (member 0's pass)
     std::vector<size_t> imgOffset, imgStride;      // per pass, in floats into images
     std::vector<Red> reds;
@@ -363,6 +397,8 @@ struct TrotterBatch {
     unsigned int* counters = nullptr;              // per instance last-block tickets
     double* dResults = nullptr;                    // per class: slot slotBase + l * size + m
     double* hResults = nullptr;                    // pinned
+    Red* dReds = nullptr;                          // (oneLaunch) every class's reductions
+    unsigned int* dTickets = nullptr;              // (oneLaunch) per slot last-block tickets
     float* dCoef = nullptr;                        // per class, reduction l, member m: kCoefs floats
     int numSlots = 0;
     cudaGraph_t graph = nullptr;
@@ -377,7 +413,8 @@ void freeDevice(TrotterBatch* b) {
     if (b->graph) cudaGraphDestroy(b->graph);
     b->exec = nullptr;
     b->graph = nullptr;
-    for (void* p : {(void*)b->re, (void*)b->im, (void*)b->images, (void*)b->dInit, (void*)b->dCoef, (void*)b->dResults})
+    for (void* p : {(void*)b->re, (void*)b->im, (void*)b->images, (void*)b->dInit, (void*)b->dCoef, (void*)b->dResults, (void*)b->dReds,
+                    (void*)b->dTickets})
         if (p) cudaFree(p);
     if (b->hResults) cudaFreeHost(b->hResults);
     smallFree(b->small);
@@ -387,6 +424,8 @@ void freeDevice(TrotterBatch* b) {
     b->images = nullptr;
     b->dInit = nullptr;
     b->dCoef = nullptr;
+    b->dReds = nullptr;
+    b->dTickets = nullptr;
     b->dResults = nullptr;
     b->hResults = nullptr;
     b->classes.clear();
@@ -650,6 +689,11 @@ bool compileBatch(TrotterBatch* b) {
         slots += (int)(cl.reds.size() * M);
     }
     b->numSlots = slots;
+    std::vector<Red> reds;
+    for (TrotterClass& cl : b->classes) {
+        cl.redOffset = reds.size();
+        reds.insert(reds.end(), cl.reds.begin(), cl.reds.end());
+    }
     // operand images of every (class, pass, member), on host threads; in one
     // program step p holds pass p of every class that has one
     std::vector<std::vector<size_t>> matOf(C);     // per class and pass: member 0's matrix
@@ -701,8 +745,13 @@ bool compileBatch(TrotterBatch* b) {
                             QG_CUDA(cudaMemcpyAsync(b->images, host.data(), host.size() * sizeof(float), cudaMemcpyHostToDevice, st), kFn)) ||
         QG_CUDA(cudaMalloc(&b->dInit, B * sizeof(long long)), kFn) ||
         QG_CUDA(cudaMalloc(&b->dCoef, std::max<size_t>(1, coef.size()) * sizeof(float)), kFn) ||
+        QG_CUDA(cudaMalloc(&b->dReds, std::max<size_t>(1, reds.size()) * sizeof(Red)), kFn) ||
+        QG_CUDA(cudaMalloc(&b->dTickets, std::max(1, b->numSlots) * sizeof(unsigned int)), kFn) ||
         QG_CUDA(cudaMalloc(&b->dResults, 2 * (size_t)b->numSlots * sizeof(double)), kFn) ||
         QG_CUDA(cudaMallocHost(&b->hResults, 2 * (size_t)b->numSlots * sizeof(double)), kFn))
+        return false;
+    if (QG_CUDA(cudaMemcpyAsync(b->dReds, reds.data(), reds.size() * sizeof(Red), cudaMemcpyHostToDevice, st), kFn) ||
+        QG_CUDA(cudaMemsetAsync(b->dTickets, 0, std::max(1, b->numSlots) * sizeof(unsigned int), st), kFn))
         return false;
     if (QG_CUDA(cudaMemcpyAsync(b->dInit, init.data(), B * sizeof(long long), cudaMemcpyHostToDevice, st), kFn) ||
         QG_CUDA(cudaMemcpyAsync(b->dCoef, coef.data(), coef.size() * sizeof(float), cudaMemcpyHostToDevice, st), kFn) ||
@@ -746,24 +795,33 @@ bool queueRun(TrotterBatch* b, cudaStream_t st) {
         const float* im = b->im + cl.stateOffset;
         double* partials = b->partials + (size_t)cl.posBase * kMaxBlocksPerInst;
         unsigned int* counters = b->counters + cl.posBase;
+        const int R = (int)cl.reds.size();
+        if (b->oneLaunch && R <= 64) {
+            // enough blocks for the widest reduction; an instance's partials hold R x bx
+            const unsigned bx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(kMaxBlocksPerInst / R, dim / 2 / (4 * red::kThreads)));
+            kReduceAll<<<dim3(bx, (unsigned)M, (unsigned)R), red::kThreads, 0, st>>>(
+                re, im, dim, b->dReds + cl.redOffset, b->dCoef + cl.coefOffset, partials, b->dTickets + cl.slotBase,
+                b->dResults + 2 * (size_t)cl.slotBase);
+            if (launchFailed(kFn)) return false;
+            continue;
+        }
         for (size_t l = 0; l < cl.reds.size(); ++l) {
             const Red& r = cl.reds[l];
             const float* coef = b->dCoef + cl.coefOffset + l * (size_t)M * kCoefs;
             double* out = b->dResults + 2 * ((size_t)cl.slotBase + l * (size_t)M);
-            // items: a pair (kind 0), four pairs or 8 amplitudes (kinds 3, 2), kDiagItem amplitudes (kind 1)
-            const uint64_t items = r.kind == 0 ? dim / 2 : r.kind == 1 ? dim / kDiagItem : dim / 8;
+            const uint64_t items = reduceItems(r.kind, dim);
             const unsigned bx = (unsigned)std::max<uint64_t>(
                 1, std::min<uint64_t>({(uint64_t)kMaxBlocksPerInst, (items + red::kThreads - 1) / red::kThreads,
                                        std::max<uint64_t>(1, 8ull * (uint64_t)numSMs() / (uint64_t)M)}));
             const dim3 grid(bx, (unsigned)M);
             if (r.kind == 0)
-                kReduceBatch<<<grid, red::kThreads, 0, st>>>(PairsF32{re, im, dim, r.ps, coef}, items, partials,
+                kReduceBatch<<<grid, red::kThreads, 0, st>>>(PairsF32<>{re, im, dim, r.ps, coef}, items, partials,
                                                              counters, out);
             else if (r.kind == 3)
-                kReduceBatch<<<grid, red::kThreads, 0, st>>>(PairsF32x4{re, im, dim, r.ps, coef}, items, partials,
+                kReduceBatch<<<grid, red::kThreads, 0, st>>>(PairsF32x4<>{re, im, dim, r.ps, coef}, items, partials,
                                                              counters, out);
             else if (r.kind == 1)
-                kReduceBatch<<<grid, red::kThreads, 0, st>>>(DiagF32{re, im, dim, r.ds, coef}, items, partials,
+                kReduceBatch<<<grid, red::kThreads, 0, st>>>(DiagF32<>{re, im, dim, r.ds, coef}, items, partials,
                                                              counters, out);
             else
                 kReduceBatch<<<grid, red::kThreads, 0, st>>>(NormF32b{re, im, dim}, items, partials, counters, out);
