@@ -13,13 +13,11 @@
 //   * the next pass's matrix is copied (cp.async) and its addresses are worked
 //     out between a block's arrival at the barrier between passes and the
 //     last one's; amplitudes stay in L2.
-// A pass then takes about its 2 x 0.6 us of loads and barrier plus its
-// multiply-adds, 2^n * 256 of them over 152 SMs (0.9 us at 16 qubits), FP32
-// with each sum rounded to nearest, where the tensor cores' truncating
-// accumulation needs a norm correction.  16 qubits, 19 passes: 283 us before,
-// 105 us now (whole pass of the caller); the batch of nine Trotter instances of 16 qubits, 390 passes
-// one class after the other before, all classes side by side now: 3.79 ms
-// before, 2.26 ms now.
+// At 16 qubits a pass is some 6000 clocks: loads 600, the 64 x 8 sums 1500
+// (1024 at the FP32 rate), their shuffles and stores 1000, the fence and
+// barrier 2900.  Sums are FP32 rounded to nearest, where the tensor cores
+// truncate and need a norm correction.  19 passes, the caller's whole step with
+// its copies: 285 -> 100 us.
 //
 // Every wait on the barrier is bounded: a block that gives up sets the error
 // flag and ends.
@@ -40,13 +38,8 @@ namespace {
 constexpr int kD = 64;                       // a pass acts on 6 qubits (narrower ones are widened)
 constexpr unsigned long long kBarrierNs = 2000000000ull;
 
-struct Seg {                                 // one pass of one class of registers
-    uint64_t state;                          // floats from the base to the class's first register
-    uint64_t mat;                            // floats to its first matrix
-    uint32_t chunks;                         // over all its registers
-    uint32_t each, more;                     // (first of a step) chunks a block, blocks with one more
-    int chunkBits;                           // log2 of a register's chunks
-    int n;
+struct Seg {                                 // a pass
+    uint64_t mat;                            // floats to its matrix
     unsigned char pos[12];                   // the chunk's qubits, ascending
     unsigned short word[12];                 // what each stands for: a bit of row << 8 | group
 };
@@ -105,26 +98,27 @@ struct Shape {
 template <int GC>
 __global__ void __launch_bounds__(kThreads, 1) kSmallPasses(float* __restrict__ re, float* __restrict__ im,
                                                          const float* __restrict__ mats, const Seg* __restrict__ segs,
-                                                         int perStep, int step0, int step1,
+                                                         uint32_t chunks, int step0, int step1,
                                                          unsigned* __restrict__ counters, int* __restrict__ errFlag) {
     using S = Shape<GC>;
     extern __shared__ float4 smem4[];
     float* const g0 = reinterpret_cast<float*>(smem4);           // the matrix: 64 x 64 re, im, column by column
     float* const x0 = g0 + 2 * kD * kD;                          // staged re, im; later the KH column shares' sums
-    __shared__ Seg sg[3][kSmallMaxSegs];                         // this step's, the next two's
+    __shared__ Seg sg[3];                                        // this step's, the next two's
     __shared__ int alive;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int rt = lane & 7, kl = lane >> 3, gt = warp % (GC / 4), kh = warp / (GC / 4);
 
-    const int segWords = (int)sizeof(Seg) / 4 * perStep;         // at most 160
+    constexpr int segWords = (int)sizeof(Seg) / 4;
     auto segWord = [&](int step) {
-        return tid < segWords && step < step1 ? __ldg(reinterpret_cast<const uint32_t*>(segs + (size_t)step * perStep) + tid) : 0u;
+        return tid < segWords && step < step1 ? __ldg(reinterpret_cast<const uint32_t*>(segs + step) + tid) : 0u;
     };
     auto putSegs = [&](int buf, uint32_t w) {
-        if (tid < segWords) reinterpret_cast<uint32_t*>(sg[buf])[tid] = w;
+        if (tid < segWords) reinterpret_cast<uint32_t*>(sg + buf)[tid] = w;
     };
-    // block b's chunks of a step are [begin(b), begin(b + 1)) of all its segments' chunks
-    auto begin = [&](int buf, uint32_t b) { return sg[buf][0].each * b + min(b, sg[buf][0].more); };
+    // this block's chunks of a pass
+    const uint32_t each = chunks / gridDim.x, more = chunks % gridDim.x;
+    const uint32_t c0 = each * blockIdx.x + min(blockIdx.x, more), c1 = c0 + each + (blockIdx.x < more ? 1 : 0);
     // a chunk: its matrix, and where this thread's words of it lie (word i:
     // plane, amplitudes from the base, row and group of its first amplitude;
     // its others differ by d0, d1, both)
@@ -134,13 +128,10 @@ __global__ void __launch_bounds__(kThreads, 1) kSmallPasses(float* __restrict__ 
     };
     auto offset = [](uint32_t word, int stride) { return (word >> 8) * stride + (word & 255u); };
     auto chunk = [&](int buf, uint32_t c) {
-        int s = 0;
-        while (c >= sg[buf][s].chunks) c -= sg[buf][s++].chunks;
-        const Seg& g = sg[buf][s];
-        const uint32_t inst = c >> g.chunkBits;
-        uint32_t base = c & ((1u << g.chunkBits) - 1u);
+        const Seg& g = sg[buf];
+        uint32_t base = c;
         Chunk k;
-        k.mat = g.mat + (uint64_t)inst * (2 * kD * kD);
+        k.mat = g.mat;
         for (int i = 0; i < S::bits; ++i) base = ((base >> g.pos[i]) << (g.pos[i] + 1)) | (base & ((1u << g.pos[i]) - 1u));
         k.d0 = g.word[0];
         k.d1 = g.word[1];
@@ -153,7 +144,7 @@ __global__ void __launch_bounds__(kThreads, 1) kSmallPasses(float* __restrict__ 
                 off |= bit << g.pos[i];
                 word += bit * g.word[i];
             }
-            k.at[w] = g.state + ((uint64_t)inst << g.n) + (base | off);
+            k.at[w] = base | off;
             k.word[w] = word;
         }
         return k;
@@ -170,17 +161,10 @@ __global__ void __launch_bounds__(kThreads, 1) kSmallPasses(float* __restrict__ 
     putSegs(0, segWord(step0));
     putSegs(1, segWord(step0 + 1));
     __syncthreads();
-    uint32_t c0, c1;
-    Chunk cur{};
-    unsigned long long loaded = ~0ull;                           // the matrix in the buffer
+    // (every block has a chunk: the grid is no larger)
+    Chunk cur = chunk(0, c0);
     int sb = 0;
-    c0 = begin(0, blockIdx.x);
-    c1 = begin(0, blockIdx.x + 1);
-    if (c0 < c1) {
-        cur = chunk(0, c0);
-        loaded = cur.mat;
-        fetchMatrix(loaded);
-    }
+    fetchMatrix(cur.mat);
     for (int step = step0; step < step1; ++step) {
         const int sn = sb == 2 ? 0 : sb + 1, sa = sn == 2 ? 0 : sn + 1;
         const uint32_t ahead = segWord(step + 2);                // stored once the chunks are done
@@ -190,12 +174,8 @@ __global__ void __launch_bounds__(kThreads, 1) kSmallPasses(float* __restrict__ 
             for (int w = 0; w < S::items; ++w)
                 v[w] = __ldcg(reinterpret_cast<const float4*>((planeOf(w) ? im : re) + k.at[w]));
         };
-        if (c0 < c1) load(cur);
+        load(cur);
         for (uint32_t c = c0; c < c1; ++c) {
-            if (cur.mat != loaded) {
-                loaded = cur.mat;
-                fetchMatrix(loaded);
-            }
 #pragma unroll
             for (int w = 0; w < S::items; ++w) {
                 float* x = x0 + planeOf(w) * S::xPlane + offset(cur.word[w], S::xs);
@@ -285,15 +265,8 @@ __global__ void __launch_bounds__(kThreads, 1) kSmallPasses(float* __restrict__ 
         if (tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counters) : "memory");
         putSegs(sa, ahead);
         sb = sn;
-        c0 = begin(sb, blockIdx.x);
-        c1 = begin(sb, blockIdx.x + 1);
-        if (c0 < c1) {
-            cur = chunk(sb, c0);
-            if (cur.mat != loaded) {
-                loaded = cur.mat;
-                fetchMatrix(loaded);
-            }
-        }
+        cur = chunk(sb, c0);
+        fetchMatrix(cur.mat);
         if (tid == 0 && !awaitAll(counters, (unsigned)(step - step0 + 1) * gridDim.x)) {
             alive = 0;
             *errFlag = 7;
@@ -315,15 +288,6 @@ __global__ void __launch_bounds__(kThreads, 1) kSmallPasses(float* __restrict__ 
 
 }  // namespace
 
-int smallGroups(uint64_t amps) {
-    const uint64_t groups = amps / kD, sms = (uint64_t)numSMs();
-    return groups / 16 <= sms / 2 ? 8 : groups / 32 <= sms / 2 ? 16 : 32;
-}
-
-bool smallFits(int n, const std::vector<int>& targets) {
-    return n >= 10 && n <= 30 && !targets.empty() && targets.size() <= 6;
-}
-
 // a pass's qubits, filled up to six with the lowest others
 static std::vector<int> widened(std::vector<int> t, int n) {
     for (int q = 0; q < n && (int)t.size() < 6; ++q)
@@ -332,30 +296,26 @@ static std::vector<int> widened(std::vector<int> t, int n) {
     return t;
 }
 
-size_t smallAddPass(SmallProgram& p, const FusedPass& pass, int n, size_t stateOffset, int registers, size_t mat) {
+static Seg segOf(const FusedPass& pass, int n, int groups, size_t mat) {
     const std::vector<int> t = widened(pass.targets, n);
     std::vector<int> all = t;
-    const int bits = p.groups == 32 ? 11 : p.groups == 16 ? 10 : 9;
+    const int bits = groups == 32 ? 11 : groups == 16 ? 10 : 9;
     for (int q = 0; (int)all.size() < bits; ++q)
         if (std::find(t.begin(), t.end(), q) == t.end()) all.push_back(q);
     std::sort(all.begin(), all.end());
-    SmallSeg s{};
-    s.state = stateOffset;
+    Seg s{};
     s.mat = mat;
-    s.chunkBits = n - bits;
-    s.chunks = (uint32_t)registers << s.chunkBits;
-    s.n = n;
     int row = 0, group = 0;
     for (int i = 0; i < bits; ++i) {
         s.pos[i] = (unsigned char)all[i];
         const bool target = std::find(t.begin(), t.end(), all[i]) != t.end();
         s.word[i] = (unsigned short)(target ? 256 << row++ : 1 << group++);
     }
-    p.segs.push_back(s);
-    return mat + (size_t)registers * 2 * kD * kD;
+    return s;
 }
 
-void smallMatrix(const FusedPass& pass, int n, float* out) {
+// the pass's matrix as the kernel reads it
+static void smallMatrix(const FusedPass& pass, int n, float* out) {
     const std::vector<int> t = widened(pass.targets, n);
     const int Dk = 1 << pass.targets.size();
     int old[kD], rest[kD];                    // a 6-qubit index's bits on the pass's own qubits, and the others
@@ -375,85 +335,50 @@ void smallMatrix(const FusedPass& pass, int n, float* out) {
         }
 }
 
-bool smallLaunch(const SmallProgram& p, float* re, float* im, int step0, int step1, int* errFlag, cudaStream_t st, const char* caller) {
-    static_assert(sizeof(Seg) == sizeof(SmallSeg), "device layout");
-    if (step0 >= step1) return true;
-    const Seg* segs = reinterpret_cast<const Seg*>(p.dSegs);
-    const float* mats = p.dMats;
-    int perStep = p.perStep;
-    unsigned* counters = p.counters;
-    void* args[] = {&re, &im, &mats, &segs, &perStep, &step0, &step1, &counters, &errFlag};
-    const void* fn = p.groups == 32 ? (const void*)kSmallPasses<32> : p.groups == 16 ? (const void*)kSmallPasses<16>
-                                                                                  : (const void*)kSmallPasses<8>;
-    const size_t smem = p.groups == 32 ? Shape<32>::smem : p.groups == 16 ? Shape<16>::smem : Shape<8>::smem;
-    if (QG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), caller)) return false;
-    if (QG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(p.grid), dim3(kThreads), args, smem, st), caller)) return false;
-    return !launchFailed(caller);
-}
-
-bool smallUpload(SmallProgram& p, const float* mats, size_t matFloats, const char* caller) {
-    // every step's segments at the same stride (absent ones have no chunks)
-    const size_t steps = p.first.size() - 1;
-    p.perStep = 1;
-    for (size_t s = 0; s < steps; ++s) p.perStep = std::max(p.perStep, p.first[s + 1] - p.first[s]);
-    if (p.perStep > kSmallMaxSegs) return false;
-    std::vector<SmallSeg> segs(steps * p.perStep);
-    memset(segs.data(), 0, segs.size() * sizeof(SmallSeg));
-    p.maxChunks = 0;
-    for (size_t s = 0; s < steps; ++s) {
-        uint32_t c = 0;
-        for (int i = p.first[s]; i < p.first[s + 1]; ++i) {
-            segs[s * p.perStep + (i - p.first[s])] = p.segs[i];
-            c += p.segs[i].chunks;
-        }
-        p.maxChunks = std::max(p.maxChunks, c);
-        segs[s * p.perStep].each = c;                // (its total, for now)
-    }
-    p.grid = std::max(1u, std::min((unsigned)numSMs(), p.maxChunks));
-    for (size_t s = 0; s < steps; ++s) {
-        SmallSeg& g = segs[s * p.perStep];
-        g.more = g.each % p.grid;
-        g.each /= p.grid;
-    }
-    const size_t segBytes = segs.size() * sizeof(SmallSeg), segAt = matFloats * sizeof(float);
-    const size_t countersAt = segAt + (segBytes + 31) / 32 * 32, counterBytes = 2 * sizeof(unsigned);
-    if (p.bytes < countersAt + counterBytes) {
-        smallFree(p);
-        if (QG_CUDA(cudaMalloc(&p.buffer, countersAt + counterBytes), caller)) return false;
-        p.bytes = countersAt + counterBytes;
-    }
-    char* b = reinterpret_cast<char*>(p.buffer);
-    p.dMats = reinterpret_cast<float*>(b);
-    p.dSegs = b + segAt;
-    p.counters = reinterpret_cast<unsigned*>(b + countersAt);
-    // pageable sources: a copy returns once its source is staged
-    return (!mats || !QG_CUDA(cudaMemcpyAsync(p.dMats, mats, segAt, cudaMemcpyHostToDevice, stream()), caller)) &&
-           !QG_CUDA(cudaMemcpyAsync(p.dSegs, segs.data(), segBytes, cudaMemcpyHostToDevice, stream()), caller) &&
-           !QG_CUDA(cudaMemsetAsync(p.counters, 0, counterBytes, stream()), caller);
-}
-
-// after an error: a launch that gave up leaves the counters as they stood
-void smallReset(SmallProgram& p) { cudaMemsetAsync(p.counters, 0, 2 * sizeof(unsigned), stream()); }
-
-void smallFree(SmallProgram& p) {
-    if (p.buffer) cudaFree(p.buffer);
-    p.buffer = nullptr;
-    p.bytes = 0;
-}
-
 // ------------------------------------------------------------ a plan on one register
 namespace {
 struct PlanProgram {
-    SmallProgram p;
+    int groups = 16;                          // groups of 64 amplitudes a chunk
+    uint32_t chunks = 0;
     BuildScratch scratch;                     // of products formed on the device
     int* errFlag = nullptr;                   // page-locked: a kernel writes it only when it gives up
+    size_t bytes = 0;                         // room in buffer
+    char* buffer = nullptr;                   // device: matrices, passes, barrier counters
+    float* mats = nullptr;
+    Seg* segs = nullptr;
+    unsigned* counters = nullptr;             // arrivals at the barrier, ended blocks; zero between launches
 };
+constexpr size_t kCounterBytes = 2 * sizeof(unsigned);
+
+bool launch(const PlanProgram& p, float* re, float* im, int step0, int step1, cudaStream_t st, const char* caller) {
+    if (step0 >= step1) return true;
+    const Seg* segs = p.segs;
+    const float* mats = p.mats;
+    uint32_t chunks = p.chunks;
+    unsigned* counters = p.counters;
+    int* errFlag = p.errFlag;
+    void* args[] = {&re, &im, &mats, &segs, &chunks, &step0, &step1, &counters, &errFlag};
+    const void* fn = p.groups == 32 ? (const void*)kSmallPasses<32> : p.groups == 16 ? (const void*)kSmallPasses<16>
+                                                                                  : (const void*)kSmallPasses<8>;
+    const size_t smem = p.groups == 32 ? Shape<32>::smem : p.groups == 16 ? Shape<16>::smem : Shape<8>::smem;
+    const unsigned grid = std::min((unsigned)numSMs(), chunks);
+    if (QG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), caller)) return false;
+    if (QG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, smem, st), caller)) return false;
+    return !launchFailed(caller);
+}
+
+// the most of 8, 16, 32 groups a chunk that leaves at most half the SMs
+// without a chunk
+int groupsFor(uint64_t amps) {
+    const uint64_t groups = amps / kD, sms = (uint64_t)numSMs();
+    return groups / 16 <= sms / 2 ? 8 : groups / 32 <= sms / 2 ? 16 : 32;
+}
 }  // namespace
 
 bool smallPlanFits(const FusedPlan& plan) {
-    if (plan.numQubits > kSmallMaxQubits || plan.passes.empty() || !tcDefaultAppliers()) return false;
+    if (plan.numQubits < 10 || plan.numQubits > kSmallMaxQubits || plan.passes.empty() || !tcDefaultAppliers()) return false;
     for (const FusedPass& pass : plan.passes)
-        if (!pass.controls.empty() || !smallFits(plan.numQubits, pass.targets)) return false;
+        if (!pass.controls.empty() || pass.targets.empty() || pass.targets.size() > 6) return false;
     return true;
 }
 
@@ -461,15 +386,11 @@ void* smallPlanUpload(const FusedPlan& plan, void* reuse) {
     PlanProgram* pp = reinterpret_cast<PlanProgram*>(reuse);
     if (!pp) pp = new PlanProgram();
     const int n = plan.numQubits;
-    pp->p.segs.clear();
-    pp->p.first.clear();
-    pp->p.groups = smallGroups((uint64_t)1 << n);
-    size_t at = 0;
-    pp->p.first.push_back(0);
-    for (const FusedPass& pass : plan.passes) {
-        at = smallAddPass(pp->p, pass, n, 0, 1, at);
-        pp->p.first.push_back((int)pp->p.segs.size());
-    }
+    pp->groups = groupsFor((uint64_t)1 << n);
+    pp->chunks = (uint32_t)(((uint64_t)1 << n) / kD / pp->groups);
+    const size_t at = plan.passes.size() * 2 * kD * kD;
+    std::vector<Seg> segs;
+    for (size_t i = 0; i < plan.passes.size(); ++i) segs.push_back(segOf(plan.passes[i], n, pp->groups, i * 2 * kD * kD));
     std::vector<float> mats;
     std::vector<int> deferred;
     std::vector<BuildOutput> outputs;
@@ -489,9 +410,29 @@ void* smallPlanUpload(const FusedPlan& plan, void* reuse) {
         smallMatrix(pass, n, mats.data() + i * 2 * kD * kD);
     }
     const char* caller = "applyPlanF32";
-    if ((!pp->errFlag && QG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&pp->errFlag), sizeof(int), cudaHostAllocMapped), caller)) ||
-        !smallUpload(pp->p, mats.empty() ? nullptr : mats.data(), at, caller) ||
-        !queueBuild(plan, deferred, outputs, pp->p.dMats, pp->scratch, stream(), caller)) {
+    const size_t matBytes = at * sizeof(float), segBytes = (segs.size() * sizeof(Seg) + 31) / 32 * 32;
+    if (!pp->errFlag && QG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&pp->errFlag), sizeof(int), cudaHostAllocMapped), caller)) {
+        smallPlanFree(pp);
+        return nullptr;
+    }
+    if (pp->bytes < matBytes + segBytes + kCounterBytes) {
+        if (pp->buffer) cudaFree(pp->buffer);
+        pp->buffer = nullptr;
+        pp->bytes = 0;
+        if (QG_CUDA(cudaMalloc(&pp->buffer, matBytes + segBytes + kCounterBytes), caller)) {
+            smallPlanFree(pp);
+            return nullptr;
+        }
+        pp->bytes = matBytes + segBytes + kCounterBytes;
+    }
+    pp->mats = reinterpret_cast<float*>(pp->buffer);
+    pp->segs = reinterpret_cast<Seg*>(pp->buffer + matBytes);
+    pp->counters = reinterpret_cast<unsigned*>(pp->buffer + matBytes + segBytes);
+    // pageable sources: a copy returns once its source is staged
+    if ((!mats.empty() && QG_CUDA(cudaMemcpyAsync(pp->mats, mats.data(), matBytes, cudaMemcpyHostToDevice, stream()), caller)) ||
+        QG_CUDA(cudaMemcpyAsync(pp->segs, segs.data(), segs.size() * sizeof(Seg), cudaMemcpyHostToDevice, stream()), caller) ||
+        QG_CUDA(cudaMemsetAsync(pp->counters, 0, kCounterBytes, stream()), caller) ||
+        !queueBuild(plan, deferred, outputs, pp->mats, pp->scratch, stream(), caller)) {
         smallPlanFree(pp);
         return nullptr;
     }
@@ -503,7 +444,7 @@ void smallPlanFree(void* h) {
     PlanProgram* pp = reinterpret_cast<PlanProgram*>(h);
     if (!pp) return;
     cudaStreamSynchronize(stream());
-    smallFree(pp->p);
+    if (pp->buffer) cudaFree(pp->buffer);
     freeBuildScratch(pp->scratch);
     if (pp->errFlag) cudaFreeHost(pp->errFlag);
     delete pp;
@@ -512,12 +453,13 @@ void smallPlanFree(void* h) {
 // passes [first, last) of the plan; 0, a kernel's error code, or -1 when the launch failed
 int smallPlanApply(void* h, float* re, float* im, int first, int last) {
     PlanProgram* pp = reinterpret_cast<PlanProgram*>(h);
-    if (!smallLaunch(pp->p, re, im, first, last, pp->errFlag, stream(), "applyPlanF32")) return -1;
+    if (!launch(*pp, re, im, first, last, stream(), "applyPlanF32")) return -1;
     if (QG_CUDA(cudaStreamSynchronize(stream()), "applyPlanF32")) return -1;
     const int e = *reinterpret_cast<volatile int*>(pp->errFlag);
     if (e) {
         *pp->errFlag = 0;
-        smallReset(pp->p);
+        // a launch that gave up leaves the counters as they stood
+        cudaMemsetAsync(pp->counters, 0, kCounterBytes, stream());
     }
     return e;
 }

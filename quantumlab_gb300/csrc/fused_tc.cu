@@ -294,6 +294,7 @@ struct NormLinks {
     const double* corrScaleSq;
     const double* corrTarget;
     const double* boundSq;
+    bool imageReady = false;     // the operand image is older than any launch still running
 };
 // the scale minus one (kept exact to FP32 relative precision)
 __device__ __forceinline__ float driftCorrection(const NormLinks& nl) {
@@ -733,6 +734,12 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
     __shared__ volatile int abortF;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    auto copyImage = [&]() {
+        mbarExpectTx(&barG, S::NGP * kGW * 4);
+        bulkG2S(gh, gImage, kGW * 4, &barG);
+        bulkG2S(gl, gImage + kGW, kGW * 4, &barG);
+        if (BF) bulkG2S(gll, gImage + 2 * kGW, kGW * 4, &barG);
+    };
     if (warp == kMmaWarp) {
         if (lane == 0) {
             abortF = 0;
@@ -749,12 +756,14 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
                 for (int b = 0; b < kStageBars; ++b) mbarInit(&stageB[b], 1);
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
+        // an image that is in place already comes while the grid before ends
+        if (lane == 0 && nl.imageReady) copyImage();
         tmemAlloc(&tmemBase, kCols);
     }
     fenceBefore();
     __syncthreads();
     fenceAfter();
-    chainStart();                                        // the state, norms and images are the grids' before
+    chainStart();                                        // the state, norms and new images are the grids' before
     // split-FP16: X's scale 2^xe before the split (the epilogue undoes it)
     const int xe = F16 ? f16XExp(nl) : 0;
     const float kXs = __int_as_float((127 + xe) << 23);
@@ -1045,10 +1054,7 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
         if (lane == 0 && nl.out) atomicAdd(nl.out, normOut);
     } else if (lane == 0) {
         // ------------------------------------------------ TMA of G, then MMAs
-        mbarExpectTx(&barG, S::NGP * kGW * 4);
-        bulkG2S(gh, gImage, kGW * 4, &barG);
-        bulkG2S(gl, gImage + kGW, kGW * 4, &barG);
-        if (BF) bulkG2S(gll, gImage + 2 * kGW, kGW * 4, &barG);
+        if (!nl.imageReady) copyImage();
         bool ok = mbarWaitOrAbort(&barG, 0, &abortF);
         if (!ok) mbarWaitOrAbort(&barG, 0, &abortF);                // once more for the copies in flight
         const uint32_t ghA = smemAddr(gh), glA = smemAddr(gl), gllA = smemAddr(gll);
@@ -1156,6 +1162,7 @@ struct DevicePlan {
     // unitary pass is corrected; a non-unitary pass changes the norm on purpose.
     std::vector<char> unitary;
     int parts = 0;          // the image parts built (kPart*)
+    bool imagesReady = false;   // all of them copied from the host (and the copy waited for)
     size_t imageFloats = 0, normPasses = 0;          // room in imageBuf, norms
     BuildScratch scratch;                            // of products formed on the device
 };
@@ -1665,6 +1672,7 @@ void* uploadPlanTC(const FusedPlan& plan, void* reuse) {
         deferred.push_back((int)i);
         outputs.push_back(o);
     }
+    dp->imagesReady = deferred.empty();
     auto finish = [&]() {
         if (!queueBuild(plan, deferred, outputs, dp->imageBuf, dp->scratch, stream(), "applyPlanF32")) return dp;
         for (size_t i = 0; i < np; ++i)
@@ -2063,6 +2071,7 @@ int applyPassTCIndexed(QuregF32& q, const FusedPass& pass, const void* devPlan, 
     const int version = tcKernelFor(pass, n);
     if (version == 0) return 0;
     NormLinks nl{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    nl.imageReady = dp->imagesReady;
     if (dp->norms) {
         if (dp->inNorm.size() != dp->images.size()) dp->inNorm.assign(dp->images.size(), nullptr);
         if (dp->target.size() != dp->images.size()) dp->target.assign(dp->images.size(), nullptr);
@@ -2153,7 +2162,7 @@ bool applyPassTCBatch(float* re, float* im, int n, const FusedPass& pass, const 
                       int parts, int batch, int* errFlag, cudaStream_t st) {
     const int version = tcKernelFor(pass, n);
     if (version < 2 || !images || !pass.controls.empty()) return false;
-    const NormLinks nl{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    const NormLinks nl{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, true};   // (compileBatch waits for the copy)
     return launchPassTC(version, pass, re, im, n, images, parts, errFlag, nl, st, batch, 1ull << n,
                         (uint64_t)imageStride);
 }

@@ -18,11 +18,7 @@
 //   * each pass is one launch of the tensor-core applier over all the class's
 //     states (the CTAs are shared out among the states, each state's CTAs
 //     load that state's operands); passes narrower than 4 qubits are widened
-//     with identity factors so that every pass runs on the tensor cores.
-//     Classes of small states (2^19 amplitudes at most) run side by side
-//     instead, all their passes in one launch (fused_small.cu): nine 16-qubit
-//     instances in three classes took 3.79 ms one class after the other,
-//     2.26 ms side by side;
+//     with identity factors so that every pass runs on the tensor cores;
 //   * the energies <H_b> are reduced from the FP32 states (FP32 products per
 //     amplitude pair, FP64 sums), one launch per term group over the class's
 //     states, divided by each state's norm, which also removes the norm drift
@@ -31,7 +27,6 @@
 //     passes and reductions, and the copy of the results to pinned host
 //     memory) is one CUDA graph that later runs replay.
 #include "fused_plan.h"
-#include "fused_small.h"
 #include "qg_internal.h"
 #include "quest_gb300.h"
 #include "reduce_kernel.cuh"
@@ -50,7 +45,6 @@ namespace qg {
 size_t tcImageFloats(int k, int parts);
 void tcBuildImage(const FusedPass& pass, float* img, int parts);
 int tcImageParts();
-bool tcDefaultAppliers();
 bool applyPassTCBatch(float* re, float* im, int n, const FusedPass& pass, const float* images, size_t imageStride,
                       int parts, int batch, int* errFlag, cudaStream_t st);
 
@@ -247,7 +241,7 @@ __host__ __device__ inline uint64_t reduceItems(int kind, uint64_t dim) {
 }
 // All reductions (blockIdx.z) of a class of small states, in one launch: 15
 // launches of about 5 us a class were 0.28 of the 2.25 ms of nine 16-qubit
-// instances, 0.08 in 3.
+// instances, 0.08 in 3 launches.
 __global__ void __launch_bounds__(red::kThreads) kReduceAll(const float* re, const float* im, uint64_t dim,
                                                             const Red* __restrict__ reds, const float* __restrict__ coef,
                                                             double* __restrict__ partials, unsigned int* __restrict__ tickets,
@@ -385,8 +379,6 @@ struct TrotterBatch {
     std::vector<Instance> inst;
     bool compiled = false;
     int parts = 0;                                 // operand image parts built (tcImageParts)
-    bool oneLaunch = false;                        // all passes as one program instead
-    SmallProgram small;
     std::vector<TrotterClass> classes;
     std::vector<int> classOf, posOf;               // per instance: its class, its place in it
     float *re = nullptr, *im = nullptr;            // every class's states, class after class
@@ -397,8 +389,8 @@ struct TrotterBatch {
     unsigned int* counters = nullptr;              // per instance last-block tickets
     double* dResults = nullptr;                    // per class: slot slotBase + l * size + m
     double* hResults = nullptr;                    // pinned
-    Red* dReds = nullptr;                          // (oneLaunch) every class's reductions
-    unsigned int* dTickets = nullptr;              // (oneLaunch) per slot last-block tickets
+    Red* dReds = nullptr;                          // every class's reductions (kReduceAll)
+    unsigned int* dTickets = nullptr;              // its last-block tickets, per slot
     float* dCoef = nullptr;                        // per class, reduction l, member m: kCoefs floats
     int numSlots = 0;
     cudaGraph_t graph = nullptr;
@@ -417,9 +409,6 @@ void freeDevice(TrotterBatch* b) {
                     (void*)b->dTickets})
         if (p) cudaFree(p);
     if (b->hResults) cudaFreeHost(b->hResults);
-    smallFree(b->small);
-    b->small = SmallProgram();
-    b->oneLaunch = false;
     b->re = b->im = nullptr;
     b->images = nullptr;
     b->dInit = nullptr;
@@ -655,15 +644,6 @@ bool compileBatch(TrotterBatch* b) {
     size_t stateFloats = 0, imgTotal = 0;
     // the operand image parts the current precision and kernel choice read
     b->parts = tcImageParts();
-    // one program for all classes where each is small (the passes of the
-    // others, and split-FP16's, are launched one by one)
-    b->oneLaunch = tcDefaultAppliers() && C <= kSmallMaxSegs;
-    for (int c = 0; c < C; ++c) {
-        const TrotterClass& cl = b->classes[c];
-        b->oneLaunch = b->oneLaunch && ((uint64_t)cl.members.size() << cl.n) <= 1ull << kSmallMaxQubits;
-        for (const FusedPass& pass : planOf(c, 0).passes)
-            b->oneLaunch = b->oneLaunch && pass.controls.empty() && smallFits(cl.n, pass.targets);
-    }
     int pos = 0, slots = 0;
     std::vector<float> coef;                       // [class][reduction][member][kCoefs]
     for (int c = 0; c < C; ++c) {
@@ -681,7 +661,7 @@ bool compileBatch(TrotterBatch* b) {
             cl.shape.push_back(widenNarrow(planOf(c, 0).passes[p], cl.n));
             cl.imgStride[p] = tcImageFloats((int)cl.shape[p].targets.size(), b->parts);
             cl.imgOffset[p] = imgTotal;
-            if (!b->oneLaunch) imgTotal += cl.imgStride[p] * M;
+            imgTotal += cl.imgStride[p] * M;
         }
         cl.slotBase = slots;
         cl.coefOffset = coef.size();
@@ -694,31 +674,7 @@ bool compileBatch(TrotterBatch* b) {
         cl.redOffset = reds.size();
         reds.insert(reds.end(), cl.reds.begin(), cl.reds.end());
     }
-    // operand images of every (class, pass, member), on host threads; in one
-    // program step p holds pass p of every class that has one
-    std::vector<std::vector<size_t>> matOf(C);     // per class and pass: member 0's matrix
-    if (b->oneLaunch) {
-        size_t steps = 0;
-        uint64_t amps = 0;                         // over all steps
-        for (int c = 0; c < C; ++c) {
-            const TrotterClass& cl = b->classes[c];
-            steps = std::max(steps, cl.shape.size());
-            amps += ((uint64_t)cl.members.size() << cl.n) * cl.shape.size();
-            matOf[c].resize(cl.shape.size());
-        }
-        b->small.groups = smallGroups(amps / std::max<size_t>(steps, 1));
-        b->small.first.push_back(0);
-        for (size_t p = 0; p < steps; ++p) {
-            for (int c = 0; c < C; ++c) {
-                const TrotterClass& cl = b->classes[c];
-                if (p >= cl.shape.size()) continue;
-                matOf[c][p] = imgTotal;
-                imgTotal = smallAddPass(b->small, planOf(c, 0).passes[p], cl.n, cl.stateOffset, (int)cl.members.size(), imgTotal);
-            }
-            b->small.first.push_back((int)b->small.segs.size());
-        }
-        b->oneLaunch = steps > 0;
-    }
+    // operand images of every (class, pass, member), on host threads
     std::vector<float> host(std::max<size_t>(imgTotal, 4));
     std::vector<std::tuple<int, int, int>> imgJobs;            // class, pass, member
     for (int c = 0; c < C; ++c)
@@ -727,10 +683,6 @@ bool compileBatch(TrotterBatch* b) {
     parallelFor(imgJobs.size(), std::min(hw, 16u), [&](size_t j) {
         const int c = std::get<0>(imgJobs[j]), p = std::get<1>(imgJobs[j]), m = std::get<2>(imgJobs[j]);
         const TrotterClass& cl = b->classes[c];
-        if (b->oneLaunch) {
-            smallMatrix(planOf(c, m).passes[p], cl.n, host.data() + matOf[c][p] + m * kSmallMatrixFloats);
-            return;
-        }
         tcBuildImage(widenNarrow(planOf(c, m).passes[p], cl.n), host.data() + cl.imgOffset[p] + m * cl.imgStride[p],
                      b->parts);
     });
@@ -740,9 +692,7 @@ bool compileBatch(TrotterBatch* b) {
     for (int k = 0; k < B; ++k) init[b->classes[b->classOf[k]].posBase + b->posOf[k]] = b->inst[k].init;
     if (QG_CUDA(cudaMalloc(&b->re, stateFloats * sizeof(float)), kFn) ||
         QG_CUDA(cudaMalloc(&b->im, stateFloats * sizeof(float)), kFn) ||
-        (b->oneLaunch ? !smallUpload(b->small, host.data(), imgTotal, kFn)
-                      : QG_CUDA(cudaMalloc(&b->images, host.size() * sizeof(float)), kFn) ||
-                            QG_CUDA(cudaMemcpyAsync(b->images, host.data(), host.size() * sizeof(float), cudaMemcpyHostToDevice, st), kFn)) ||
+        QG_CUDA(cudaMalloc(&b->images, host.size() * sizeof(float)), kFn) ||
         QG_CUDA(cudaMalloc(&b->dInit, B * sizeof(long long)), kFn) ||
         QG_CUDA(cudaMalloc(&b->dCoef, std::max<size_t>(1, coef.size()) * sizeof(float)), kFn) ||
         QG_CUDA(cudaMalloc(&b->dReds, std::max<size_t>(1, reds.size()) * sizeof(Red)), kFn) ||
@@ -753,7 +703,8 @@ bool compileBatch(TrotterBatch* b) {
     if (QG_CUDA(cudaMemcpyAsync(b->dReds, reds.data(), reds.size() * sizeof(Red), cudaMemcpyHostToDevice, st), kFn) ||
         QG_CUDA(cudaMemsetAsync(b->dTickets, 0, std::max(1, b->numSlots) * sizeof(unsigned int), st), kFn))
         return false;
-    if (QG_CUDA(cudaMemcpyAsync(b->dInit, init.data(), B * sizeof(long long), cudaMemcpyHostToDevice, st), kFn) ||
+    if (QG_CUDA(cudaMemcpyAsync(b->images, host.data(), host.size() * sizeof(float), cudaMemcpyHostToDevice, st), kFn) ||
+        QG_CUDA(cudaMemcpyAsync(b->dInit, init.data(), B * sizeof(long long), cudaMemcpyHostToDevice, st), kFn) ||
         QG_CUDA(cudaMemcpyAsync(b->dCoef, coef.data(), coef.size() * sizeof(float), cudaMemcpyHostToDevice, st), kFn) ||
         QG_CUDA(cudaStreamSynchronize(st), kFn))
         return false;
@@ -761,14 +712,46 @@ bool compileBatch(TrotterBatch* b) {
     return true;
 }
 
-// the run's work, queued on `st` (the library stream, or a capture stream):
-// class after class, its states' initialisation and its passes (one launch each
-// over the class's states, or one launch for all passes of all classes), then
-// its reductions (one launch each over the class's states), then one copy of
-// every result to pinned host memory
-bool queueRun(TrotterBatch* b, cudaStream_t st) {
+// The run's work: class after class, its states' initialisation, its passes
+// (one launch each over the class's states) and its reductions, then one copy
+// of every result to pinned host memory.  Queued on `st`; while `st` is being
+// captured into a graph each class goes to a branch of its own, so that the
+// classes run side by side (a pass over three 16-qubit states is 24 CTAs):
+// nine instances of 10, 20 and 100 steps 3.80 ms one class after the other,
+// 2.47 ms so, with the same bits.
+struct Branches {                    // (alive until the capture has ended)
+    cudaEvent_t start = nullptr;
+    std::vector<cudaStream_t> st;
+    std::vector<cudaEvent_t> done;
+    ~Branches() {
+        if (start) cudaEventDestroy(start);
+        for (cudaEvent_t e : done) cudaEventDestroy(e);
+        for (cudaStream_t s : st) cudaStreamDestroy(s);
+    }
+    bool open(size_t count, cudaStream_t from) {
+        if (QG_CUDA(cudaEventCreateWithFlags(&start, cudaEventDisableTiming), kFn) || QG_CUDA(cudaEventRecord(start, from), kFn))
+            return false;
+        for (size_t k = 0; k < count; ++k) {
+            cudaStream_t s = nullptr;
+            cudaEvent_t e = nullptr;
+            if (QG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), kFn)) return false;
+            st.push_back(s);
+            if (QG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), kFn)) return false;
+            done.push_back(e);
+            if (QG_CUDA(cudaStreamWaitEvent(s, start, 0), kFn)) return false;
+        }
+        return true;
+    }
+};
+bool queueRun(TrotterBatch* b, cudaStream_t st, Branches* branches) {
     if (QG_CUDA(cudaMemsetAsync(b->errFlag, 0, sizeof(int), st), kFn)) return false;
-    for (const TrotterClass& cl : b->classes) {
+    const size_t C = b->classes.size();
+    const bool fork = branches && C > 1 && C <= 16;
+    if (fork && !branches->open(C, st)) return false;
+    const cudaStream_t whole = st;
+    for (size_t c = 0; c < b->classes.size(); ++c) {
+        const TrotterClass& cl = b->classes[c];
+        const cudaStream_t st = fork ? branches->st[c] : whole;
         const int M = (int)cl.members.size();
         const uint64_t dim = 1ull << cl.n, all = dim * (uint64_t)M;
         float* re = b->re + cl.stateOffset;
@@ -778,34 +761,26 @@ bool queueRun(TrotterBatch* b, cudaStream_t st) {
             return false;
         kBatchClassical<<<(M + 127) / 128, 128, 0, st>>>(re, dim, b->dInit + cl.posBase, M);
         if (launchFailed(kFn)) return false;
-        for (size_t p = 0; p < cl.shape.size() && !b->oneLaunch; ++p)
+        for (size_t p = 0; p < cl.shape.size(); ++p)
             if (!applyPassTCBatch(re, im, cl.n, cl.shape[p], b->images + cl.imgOffset[p], cl.imgStride[p], b->parts, M,
                                   b->errFlag, st)) {
                 invalidQuESTInputError("A pass of the Trotter batch could not be launched on the tensor cores.", kFn);
                 return false;
             }
-    }
-    if (b->oneLaunch &&
-        !smallLaunch(b->small, b->re, b->im, 0, (int)b->small.first.size() - 1, b->errFlag, st, kFn))
-        return false;
-    for (const TrotterClass& cl : b->classes) {
-        const int M = (int)cl.members.size();
-        const uint64_t dim = 1ull << cl.n;
-        const float* re = b->re + cl.stateOffset;
-        const float* im = b->im + cl.stateOffset;
         double* partials = b->partials + (size_t)cl.posBase * kMaxBlocksPerInst;
         unsigned int* counters = b->counters + cl.posBase;
         const int R = (int)cl.reds.size();
-        if (b->oneLaunch && R <= 64) {
+        bool reduced = false;
+        if (all <= 1ull << 20 && R <= 64) {
             // enough blocks for the widest reduction; an instance's partials hold R x bx
             const unsigned bx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(kMaxBlocksPerInst / R, dim / 2 / (4 * red::kThreads)));
             kReduceAll<<<dim3(bx, (unsigned)M, (unsigned)R), red::kThreads, 0, st>>>(
                 re, im, dim, b->dReds + cl.redOffset, b->dCoef + cl.coefOffset, partials, b->dTickets + cl.slotBase,
                 b->dResults + 2 * (size_t)cl.slotBase);
             if (launchFailed(kFn)) return false;
-            continue;
+            reduced = true;
         }
-        for (size_t l = 0; l < cl.reds.size(); ++l) {
+        for (size_t l = 0; l < cl.reds.size() && !reduced; ++l) {
             const Red& r = cl.reds[l];
             const float* coef = b->dCoef + cl.coefOffset + l * (size_t)M * kCoefs;
             double* out = b->dResults + 2 * ((size_t)cl.slotBase + l * (size_t)M);
@@ -828,6 +803,10 @@ bool queueRun(TrotterBatch* b, cudaStream_t st) {
             if (launchFailed(kFn)) return false;
         }
     }
+    for (size_t c = 0; fork && c < C; ++c)
+        if (QG_CUDA(cudaEventRecord(branches->done[c], branches->st[c]), kFn) ||
+            QG_CUDA(cudaStreamWaitEvent(whole, branches->done[c], 0), kFn))
+            return false;
     return !QG_CUDA(cudaMemcpyAsync(b->hResults, b->dResults, 2 * (size_t)b->numSlots * sizeof(double),
                                     cudaMemcpyDeviceToHost, st), kFn);
 }
@@ -951,7 +930,7 @@ int quest_gb300_trotterBatchRun(void* batch, double* energies) {
     TrotterBatch* b = reinterpret_cast<TrotterBatch*>(batch);
     if (!b) return -1;
     // images built for another precision or kernel choice are rebuilt
-    if (b->compiled && (((qg::tcImageParts() & ~b->parts) != 0 && !b->oneLaunch) || (b->oneLaunch && !qg::tcDefaultAppliers()))) {
+    if (b->compiled && (qg::tcImageParts() & ~b->parts) != 0) {
         cudaStreamSynchronize(qg::stream());
         qg::freeDevice(b);
     }
@@ -964,13 +943,12 @@ int quest_gb300_trotterBatchRun(void* batch, double* energies) {
         if (QG_CUDA(cudaGraphLaunch(b->exec, st), fn)) return -1;
         qg::g_launches.fetch_add(1);
     } else {
-        if (!qg::queueRun(b, st)) return -1;
+        if (!qg::queueRun(b, st, nullptr)) return -1;
     }
     if (QG_CUDA(cudaStreamSynchronize(st), fn)) return -1;
     int err = 0;
     if (QG_CUDA(cudaMemcpy(&err, b->errFlag, sizeof(int), cudaMemcpyDeviceToHost), fn)) return -1;
     if (err) {
-        if (b->oneLaunch) qg::smallReset(b->small);
         invalidQuESTInputError(err == 6 ? "A split-FP16 tensor-core pass of the Trotter batch gave a non-finite output."
                                         : "A tensor-core pass of the Trotter batch timed out waiting on its pipeline.",
                                fn);
@@ -989,9 +967,10 @@ int quest_gb300_trotterBatchRun(void* batch, double* energies) {
         // later runs replay the same work as one graph
         cudaStream_t cap = nullptr;
         if (!QG_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking), fn)) {
+            qg::Branches branches;
             bool ok = !QG_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal), fn);
             if (ok) {
-                const bool queued = qg::queueRun(b, cap);
+                const bool queued = qg::queueRun(b, cap, &branches);
                 ok = !QG_CUDA(cudaStreamEndCapture(cap, &b->graph), fn) && queued;
             }
             if (ok) ok = !QG_CUDA(cudaGraphInstantiate(&b->exec, b->graph, 0), fn);
