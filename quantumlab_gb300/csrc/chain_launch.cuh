@@ -33,7 +33,8 @@ __device__ __forceinline__ void chainStart() {
 // memory that is not used keeps an SM to the even share.
 inline size_t evenShare(unsigned blocks) {
     const unsigned sms = (unsigned)numSMs(), each = (blocks + sms - 1) / sms;
-    return 2 * blocks > sms && each <= 4 ? 220 * 1024 / each - 2048 : 0;
+    // each + 1 such blocks do not fit 228 KB, and one leaves 27 KB for a kernel's own
+    return 2 * blocks > sms && each <= 4 ? 200 * 1024 / each : 0;
 }
 
 template <class... Params, class... Args>
