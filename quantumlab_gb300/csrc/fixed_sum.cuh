@@ -7,10 +7,9 @@
 // total becomes a double.  An aligned value is within 2^-55 of the group's
 // largest, so a product's error is below the rounding of an FP64
 // multiply-add on the group's largest product.  Groups are the four amplitudes
-// of a thread's item: total probability at 24 qubits 86 -> 43 us, probability
-// of one outcome 49 -> 29, inner product 163 -> 121 (two states to read, floor
-// 79).  Leaving some warps in FP64, as the gates do, lost here: the slower
-// warps of a fixed share end last (29 us with none, 35 to 38 with one in 6 to 2).
+// of a thread's item.  On a dense state of 26 qubits, the whole call (HBM floors
+// 158, 79, 316): total probability 319 us -> 203, probability of one outcome 174
+// -> 116, inner product 615 -> 500.
 #pragma once
 
 #include <stdint.h>
@@ -21,16 +20,23 @@ namespace fsum {
 // exponent field of the largest of some values, from the high words
 __device__ __forceinline__ uint32_t magnitude(double x) { return (uint32_t)__double2hiint(x) & 0x7FFFFFFFu; }
 
-// x 2^(1076 - E) rounded to an integer below 2^54, as h 2^27 + l with x's sign
-__device__ __forceinline__ int2 digits(double x, int E) {
+// |x| 2^(1076 - E) rounded to an integer below 2^54, as h 2^27 + l.  (Not
+// through fabs, which is an instruction of the FP64 pipe: eight of them an item
+// left the norm of a dense state at 26 qubits FP64-bound, 338 us; 213 without.)
+__device__ __forceinline__ int2 absDigits(double x, int E) {
     const uint32_t hi = (uint32_t)__double2hiint(x);
     const int e = (int)(hi >> 20) & 0x7FF;
     const uint64_t m = ((uint64_t)((hi & 0xFFFFFu) | (e ? 0x100000u : 0u)) << 32) | (uint32_t)__double2loint(x);
     uint64_t t;                                  // the shift gives 0 from 64 up
     asm("shr.u64 %0, %1, %2;" : "=l"(t) : "l"(m << 11), "r"(E - max(e, 1) + 9));
     t = (t + 1) >> 1;
-    const int s = ((int)hi >> 31) | 1;
-    return make_int2((int)(t >> 27) * s, (int)((uint32_t)t & 0x7FFFFFFu) * s);
+    return make_int2((int)(t >> 27), (int)((uint32_t)t & 0x7FFFFFFu));
+}
+// the same with x's sign
+__device__ __forceinline__ int2 digits(double x, int E) {
+    const int s = (__double2hiint(x) >> 31) | 1;
+    const int2 d = absDigits(x, E);
+    return make_int2(d.x * s, d.y * s);
 }
 __device__ __forceinline__ int64_t mad(int a, int b, int64_t c) { return c + (int64_t)a * b; }
 
@@ -54,12 +60,20 @@ struct Sums {                                    // h h, h l + l h, l l; at most
 __device__ __forceinline__ double unit(int a, int b) { return __hiloint2double((a + b - 1080) << 20, 0); }
 __device__ __forceinline__ bool unitFits(int a, int b) { return a + b > 1080 && a + b < 3000 && max(a, b) < 0x7FF; }
 
-__device__ __forceinline__ bool allZero(double2 a, double2 b) { return a.x == 0.0 && a.y == 0.0 && b.x == 0.0 && b.y == 0.0; }
+__device__ __forceinline__ uint32_t lowWords(double2 a, double2 b) {
+    return (uint32_t)(__double2loint(a.x) | __double2loint(a.y) | __double2loint(b.x) | __double2loint(b.y));
+}
 
 // sum of squares of eight values
 static __device__ __noinline__ double squaresFp64(double2 a, double2 b, double2 c, double2 d) {
     return a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y + c.x * c.x + c.y * c.y + d.x * d.x + d.y * d.y;
 }
+// One warp in kFp64Share stays in FP64, so that both kinds of pipe work (after
+// the zeros are told, which cost neither): the norm of a dense state at 26
+// qubits 203, 217, 231 us with one in 4, 8 and none; inner products are best
+// with none.
+constexpr unsigned kFp64Share = 4;
+__device__ __forceinline__ bool fp64Warp() { return ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) % kFp64Share == 0; }
 // acc plus it
 __device__ __forceinline__ double addSquares(double acc, double2 a, double2 b, double2 c, double2 d) {
     const double v[8] = {a.x, a.y, b.x, b.y, c.x, c.y, d.x, d.y};
@@ -71,11 +85,11 @@ __device__ __forceinline__ double addSquares(double acc, double2 a, double2 b, d
     }
     if ((top | any) == 0) return acc;
     const int E = (int)(top >> 20);
-    if (!unitFits(E, E)) return acc + squaresFp64(a, b, c, d);
+    if (!unitFits(E, E) || fp64Warp()) return acc + squaresFp64(a, b, c, d);
     int64_t hh = 0, x = 0, ll = 0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        const int2 t = digits(fabs(v[k]), E);
+        const int2 t = absDigits(v[k], E);
         hh = mad(t.x, t.x, hh);
         x = mad(t.x, t.y, x);
         ll = mad(t.y, t.y, ll);

@@ -22,28 +22,34 @@ namespace {
 using namespace red;
 
 // ------------------------------------------------------------------ functors
-// Sums of squares, four amplitudes an item on the integer pipes (fixed_sum.cuh).
-// First amplitudes of the pairs i, i + 1 and j, j + 1.
+// Sums of squares, four amplitudes an item on the integer pipes
+// (fixed_sum.cuh).  An item's amplitudes come from `items` apart, so that the
+// lanes of a warp read side by side whatever the target.
+struct Four {
+    double2 a, b, c, d;
+};
 struct Squares {
     const double *re, *im;
-    __device__ __forceinline__ double pairs(double acc, uint64_t i, uint64_t j) const {
-        return fsum::addSquares(acc, ld2(re + i), ld2(re + j), ld2(im + i), ld2(im + j));
-    }
+    uint64_t items;
+    __device__ __forceinline__ Four pairs(uint64_t i, uint64_t j) const { return Four{ld2(re + i), ld2(re + j), ld2(im + i), ld2(im + j)}; }
+    __device__ __forceinline__ double add(double acc, const Four& v) const { return fsum::addSquares(acc, v.a, v.b, v.c, v.d); }
 };
 struct NormSq4 : Squares {
-    __device__ __forceinline__ double operator()(double acc, uint64_t k) const { return pairs(acc, 4 * k, 4 * k + 2); }
+    __device__ __forceinline__ Four load(uint64_t k) const { return pairs(2 * k, 2 * (k + items)); }
 };
 struct ProbZero4 : Squares {       // target >= 1: the amplitudes with bit t clear
     int t;
-    __device__ __forceinline__ double operator()(double acc, uint64_t k) const {
-        return pairs(acc, ins0(4 * k, t), ins0(4 * k + 2, t));
-    }
+    __device__ __forceinline__ Four load(uint64_t k) const { return pairs(ins0(2 * k, t), ins0(2 * (k + items), t)); }
 };
 struct ProbZeroEven : Squares {    // target 0
-    __device__ __forceinline__ double operator()(double acc, uint64_t k) const {
-        const double *r = re + 8 * k, *m = im + 8 * k;
-        const double2 a = ld2(r), b = ld2(r + 2), c = ld2(r + 4), d = ld2(r + 6), e = ld2(m), f = ld2(m + 2), g = ld2(m + 4), h = ld2(m + 6);
-        return fsum::addSquares(acc, make_double2(a.x, b.x), make_double2(c.x, d.x), make_double2(e.x, f.x), make_double2(g.x, h.x));
+    __device__ __forceinline__ Four load(uint64_t k) const {
+        double x[4], y[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            x[u] = ld2(re + 2 * (k + u * items)).x;
+            y[u] = ld2(im + 2 * (k + u * items)).x;
+        }
+        return Four{make_double2(x[0], x[1]), make_double2(x[2], x[3]), make_double2(y[0], y[1]), make_double2(y[2], y[3])};
     }
 };
 struct NormSq1 {
@@ -78,14 +84,15 @@ __device__ __noinline__ double2 innerFp64(double2 a, double2 b, double2 c, doubl
 }
 struct Inner2 {
     const double *br, *bi, *kr, *ki;
-    __device__ __forceinline__ double2 operator()(double2 acc, uint64_t i) const {
-        const double2 a = ld2(br + 2 * i), b = ld2(bi + 2 * i), c = ld2(kr + 2 * i), d = ld2(ki + 2 * i);
+    __device__ __forceinline__ Four load(uint64_t i) const { return Four{ld2(br + 2 * i), ld2(bi + 2 * i), ld2(kr + 2 * i), ld2(ki + 2 * i)}; }
+    __device__ __forceinline__ double2 add(double2 acc, const Four& v) const {
+        const double2 a = v.a, b = v.b, c = v.c, d = v.d;
         using namespace fsum;
         const uint32_t wb = max(max(magnitude(a.x), magnitude(a.y)), max(magnitude(b.x), magnitude(b.y)));
         const uint32_t wk = max(max(magnitude(c.x), magnitude(c.y)), max(magnitude(d.x), magnitude(d.y)));
         const int E = (int)(wb >> 20), F = (int)(wk >> 20);
         // (a zero factor adds nothing, unless the other is infinite or NaN)
-        if ((wb == 0 && allZero(a, b) && F < 0x7FF) || (wk == 0 && allZero(c, d) && E < 0x7FF)) return acc;
+        if (((wb | lowWords(a, b)) == 0 && F < 0x7FF) || ((wk | lowWords(c, d)) == 0 && E < 0x7FF)) return acc;
         if (!unitFits(E, F)) {
             const double2 v = innerFp64(a, b, c, d);
             return make_double2(acc.x + v.x, acc.y + v.y);
@@ -277,7 +284,7 @@ __global__ void __launch_bounds__(1 << kLowQubits) kOutcomes(const double* __res
 double reduceTotalProbSV(SV s, const Scratch& w) {                 // replaces QuEST_gpu.cu:1649-1679
     double v = 0;
     const uint64_t n = 1ull << s.n;
-    if (n >= 4) runSum<double>(NormSq4{{s.re, s.im}}, n / 4, w, &v, nullptr, "calcTotalProb");
+    if (n >= 4) runSum<double>(NormSq4{{s.re, s.im, n / 4}}, n / 4, w, &v, nullptr, "calcTotalProb");
     else runReduce(NormSq1{s.re, s.im}, n, w, &v, nullptr, "calcTotalProb");
     return v;
 }
@@ -294,8 +301,8 @@ double reduceProbZeroSV(SV s, int t, const Scratch& w) {           // QuEST_gpu.
     double v = 0;
     const uint64_t half = 1ull << (s.n - 1);
     if (half < 4) runReduce(ProbZeroFew{s.re, s.im, t}, half, w, &v, nullptr, "calcProbOfOutcome");
-    else if (t >= 1) runSum<double>(ProbZero4{{s.re, s.im}, t}, half / 4, w, &v, nullptr, "calcProbOfOutcome");
-    else runSum<double>(ProbZeroEven{{s.re, s.im}}, half / 4, w, &v, nullptr, "calcProbOfOutcome");
+    else if (t >= 1) runSum<double>(ProbZero4{{s.re, s.im, half / 4}, t}, half / 4, w, &v, nullptr, "calcProbOfOutcome");
+    else runSum<double>(ProbZeroEven{{s.re, s.im, half / 4}}, half / 4, w, &v, nullptr, "calcProbOfOutcome");
     return v;
 }
 

@@ -102,24 +102,28 @@ __global__ void __launch_bounds__(kThreads) kReduce(F f, uint64_t nItems, double
     gridSum(ax.value(), ay.value(), partials, counter, result);
 }
 
-// f(acc, i) -> acc plus item i, T double or double2 (functors whose item is
-// worth several FP64 operations saved)
+// Sum of items (f.load(i), then f.add(acc, item)), T double or double2: the
+// next item's loads are on their way while an item is added.
 __device__ __forceinline__ double first(double v) { return v; }
 __device__ __forceinline__ double first(double2 v) { return v.x; }
 __device__ __forceinline__ double second(double) { return 0.0; }
 __device__ __forceinline__ double second(double2 v) { return v.y; }
 template <class T, class F>
-__global__ void __launch_bounds__(kThreads) kSum(F f, uint64_t nItems, double* __restrict__ partials,
+__global__ void __launch_bounds__(kThreads, 4) kSum(F f, uint64_t nItems, double* __restrict__ partials,
                                                  unsigned int* __restrict__ counter, double* __restrict__ result) {
-    T a{}, b{};
+    T acc{};
     const uint64_t stride = (uint64_t)gridDim.x * kThreads;
     uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
-    for (; i + stride < nItems; i += 2 * stride) {
-        a = f(a, i);
-        b = f(b, i + stride);
+    if (i < nItems) {
+        auto cur = f.load(i);
+        for (; i + stride < nItems; i += stride) {
+            const auto next = f.load(i + stride);
+            acc = f.add(acc, cur);
+            cur = next;
+        }
+        acc = f.add(acc, cur);
     }
-    if (i < nItems) a = f(a, i);
-    gridSum(first(a) + first(b), second(a) + second(b), partials, counter, result);
+    gridSum(first(acc), second(acc), partials, counter, result);
 }
 
 inline int reduceGrid(uint64_t nItems) {
@@ -145,8 +149,8 @@ inline bool runReduce(const F& f, uint64_t nItems, const Scratch& w, double* out
 }
 template <class T, class F>
 inline bool runSum(const F& f, uint64_t nItems, const Scratch& w, double* out0, double* out1, const char* caller) {
-    // six blocks an SM are resident (40 registers): one wave
-    const unsigned grid = (unsigned)std::min<uint64_t>(reduceGrid(nItems), 6ull * (uint64_t)numSMs());
+    // one wave
+    const unsigned grid = (unsigned)std::min<uint64_t>(reduceGrid(nItems), 4ull * (uint64_t)numSMs());
     kSum<T, F><<<grid, kThreads, 0, stream()>>>(f, nItems, w.partials, w.counter, w.host);
     return takeResult(w, out0, out1, caller);
 }
