@@ -1172,13 +1172,22 @@ void applyTrotterCircuit(Qureg q, PauliHamil h, qreal time, int order, int reps)
     for (int r = 0; r < reps; ++r) {
         symTrotter(terms, time / reps, order, seq);
         if (seq.size() < 4096 && r + 1 < reps) continue;
+        const qg::SV state = svg(q);
         const size_t rows = seq.size();
+        if (state.cap) {                     // queued one by one
+            for (const qg::PauliRotation& c : seq) {
+                qg::gatePauliRotation(state, 0, c.x, c.y, c.z, c.angle, 0);
+                if (q.isDensityMatrix) qg::gatePauliRotation(state, 0, c.x << s, c.y << s, c.z << s, c.angle, 1);
+            }
+            seq.clear();
+            continue;
+        }
         if (q.isDensityMatrix)
             for (size_t i = 0; i < rows; ++i) {
                 const qg::PauliRotation c = seq[i];
                 seq.push_back(qg::PauliRotation{c.x << s, c.y << s, c.z << s, c.angle, 1});
             }
-        qg::gatePauliSequence(svg(q), seq, q.firstLevelReduction + qg::kScratchDoubles);
+        qg::gatePauliSequence(state, seq, q.firstLevelReduction + qg::kScratchDoubles);
         seq.clear();
     }
 }

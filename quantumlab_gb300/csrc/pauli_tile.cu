@@ -448,10 +448,6 @@ double cost(const std::vector<PassPlan>& plan, const std::vector<Step>& steps, c
 
 void gatePauliSequence(SV s, const std::vector<PauliRotation>& seq, double* tables) {
     const char* caller = "applyTrotterCircuit";
-    if (s.cap) {
-        for (const PauliRotation& r : seq) gatePauliRotation(s, 0, r.x, r.y, r.z, r.angle, r.conj);
-        return;
-    }
     std::vector<Step> steps;
     merge(seq, steps);
     std::vector<Windows> win(steps.size());

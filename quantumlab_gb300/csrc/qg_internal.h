@@ -109,7 +109,7 @@ void gateRotateZ(SV s, uint64_t ctrl, uint64_t targ, double angle);
 // exp(-i angle/2 P) with P a Pauli string given by x/y/z masks, where ctrl bits set;
 // conj!=0 applies the elementwise conjugate operator.
 void gatePauliRotation(SV s, uint64_t ctrl, uint64_t xmask, uint64_t ymask, uint64_t zmask, double angle, int conj);
-// the same for a sequence without controls, many rotations per pass
+// the same at once (not captured) for a sequence without controls, many rotations per pass
 // (pauli_tile.cu); tables: kPhaseTableDoubles of the register's workspace
 struct PauliRotation { uint64_t x, y, z; double angle; int conj; };
 void gatePauliSequence(SV s, const std::vector<PauliRotation>& seq, double* tables);
