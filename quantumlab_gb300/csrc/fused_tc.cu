@@ -763,20 +763,35 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
     fenceBefore();
     __syncthreads();
     fenceAfter();
+    // The parameters' tables come from a cold constant cache, and a tile's base
+    // from a chain of them: 4000 of the 14,000 clocks of a pass with one tile a
+    // CTA.  Spent here, while the grid before still runs, 300 dependent passes
+    // over three 16-qubit states take 2.17 ms instead of 2.46.
+    const int rw = warp & 3;                             // warp within its role = TMEM lane quarter
+    const uint64_t laneA = p.laneOff[lane];
+    const uint32_t colBase = p.colLane[lane];
+    TileWalker<KQ> walk;
+    if (warp < kMmaWarp) {
+        const uint32_t skip = warp < kEpiWarp0 ? (S::SPLIT ? 0u : (uint32_t)(warp >> 2) / NCH) : (uint32_t)(warp - kEpiWarp0) >> 2;
+        if (cta + (uint64_t)skip * ncta < numTiles) walk.at(p, cta + (uint64_t)skip * ncta);
+        uint32_t touched = 0;
+#pragma unroll
+        for (int m = 0; m < 1 << (KQ - 2); ++m) touched ^= (uint32_t)p.warpOff[rw][m];
+#pragma unroll
+        for (int j = 0; j < 1 << KQ; j += 8) touched ^= p.colJ[j];
+        asm volatile("" ::"r"(touched));
+    }
     chainStart();                                        // the state, norms and new images are the grids' before
     // split-FP16: X's scale 2^xe before the split (the epilogue undoes it)
     const int xe = F16 ? f16XExp(nl) : 0;
     const float kXs = __int_as_float((127 + xe) << 23);
     const uint32_t tmem = tmemBase;
-    const int rw = warp & 3;                             // warp within its role = TMEM lane quarter
     const uint32_t laneSel = (uint32_t)(32 * rw) << 16;
     const uint32_t rowBase = padIdx(4u * lane);
 
     if (warp < kEpiWarp0) {
         // ------------------------------------------------ loaders
         const int g = warp >> 2;
-        const uint64_t laneA = p.laneOff[lane];
-        const uint32_t colBase = p.colLane[lane];
         // this CTA's chunks, in order: chunk s = (tile cta + (s / NCH) * ncta, K chunk s % NCH);
         // split: every s, part g; otherwise group g takes s = g, g + LG, ...
         const int p0 = S::SPLIT ? g : 0;
@@ -791,7 +806,6 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
         // 0, 1 are qubits 0, 1, so positions q = 4 lane + 128 m .. + 3 are four
         // consecutive amplitudes: one 16-byte copy to pad(q); a warp's copy
         // reads four 128-byte lines.
-        TileWalker<KQ> walk;
         // bulk staging: lane l < ROWS copies row l of each part, region
         // indices 32 l .. 32 l + 31 (qubits 0..4 are region bits 0..4, so a
         // row is 128 contiguous bytes in global memory; in the padded layout
@@ -964,8 +978,6 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
         // epilogue group eg drains accumulator eg, i.e. tiles tl with tl % EG == eg
         const int et = threadIdx.x - 32 * kEpiWarp0;
         const int eg = et >> 7;
-        const uint64_t laneA = p.laneOff[lane];
-        const uint32_t colBase = p.colLane[lane];
         float* const er = es + (size_t)(eg * 4 + rw) * R;
         // the drift correction: every output is scaled by 1 + sm1 in FP32
         // (split-BF16 parts of a rescaled G would carry the scale only to their
@@ -978,7 +990,6 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
         const float unscale = F16 ? __ldg(gImage + 2 * kGW) * __int_as_float((127 + kF16XExp - xe) << 23) : 1.f;
         uint32_t tl = eg;
         double normOut = 0.0;
-        TileWalker<KQ> walk;
         for (uint64_t tile = cta + (uint64_t)eg * ncta; tile < numTiles && ok;
              tile += (uint64_t)EG * ncta, tl += EG) {
             const uint64_t tb = walk.at(p, tile) + laneA;
