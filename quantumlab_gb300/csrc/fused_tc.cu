@@ -322,11 +322,12 @@ __device__ __forceinline__ void recordScale(const NormLinks& nl, float sm1, bool
 // ~3.99).
 __device__ __forceinline__ int f16XExp(const NormLinks& nl) {
     if (!nl.boundSq) return kF16XExp;
-    const double b = *nl.boundSq;
-    if (!(b > 0.0) || !(b < 1.0e300)) return kF16XExp;
-    int e = 0;
-    frexp(sqrt(b), &e);                                  // sqrt(b) < 2^e
-    return min(40, max(-40, 15 - e));
+    // b = m 2^E, m in [1/2, 1): sqrt(b) < 2^e, e = E / 2 rounded up.  Taken from
+    // b's bits: FP64 instructions (two lanes a clock) took 17 warps 2 us here.
+    const long long b = __double_as_longlong(*nl.boundSq);
+    if (b <= 0 || b >= __double_as_longlong(1.0e300)) return kF16XExp;     // not positive, NaN or too large
+    const int E = (int)(b >> 52) - 1022;
+    return min(40, max(-40, 15 - ((E + 1) >> 1)));
 }
 
 __device__ __forceinline__ double warpSumD(double v) {
@@ -741,6 +742,7 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
     __shared__ __align__(8) uint64_t stageB[kStageBars];   // bulk staging: [loader warp][row stage]
     __shared__ uint32_t tmemBase;
     __shared__ volatile int abortF;
+    __shared__ float drift;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     auto copyImage = [&]() {
@@ -980,8 +982,10 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
             if (lane == 0) atomicExch(errFlag, 3);
             abortF = 1;
         }
-        normIn = warpSumD(normIn);
-        if (lane == 0 && measure) atomicAdd(nl.in, normIn);
+        if (measure) {
+            normIn = warpSumD(normIn);
+            if (lane == 0) atomicAdd(nl.in, normIn);
+        }
     } else if (warp < kMmaWarp) {
         // ------------------------------------------------ epilogue
         // epilogue group eg drains accumulator eg, i.e. tiles tl with tl % EG == eg
@@ -992,8 +996,15 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
         // (split-BF16 parts of a rescaled G would carry the scale only to their
         // ~2^-17 precision, far coarser than the drift)
         bool ok = true;
-        const float sm1 = driftCorrection(nl);
-        recordScale(nl, sm1, blockIdx.x == 0 && et == 0);
+        // (one warp's FP64 work for all: two divisions and a root in each of eight
+        // warps took as long as the tile takes to come; 20 qubits 9.1 -> 8.5 us a pass)
+        if (warp == kEpiWarp0) {
+            const float c = driftCorrection(nl);
+            if (lane == 0) drift = c;
+            recordScale(nl, c, blockIdx.x == 0 && et == 0);
+        }
+        asm volatile("bar.sync 1, %0;" ::"n"(128 * EG) : "memory");
+        const float sm1 = drift;
         // split-FP16: 2^-(xe + s), s the scale of this CTA's matrix block (its
         // image records 2^-(14 + s) after the two parts)
         const float unscale = F16 ? __ldg(gImage + 2 * kGW) * __int_as_float((127 + kF16XExp - xe) << 23) : 1.f;
@@ -1070,8 +1081,10 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
         // split-FP16: an input beyond FP16's range after scaling gave a
         // non-finite output
         if (F16 && !(normOut <= 1.0e300)) atomicExch(errFlag, 6);
-        normOut = warpSumD(normOut);
-        if (lane == 0 && nl.out) atomicAdd(nl.out, normOut);
+        if (nl.out) {
+            normOut = warpSumD(normOut);
+            if (lane == 0) atomicAdd(nl.out, normOut);
+        }
     } else if (electOne()) {
         // ------------------------------------------------ TMA of G, then MMAs
         if (!nl.imageReady) copyImage();
