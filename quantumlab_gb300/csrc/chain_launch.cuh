@@ -37,11 +37,16 @@ inline size_t evenShare(unsigned blocks) {
     return 2 * blocks > sms && each <= 4 ? 200 * 1024 / each : 0;
 }
 
+// `cluster`: blocks to a thread-block cluster (of consecutive blocks in x)
 template <class... Params, class... Args>
-inline void chain(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
+inline void chainClusters(unsigned cluster, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                          Args&&... args) {
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -49,9 +54,13 @@ inline void chain(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
         (void)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     (void)cudaLaunchKernelEx(&cfg, kernel, Params(std::forward<Args>(args))...);     // its error: launchFailed
+}
+template <class... Params, class... Args>
+inline void chain(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+    chainClusters(1, kernel, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 }  // namespace qg

@@ -11,8 +11,9 @@ namespace qg {
 // Whether a plan runs as one program: the library chooses the applier, no
 // pass has control qubits, and the register is one where it wins.  Per pass,
 // with the launch and its wait, of an 8-layer random circuit, against the
-// tensor cores pass by pass: 16 qubits 3.4 us (10.6), 17 4.2 (10.5), 18 5.7
-// (10.5), 19 9.3 (10.6); 20 qubits 16.0 (10.1).
+// tensor cores pass by pass: 16 qubits 3.4 us (7.1), 17 4.2 (6.9), 18 5.7
+// (7.1), 19 9.3 (8.1); 20 qubits 16.0 (8.5).  19 qubits stay, for sums that
+// are nearer to 64 bits than split operands.
 constexpr int kSmallMaxQubits = 19;
 bool smallPlanFits(const FusedPlan& plan);
 // reuse: an earlier program, whose memory is taken over; null when it failed

@@ -563,6 +563,9 @@ struct TC2Params {
     // and has its own operand image, imageStride floats after the previous
     // one.  A single register: ctasPerInst = gridDim.x, the strides 0.
     uint32_t ctasPerInst;
+    // Pairs: clusters of two CTAs share a tile, CTA h forming plane h of its
+    // output (ctasPerInst then counts pairs, and is the number of tiles).
+    uint32_t pair;
     uint64_t instStride;
     uint64_t imageStride;
     // Controlled passes: 2^ctrlBits matrices, one per value c of the control
@@ -671,6 +674,13 @@ __host__ __device__ __forceinline__ uint64_t tileBase(const TC2Params<KQ>& p, ui
     }
     return tb;
 }
+// The shapes whose passes two CTAs can share (see TC2Params::pair): 6 qubits,
+// a loader group on each half of a chunk, two epilogue groups.
+template <int KQ, int LG, int EG, int LS>
+constexpr bool kPairs = KQ == 6 && LG == 2 && EG == 2 && LS == 2;
+__device__ __forceinline__ void clusterArrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void clusterWait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
 // Tile bases of one role's increasing tile sequence (tiles differ by
 // multiples of ctasPerInst).  The base is the tile index deposited into
 // outMask, and deposits add by masked addition:
@@ -706,9 +716,11 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
     constexpr bool BF = (PR == kPrecBF16), F16 = (PR == kPrecF16), H16 = BF || F16;
     // this CTA's register of a batch and control value, and its place among
     // the CTAs of that pair
-    const uint32_t cta = blockIdx.x % p.ctasPerInst, ncta = p.ctasPerInst;
+    const bool pair = kPairs<KQ, LG, EG, LS> && p.pair;
+    const uint32_t block = pair ? blockIdx.x >> 1 : blockIdx.x, half = pair ? blockIdx.x & 1u : 0u;
+    const uint32_t cta = block % p.ctasPerInst, ncta = p.ctasPerInst;
     {
-        const uint64_t u = blockIdx.x / p.ctasPerInst;
+        const uint64_t u = block / p.ctasPerInst;
         const uint64_t inst = u >> p.ctrlBits, cv = u & ((1u << p.ctrlBits) - 1u);
         re += inst * p.instStride + p.ctrlOff[cv];
         im += inst * p.instStride + p.ctrlOff[cv];
@@ -726,7 +738,8 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
     constexpr uint32_t kCols = kUsed <= 64 ? 64 : (kUsed <= 128 ? 128 : (kUsed <= 256 ? 256 : 512));
     static_assert(kUsed <= 512, "TMEM");
     constexpr uint32_t kLBO = 128;
-    constexpr uint32_t idesc = BF ? idescBF16(kTile, N) : F16 ? idescF16(kTile, N) : idescTF32(kTile, N);
+    constexpr uint32_t idescAll = BF ? idescBF16(kTile, N) : F16 ? idescF16(kTile, N) : idescTF32(kTile, N);
+    constexpr uint32_t idescPlane = BF ? idescBF16(kTile, D) : F16 ? idescF16(kTile, D) : idescTF32(kTile, D);
     constexpr int kEpiWarp0 = 4 * LG, kMmaWarp = 4 * (LG + EG);
     // loader groups split every chunk (S::SPLIT) or take alternate chunks
     static_assert(LS == 1 || LG == 2, "part-split loading needs two loader groups");
@@ -783,7 +796,7 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
     const uint32_t colBase = p.colLane[lane];
     TileWalker<KQ> walk;
     if (warp < kMmaWarp) {
-        const uint32_t skip = warp < kEpiWarp0 ? (S::SPLIT ? 0u : (uint32_t)(warp >> 2) / NCH) : (uint32_t)(warp - kEpiWarp0) >> 2;
+        const uint32_t skip = warp < kEpiWarp0 ? (S::SPLIT ? 0u : (uint32_t)(warp >> 2) / NCH) : pair ? 0u : (uint32_t)(warp - kEpiWarp0) >> 2;
         if (cta + (uint64_t)skip * ncta < numTiles) walk.at(p, cta + (uint64_t)skip * ncta);
         uint32_t touched = 0;
 #pragma unroll
@@ -799,6 +812,10 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
     const uint32_t tmem = tmemBase;
     const uint32_t laneSel = (uint32_t)(32 * rw) << 16;
     const uint32_t rowBase = padIdx(4u * lane);
+    // A tile is written where it was read: in a pair the epilogues wait until
+    // the loaders of both CTAs have it (the cluster's barrier, on which every
+    // other warp arrives by itself, whatever its outcome).
+    if (pair && warp == kMmaWarp) clusterArrive();
 
     if (warp < kEpiWarp0) {
         // ------------------------------------------------ loaders
@@ -810,7 +827,7 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
         const uint32_t nMy = cta < numTiles ? (uint32_t)((numTiles - 1 - cta) / ncta + 1) * NCH : 0u;
         const uint32_t nMine = nMy > s0 ? (nMy - s0 + sStep - 1) / sStep : 0u;     // chunks of this group
         double normIn = 0.0;
-        const bool measure = nl.in != nullptr;             // input norm wanted (uniform)
+        const bool measure = nl.in != nullptr && half == 0;    // input norm wanted (uniform)
         float* const wbuf = xs + (size_t)(g * 4 + rw) * XST * PPG * R;             // this warp's stages
         // Copy this group's parts of chunk sc into a stage (a k = 6 part is a
         // plane half: region indices < 1024 or >= 1024).  Region index bits
@@ -978,6 +995,7 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
         } else {
             cpAsyncWait<0>();                                // no copy in flight when the warp leaves
         }
+        if (pair) clusterArrive();
         if (!ok) {
             if (lane == 0) atomicExch(errFlag, 3);
             abortF = 1;
@@ -1008,9 +1026,15 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
         // split-FP16: 2^-(xe + s), s the scale of this CTA's matrix block (its
         // image records 2^-(14 + s) after the two parts)
         const float unscale = F16 ? __ldg(gImage + 2 * kGW) * __int_as_float((127 + kF16XExp - xe) << 23) : 1.f;
-        uint32_t tl = eg;
+        // a pair's tile: both groups, a part each
+        uint32_t tl = pair ? 0u : eg;
+        const int ep0 = pair ? 2 * (int)half + eg : 0, ep1 = pair ? ep0 + 1 : EPARTS;
+        if (pair) {
+            clusterArrive();
+            clusterWait();
+        }
         double normOut = 0.0;
-        for (uint64_t tile = cta + (uint64_t)eg * ncta; tile < numTiles && ok;
+        for (uint64_t tile = cta + (uint64_t)tl * ncta; tile < numTiles && ok;
              tile += (uint64_t)EG * ncta, tl += EG) {
             const uint64_t tb = walk.at(p, tile) + laneA;
             const int bd = tl & 1;
@@ -1025,7 +1049,7 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
             const float* const rb = er + rowBase;
             // (rolled at k = 6, whose four unrolled parts would not fit the registers)
 #pragma unroll(KQ == 6 ? 1 : EPARTS)
-            for (int ep = 0; ep < EPARTS; ++ep) {
+            for (int ep = KQ == 6 ? ep0 : 0; ep < (KQ == 6 ? ep1 : EPARTS); ++ep) {
                 // part ep: plane pl (output rows r = pl * D + j), matrix indices j = h * 32 + jj
                 const int pl = (KQ == 6) ? ep >> 1 : ep;
                 const int h = (KQ == 6) ? ep & 1 : 0;
@@ -1034,7 +1058,7 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
                 tmemLd16(dA + c0, va);
                 if (JP == 32) tmemLd16(dA + c0 + 16, vb);
                 tmemWaitLd();
-                if (ep == EPARTS - 1) {                              // accumulator drained
+                if (ep == (KQ == 6 ? ep1 : EPARTS) - 1) {            // accumulator drained
                     fenceBefore();
                     mbarArrive(&dEmptyB[bd]);
                 }
@@ -1099,7 +1123,8 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
                 break;
             }
             fenceAfter();
-            const uint32_t dT = tmem + kDCol0 + bd * N;
+            const uint32_t dT = tmem + kDCol0 + bd * N + half * (uint32_t)D;
+            const uint32_t idesc = pair ? idescPlane : idescAll;
             for (int ch = 0; ch < NCH; ++ch, ++sq) {
                 const int b = (int)(sq % NST);
                 if (!mbarWaitOrAbort(&fullB[b], (sq / NST) & 1, &abortF)) {
@@ -1116,7 +1141,7 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
                 // next 256 bytes of B: the descriptor's start field (address >> 4)
                 // advances by 16 per step
                 const uint32_t kEnt = (KQ == 6) ? 32u * (uint32_t)S::half(ch, 0) * (NCH == 4) : (uint32_t)(ch * KC);
-                const uint32_t gOff = ((KQ == 6 && S::plane(ch, 0) == 0) ? 8u * S::GSBO : 0u) + kEnt * S::ESZ / 16u * 128u;
+                const uint32_t gOff = ((KQ == 6 && S::plane(ch, 0) == 0) ? 8u * S::GSBO : 0u) + half * (D / 8 * S::GSBO) + kEnt * S::ESZ / 16u * 128u;
                 const uint64_t dH = smemDesc(ghA + gOff, kLBO, S::GSBO);
                 const uint64_t dL = smemDesc(glA + gOff, kLBO, S::GSBO);
                 const uint64_t dLL = smemDesc(gllA + gOff, kLBO, S::GSBO);
@@ -1164,6 +1189,7 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
         // drain: wait (bounded) for the last accumulator to finish before TMEM is freed
         if (tl > 0) mbarWaitOrAbort(&dFullB[(tl - 1) & 1], ((tl - 1) >> 1) & 1, &abortF);
     }
+    if (pair && (warp < kEpiWarp0 || warp == kMmaWarp)) clusterWait();
     fenceBefore();
     __syncthreads();
     fenceAfter();
@@ -1448,6 +1474,7 @@ bool tc2Params(int n, const FusedPass& pass, int batch, uint64_t instStride, uin
     grid = ctas * groups;
     p.outMask = ~imask & ~cmask;
     p.ctasPerInst = (uint32_t)ctas;
+    p.pair = 0;
     p.instStride = instStride;
     p.imageStride = imageStride;
     p.ctrlBits = (uint32_t)nctl;
@@ -1491,6 +1518,12 @@ bool launchTC2(float* re, float* im, int n, const FusedPass& pass, const float* 
     }
     img += partOff;
     p.ctrlImageStride = blockStride;
+    // Few tiles: two CTAs to each, as long as a pass and the next, whose CTAs
+    // come early, find an SM for each CTA.  A pass on so few tiles is one
+    // tile's latency, and half its MMAs and an epilogue part for each of four
+    // groups shorten it: 300 passes over three 16-qubit states 1905 -> 1607 us,
+    // split-FP16 passes on 16 qubits 7.6 -> 7.3 us, on 18 qubits 7.6 -> 7.2.
+    p.pair = kPairs<KQ, LG, EG, LS> && p.ctasPerInst == numTiles && 4 * grid <= (uint64_t)numSMs();
     static bool configured = false;
     if (!configured) {
         if (QG_CUDA(cudaFuncSetAttribute(kApplyTC2<KQ, LG, EG, LS, PR, CV, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
@@ -1498,7 +1531,7 @@ bool launchTC2(float* re, float* im, int n, const FusedPass& pass, const float* 
             return false;
         configured = true;
     }
-    chain(kApplyTC2<KQ, LG, EG, LS, PR, CV, ST>, (unsigned)grid, (4 * (LG + EG) + 1) * 32, smem, st, re, im, img, numTiles, errFlag, nl, p);
+    chainClusters(p.pair ? 2 : 1, kApplyTC2<KQ, LG, EG, LS, PR, CV, ST>, (unsigned)grid << p.pair, (4 * (LG + EG) + 1) * 32, smem, st, re, im, img, numTiles, errFlag, nl, p);
     return !launchFailed("applyPlanF32");
 }
 

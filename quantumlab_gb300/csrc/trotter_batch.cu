@@ -718,7 +718,7 @@ bool compileBatch(TrotterBatch* b) {
 // captured into a graph each class goes to a branch of its own, so that the
 // classes run side by side (a pass over three 16-qubit states is 24 CTAs):
 // nine instances of 10, 20 and 100 steps 3.80 ms one class after the other,
-// 1.91 ms so, with the same bits.
+// 1.61 ms so, with the same bits.
 struct Branches {                    // (alive until the capture has ended)
     cudaEvent_t start = nullptr;
     std::vector<cudaStream_t> st;
