@@ -9,6 +9,11 @@
 // grids before it have ended and their writes are visible.  Every access of
 // global memory stands behind that wait, so the order of the stream is kept;
 // work that is launched plainly before or after orders as always.
+// A chained kernel's pointers are not __restrict__ and it does not use __ldg:
+// either lets the compiler read through the non-coherent path, which holds
+// only for data that stays unchanged while the kernel is resident, or move a
+// load to before the wait.  Both kinds of block are resident while the grid
+// before still writes (phase tables, pass products, operand images, the state).
 // From gate to gate, 16 qubits 4.1 -> 2.5 us, 20 qubits: compactUnitary 10.4
 // -> 8.5, rotations 8.3 -> 6.2, phases 6.2 -> 4.2; a 9-qubit circuit of 70
 // calls 285 -> 164 us, now bound by the calls.

@@ -106,10 +106,9 @@ __device__ __forceinline__ void addPairs(const PairLoop& o, const int2* sr, cons
     }
 }
 
-__global__ void __launch_bounds__(kThreads) kExpecTile(const double* __restrict__ re, const double* __restrict__ im,
+__global__ void __launch_bounds__(kThreads) kExpecTile(const double* re, const double* im,
                                                        uint64_t tiles, const __grid_constant__ ExpecPass p,
-                                                       double* __restrict__ partials, unsigned* __restrict__ counter,
-                                                       double* __restrict__ result) {
+                                                       double* partials, unsigned* counter, double* result) {
     extern __shared__ int2 sm[];
     __shared__ int shE[kWarps];
     __shared__ float shS[kWarps];

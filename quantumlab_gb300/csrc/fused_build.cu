@@ -91,9 +91,8 @@ __device__ __forceinline__ void applyGate(double2* m, const double2* u, const De
 }
 
 // products: D x D entries of pass p from p * 4096 on, row-major
-__global__ void __launch_bounds__(kThreads) kProducts(const DevPass* __restrict__ passes, const DevGate* __restrict__ gates,
-                                                      const double2* __restrict__ entries, double2* __restrict__ products,
-                                                      unsigned long long* __restrict__ largest) {
+__global__ void __launch_bounds__(kThreads) kProducts(const DevPass* passes, const DevGate* gates,
+                                                      const double2* entries, double2* products, unsigned long long* largest) {
     constexpr int kMaxEntries = 1 << (2 * kMaxGateQubits);
     __shared__ double2 m[64 * 64 / kSlices];
     __shared__ double2 entry[2][kMaxEntries];      // this gate's, the next one's
@@ -144,8 +143,8 @@ __device__ __forceinline__ size_t kMajor(int r, int j, int K) {        // packKM
     return (size_t)(r / 8) * (K / 4) * 32 + (size_t)(j / 4) * 32 + (r % 8) * 4 + j % 4;
 }
 
-__global__ void __launch_bounds__(kThreads) kImages(const DevPass* __restrict__ passes, const double2* __restrict__ products,
-                                                    const unsigned long long* __restrict__ largest, float* __restrict__ out) {
+__global__ void __launch_bounds__(kThreads) kImages(const DevPass* passes, const double2* products,
+                                                    const unsigned long long* largest, float* out) {
     chainStart();
     const DevPass p = passes[blockIdx.x];
     const int D = 1 << p.k, N = 2 * D;

@@ -708,9 +708,9 @@ struct TileWalker {
 // global memory and in the padded shared layout) per lane and part,
 // completing on one mbarrier per warp and row stage.
 template <int KQ, int LG, int EG, int LS, int PR, int CV, int ST>
-__global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* __restrict__ re, float* __restrict__ im,
-                                                                  const float* __restrict__ gImage, uint64_t numTiles,
-                                                                  int* __restrict__ errFlag, const NormLinks nl,
+__global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* re, float* im,
+                                                                  const float* gImage, uint64_t numTiles,
+                                                                  int* errFlag, const NormLinks nl,
                                                                   const __grid_constant__ TC2Params<KQ> p) {
     using S = TC2Shape<KQ, LG, EG, LS, PR>;
     constexpr bool BF = (PR == kPrecBF16), F16 = (PR == kPrecF16), H16 = BF || F16;
@@ -1025,7 +1025,7 @@ __global__ void __launch_bounds__((4 * (LG + EG) + 1) * 32, 1) kApplyTC2(float* 
         const float sm1 = drift;
         // split-FP16: 2^-(xe + s), s the scale of this CTA's matrix block (its
         // image records 2^-(14 + s) after the two parts)
-        const float unscale = F16 ? __ldg(gImage + 2 * kGW) * __int_as_float((127 + kF16XExp - xe) << 23) : 1.f;
+        const float unscale = F16 ? gImage[2 * kGW] * __int_as_float((127 + kF16XExp - xe) << 23) : 1.f;
         // a pair's tile: both groups, a part each
         uint32_t tl = pair ? 0u : eg;
         const int ep0 = pair ? 2 * (int)half + eg : 0, ep1 = pair ? ep0 + 1 : EPARTS;

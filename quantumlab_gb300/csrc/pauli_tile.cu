@@ -77,7 +77,7 @@ struct TableSpec {
 
 // Tables (1 + grow) exp(-i sum_k (-1)^popc(index & mask_k) phi_k); the sum is
 // compensated (TwoSum), so an entry is as good as one sincos of the exact sum.
-__global__ void __launch_bounds__(kThreads) kPhaseTables(const __grid_constant__ TableSpec ts, double2* __restrict__ tab) {
+__global__ void __launch_bounds__(kThreads) kPhaseTables(const __grid_constant__ TableSpec ts, double2* tab) {
     chainStart();
     const int w = blockIdx.y;
     const uint32_t i = blockIdx.x * kThreads + threadIdx.x;
@@ -109,9 +109,9 @@ __device__ __forceinline__ void rotate(double& x, double& y, double t, double s,
 }
 __device__ __forceinline__ uint32_t insert0(uint32_t k, int b) { return ((k >> b) << (b + 1)) | (k & ((1u << b) - 1u)); }
 
-__global__ void __launch_bounds__(kThreads) kPauliTile(double* __restrict__ re, double* __restrict__ im,
+__global__ void __launch_bounds__(kThreads) kPauliTile(double* re, double* im,
                                                        const __grid_constant__ TilePass p,
-                                                       const double2* __restrict__ tables) {
+                                                       const double2* tables) {
     extern __shared__ double2 sm[];
     const int b = p.b;
     const uint32_t size = 1u << b;
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kThreads) kPauliTile(double* __restrict__ re, 
                         const uint32_t bit = win.local[k] != 255 ? l >> win.local[k] : (uint32_t)(base >> win.pos[k]);
                         idx |= (bit & 1u) << k;
                     }
-                    const double2 f = __ldg(tables + ((size_t)w << kWindowBits) + idx);
+                    const double2 f = tables[((size_t)w << kWindowBits) + idx];
                     if (w == op.w0) {
                         fr = f.x;
                         fi = f.y;

@@ -200,7 +200,7 @@ struct PauliMix {
 
 // row bit t >= 1: two consecutive groups per thread with double2 loads
 template <class Op>
-__global__ void __launch_bounds__(kThreads) kChannelVec(double* __restrict__ re, double* __restrict__ im, int t, int N,
+__global__ void __launch_bounds__(kThreads) kChannelVec(double* re, double* im, int t, int N,
                                                         uint64_t nThreads, Op op) {
     const uint64_t k = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (k >= nThreads) return;
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kThreads) kChannelVec(double* __restrict__ re,
 
 // row bit t == 0: (e00, e01) and (e10, e11) are adjacent pairs
 template <class Op>
-__global__ void __launch_bounds__(kThreads) kChannelT0(double* __restrict__ re, double* __restrict__ im, int N,
+__global__ void __launch_bounds__(kThreads) kChannelT0(double* re, double* im, int N,
                                                        uint64_t nGroups, Op op) {
     const uint64_t k = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (k >= nGroups) return;
@@ -261,7 +261,7 @@ struct TwoQubitBits {
     int b[4];
 };
 template <int V, bool MIX>
-__global__ void __launch_bounds__(kThreads) kTwoQubitChannel(double* __restrict__ re, double* __restrict__ im,
+__global__ void __launch_bounds__(kThreads) kTwoQubitChannel(double* re, double* im,
                                                              const TwoQubitBits tb, uint64_t nThreads, double retain,
                                                              double diagRetain, double mix) {
     typedef typename std::conditional<V == 2, double2, double>::type vec;

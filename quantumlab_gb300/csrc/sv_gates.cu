@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kThreads, 6) kPairVec(double* re, double* im, 
 
 // partner bit is bit 0: (re[i0], re[i0+1]) is one pair; two pairs per thread
 template <bool CROSS, class Op>
-__global__ void __launch_bounds__(kThreads) kPairAdj(double* __restrict__ re, double* __restrict__ im, InsSpec ins,
+__global__ void __launch_bounds__(kThreads) kPairAdj(double* re, double* im, InsSpec ins,
                                                      uint64_t setMask, uint64_t nThreads, Op op) {
     const uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (t >= nThreads) return;
@@ -308,7 +308,7 @@ struct OpTurnFixed {
 };
 
 template <class Op>
-__global__ void __launch_bounds__(kThreads) kDiagVec(double* __restrict__ re, double* __restrict__ im, InsSpec ins,
+__global__ void __launch_bounds__(kThreads) kDiagVec(double* re, double* im, InsSpec ins,
                                                      uint64_t setMask, uint64_t nThreads, Op op) {
     const uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (t >= nThreads) return;
@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kThreads) kDiagVec(double* __restrict__ re, do
 }
 
 template <class Op>
-__global__ void __launch_bounds__(kThreads) kDiagScalar(double* __restrict__ re, double* __restrict__ im, InsSpec ins,
+__global__ void __launch_bounds__(kThreads) kDiagScalar(double* re, double* im, InsSpec ins,
                                                         uint64_t setMask, uint64_t nAmps, Op op) {
     const uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (t >= nAmps) return;
@@ -378,7 +378,7 @@ __device__ __forceinline__ void pauliPair(const PauliRot& p, uint64_t j, double&
     kr = p.c * br + sk * gar; ki = p.c * bi + sk * gai;
 }
 
-__global__ void __launch_bounds__(kThreads) kPauliRotVec(double* __restrict__ re, double* __restrict__ im, InsSpec ins,
+__global__ void __launch_bounds__(kThreads) kPauliRotVec(double* re, double* im, InsSpec ins,
                                                          uint64_t setMask, uint64_t nThreads, PauliRot p) {
     const uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (t >= nThreads) return;
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kThreads) kPauliRotVec(double* __restrict__ re
     st2(re + j0, jr); st2(im + j0, ji); st2(re + k0, kr); st2(im + k0, ki);
 }
 
-__global__ void __launch_bounds__(kThreads) kPauliRotScalar(double* __restrict__ re, double* __restrict__ im, InsSpec ins,
+__global__ void __launch_bounds__(kThreads) kPauliRotScalar(double* re, double* im, InsSpec ins,
                                                             uint64_t setMask, uint64_t nPairs, PauliRot p) {
     const uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (t >= nPairs) return;
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kThreads) kPauliRotScalar(double* __restrict__
 }
 
 // ------------------------------------------------------- swap (QuEST_gpu.cu:1737-1769)
-__global__ void __launch_bounds__(kThreads) kSwap(double* __restrict__ re, double* __restrict__ im, InsSpec ins,
+__global__ void __launch_bounds__(kThreads) kSwap(double* re, double* im, InsSpec ins,
                                                   uint64_t b1, uint64_t b2, uint64_t n) {
     const uint64_t t = (uint64_t)blockIdx.x * kThreads + threadIdx.x;
     if (t >= n) return;
