@@ -227,8 +227,10 @@ __global__ void __launch_bounds__(kThreads) kImages(const DevPass* passes, const
 }  // namespace
 
 void freeBuildScratch(BuildScratch& s) {
+    s.source.release();
     if (s.device) cudaFree(s.device);
-    s = BuildScratch();
+    s.device = nullptr;
+    s.bytes = 0;
 }
 
 bool buildsOnDevice(const FusedPlan& plan, const FusedPass& pass, const std::vector<int>& members) {
@@ -275,13 +277,13 @@ bool queueBuild(const FusedPlan& plan, const std::vector<int>& which, const std:
         if (QG_CUDA(cudaMalloc(&scratch.device, need), caller)) return false;
         scratch.bytes = need;
     }
-    std::vector<char> host(upload, 0);                   // maxima start at 0
-    memcpy(host.data() + eAt, entries.data(), entries.size() * sizeof(cplx));
-    memcpy(host.data() + pAt, passes.data(), passes.size() * sizeof(DevPass));
-    memcpy(host.data() + gAt, gates.data(), gates.size() * sizeof(DevGate));
+    char* host = scratch.source.open(upload, caller);    // (maxima start at 0)
+    if (!host) return false;
+    memcpy(host + eAt, entries.data(), entries.size() * sizeof(cplx));
+    memcpy(host + pAt, passes.data(), passes.size() * sizeof(DevPass));
+    memcpy(host + gAt, gates.data(), gates.size() * sizeof(DevGate));
     char* dev = reinterpret_cast<char*>(scratch.device);
-    // pageable source: the copy returns once it is staged
-    if (QG_CUDA(cudaMemcpyAsync(dev, host.data(), upload, cudaMemcpyHostToDevice, st), caller)) return false;
+    if (!scratch.source.copy(dev, st, caller)) return false;
     const DevPass* dp = reinterpret_cast<const DevPass*>(dev + pAt);
     double2* products = reinterpret_cast<double2*>(dev + upload);
     unsigned long long* largest = reinterpret_cast<unsigned long long*>(dev + mAt);

@@ -2,6 +2,7 @@
 #pragma once
 
 #include "fused_plan.h"
+#include "upload_source.h"
 
 #include <cuda_runtime.h>
 #include <stddef.h>
@@ -21,6 +22,7 @@ struct BuildOutput {
 struct BuildScratch {
     void* device = nullptr;
     size_t bytes = 0;
+    UploadSource source;
 };
 void freeBuildScratch(BuildScratch& s);
 

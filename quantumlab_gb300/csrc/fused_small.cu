@@ -341,6 +341,7 @@ struct PlanProgram {
     int groups = 16;                          // groups of 64 amplitudes a chunk
     uint32_t chunks = 0;
     BuildScratch scratch;                     // of products formed on the device
+    UploadSource source;                      // of the buffer's contents
     int* errFlag = nullptr;                   // page-locked: a kernel writes it only when it gives up
     size_t bytes = 0;                         // room in buffer
     char* buffer = nullptr;                   // device: matrices, passes, barrier counters
@@ -391,7 +392,8 @@ void* smallPlanUpload(const FusedPlan& plan, void* reuse) {
     const size_t at = plan.passes.size() * 2 * kD * kD;
     std::vector<Seg> segs;
     for (size_t i = 0; i < plan.passes.size(); ++i) segs.push_back(segOf(plan.passes[i], n, pp->groups, i * 2 * kD * kD));
-    std::vector<float> mats;
+    const char* caller = "applyPlanF32";
+    const size_t matBytes = at * sizeof(float), segBytes = (segs.size() * sizeof(Seg) + 31) / 32 * 32;
     std::vector<int> deferred;
     std::vector<BuildOutput> outputs;
     for (size_t i = 0; i < plan.passes.size(); ++i) {
@@ -404,13 +406,19 @@ void* smallPlanUpload(const FusedPlan& plan, void* reuse) {
                 if (std::binary_search(pass.targets.begin(), pass.targets.end(), t[b])) o.smallMask |= 1 << b;
             deferred.push_back((int)i);
             outputs.push_back(o);
-            continue;
         }
-        mats.resize(at);
-        smallMatrix(pass, n, mats.data() + i * 2 * kD * kD);
     }
-    const char* caller = "applyPlanF32";
-    const size_t matBytes = at * sizeof(float), segBytes = (segs.size() * sizeof(Seg) + 31) / 32 * 32;
+    // the buffer's contents: matrices (none, when the device forms them all),
+    // passes, counters at zero
+    const size_t matHost = deferred.size() < plan.passes.size() ? matBytes : 0;
+    char* host = pp->source.open(matHost + segBytes + kCounterBytes, caller);
+    if (!host) {
+        smallPlanFree(pp);
+        return nullptr;
+    }
+    for (size_t i = 0; i < plan.passes.size(); ++i)
+        if (!plan.passes[i].m.empty()) smallMatrix(plan.passes[i], n, reinterpret_cast<float*>(host) + i * 2 * kD * kD);
+    memcpy(host + matHost, segs.data(), segs.size() * sizeof(Seg));
     if (!pp->errFlag && QG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&pp->errFlag), sizeof(int), cudaHostAllocMapped), caller)) {
         smallPlanFree(pp);
         return nullptr;
@@ -428,10 +436,7 @@ void* smallPlanUpload(const FusedPlan& plan, void* reuse) {
     pp->mats = reinterpret_cast<float*>(pp->buffer);
     pp->segs = reinterpret_cast<Seg*>(pp->buffer + matBytes);
     pp->counters = reinterpret_cast<unsigned*>(pp->buffer + matBytes + segBytes);
-    // pageable sources: a copy returns once its source is staged
-    if ((!mats.empty() && QG_CUDA(cudaMemcpyAsync(pp->mats, mats.data(), matBytes, cudaMemcpyHostToDevice, stream()), caller)) ||
-        QG_CUDA(cudaMemcpyAsync(pp->segs, segs.data(), segs.size() * sizeof(Seg), cudaMemcpyHostToDevice, stream()), caller) ||
-        QG_CUDA(cudaMemsetAsync(pp->counters, 0, kCounterBytes, stream()), caller) ||
+    if (!pp->source.copy(pp->buffer + (matBytes - matHost), stream(), caller) ||
         !queueBuild(plan, deferred, outputs, pp->mats, pp->scratch, stream(), caller)) {
         smallPlanFree(pp);
         return nullptr;
@@ -444,6 +449,7 @@ void smallPlanFree(void* h) {
     PlanProgram* pp = reinterpret_cast<PlanProgram*>(h);
     if (!pp) return;
     cudaStreamSynchronize(stream());
+    pp->source.release();
     if (pp->buffer) cudaFree(pp->buffer);
     freeBuildScratch(pp->scratch);
     if (pp->errFlag) cudaFreeHost(pp->errFlag);
