@@ -88,23 +88,27 @@ struct Inner2 {
     __device__ __forceinline__ double2 add(double2 acc, const Four& v) const {
         const double2 a = v.a, b = v.b, c = v.c, d = v.d;
         using namespace fsum;
-        const uint32_t wb = max(max(magnitude(a.x), magnitude(a.y)), max(magnitude(b.x), magnitude(b.y)));
-        const uint32_t wk = max(max(magnitude(c.x), magnitude(c.y)), max(magnitude(d.x), magnitude(d.y)));
+        const uint32_t ma = magnitude(a.x), na = magnitude(a.y), mb = magnitude(b.x), nb = magnitude(b.y);
+        const uint32_t mc = magnitude(c.x), nc = magnitude(c.y), md = magnitude(d.x), nd = magnitude(d.y);
+        const uint32_t wb = max(max(ma, na), max(mb, nb)), wk = max(max(mc, nc), max(md, nd));
         const int E = (int)(wb >> 20), F = (int)(wk >> 20);
         // (a zero factor adds nothing, unless the other is infinite or NaN)
         if (((wb | lowWords(a, b)) == 0 && F < 0x7FF) || ((wk | lowWords(c, d)) == 0 && E < 0x7FF)) return acc;
-        if (!unitFits(E, F)) {
+        const int ea = exponentOf(ma), eb = exponentOf(mb), ec = exponentOf(mc), ed = exponentOf(md);
+        const int fa = exponentOf(na), fb = exponentOf(nb), fc = exponentOf(nc), fd = exponentOf(nd);
+        if (!unitFits(E, F) || !productsFit(E, F, ea + ec, eb + ed, fa + fc, fb + fd) ||
+            !productsFit(E, F, ea + ed, eb + ec, fa + fd, fb + fc)) {
             const double2 v = innerFp64(a, b, c, d);
             return make_double2(acc.x + v.x, acc.y + v.y);
         }
-        const int2 ax = digits(a.x, E), ay = digits(a.y, E), bx = digits(b.x, E), by = digits(b.y, E);
-        const int2 cx = digits(c.x, F), cy = digits(c.y, F), dx = digits(d.x, F), dy = digits(d.y, F);
+        const int2 ax = wideDigits(a.x, E), ay = wideDigits(a.y, E), bx = wideDigits(b.x, E), by = wideDigits(b.y, E);
+        const int2 cx = wideDigits(c.x, F), cy = wideDigits(c.y, F), dx = wideDigits(d.x, F), dy = wideDigits(d.y, F);
         const int2 nx = make_int2(-bx.x, -bx.y), ny = make_int2(-by.x, -by.y);
         Sums r{0, 0, 0}, m{0, 0, 0};
         r.add(ax, cx); r.add(bx, dx); r.add(ay, cy); r.add(by, dy);
         m.add(ax, dx); m.add(nx, cx); m.add(ay, dy); m.add(ny, cy);
-        const double u = unit(E, F);
-        return make_double2(fma(u, r.few(), acc.x), fma(u, m.few(), acc.y));
+        const double u = wideUnit(E, F);
+        return make_double2(fma(u, r.wide(), acc.x), fma(u, m.wide(), acc.y));
     }
 };
 struct Inner1 {
