@@ -1,23 +1,26 @@
 // expec_tile.cu -- the expectation value of a Pauli sum on a state vector,
-// many terms per pass over the state, on the integer pipes (sm_103a).
+// many terms per pass over the state (sm_103a).
 //
 // One reduction per X/Y mask (reduce.cu) reads the state once per mask and
 // spends 3 to 5 FP64 operations on a pair: at 24 qubits 151 us a mask and 501
 // us for the diagonal terms, bound by the FP64 pipe, against 39 us of HBM
-// time.  Here a block takes tiles of 2^b amplitudes into shared memory, as
-// 54-bit integers against the tile's largest exponent, and adds up every mask
-// that lies in the tile's qubits:
-//   * Re or Im of conj(psi_j) psi_k as products of 27-bit digits summed in 64
-//     bits (8 wide multiply-adds a pair; FP64 runs at a 30th of their rate),
-//     over the pairs on which the mask's terms do not cancel; two terms a step,
-//     steps of equal weights into one sum, converted once;
+// time.  Here a block takes tiles of 2^b amplitudes into shared memory and adds
+// up every mask that lies in the tile's qubits:
+//   * Re or Im of conj(psi_j) psi_k in two FP64 multiply-adds, over the pairs
+//     on which the mask's terms do not cancel (a quarter of the amplitudes for
+//     X..X and Y..Y of equal weight); two terms a step, steps of equal weights
+//     into one sum.  Warps whose pairs hold a zero each (particle-number
+//     sectors leave most of a register zero) spend no FP64.  Integer products
+//     against the tile's largest amplitude would be faster on dense states,
+//     but lose the products that are far below it: <X> of (1, e) is e.
 //   * all diagonal terms through one Walsh-Hadamard transform of the tile's
 //     |psi|^2 in 64-bit integers, scaled so that the tile's sum fills them:
-//     a term is then one entry, whatever its weight.
-// A value is rounded to 2^-55 of the tile's largest amplitude, a probability to
-// 2^-62 of the tile's sum: less than the rounding of FP64 sums of the same
-// products.  Energy of a 12-site Hubbard chain (24 qubits, 22 masks and 36
-// diagonal terms), the whole call: 3.90 ms -> 0.61 ms; 16 qubits 152 -> 46 us.
+//     a term is then one entry, whatever its weight.  A value is rounded to
+//     2^-55 of the tile's largest amplitude, a probability to 2^-62 of the
+//     tile's sum: less than the rounding of FP64 sums of |psi|^2.
+// Energy of a 12-site Hubbard chain (24 qubits, 22 masks and 36 diagonal terms),
+// the whole call: 3.91 ms -> 0.64 ms on a state without zeros, 0.50 ms after a
+// short evolution from a classical state; 16 qubits 147 -> 47 us.
 #include "chain_launch.cuh"
 #include "fixed_sum.cuh"
 #include "pauli_expec.h"
@@ -28,8 +31,7 @@
 namespace qg {
 namespace {
 
-using fsum::digits;
-using fsum::Sums;
+using fsum::absDigits;
 
 constexpr int kThreads = 256, kWarps = kThreads / 32;
 constexpr int kMaxTileBits = 12, kMinTileBits = 8;
@@ -65,18 +67,26 @@ __device__ __forceinline__ uint32_t place(uint32_t i) { return i ^ ((i >> 3) & 1
 struct PairLoop {                                // a step on this tile
     uint32_t xl, ml, dl, outM, outD, pairs;
     int pair, fix, one;          // one: the parity that acts, -1: both
+    bool skip;                   // pairs with a zero add nothing
 };
+__device__ __forceinline__ double flip(double v, uint32_t sign) {      // sign: 0 or 1
+    return __hiloint2double(__double2hiint(v) ^ (int)(sign << 31), __double2loint(v));
+}
+__device__ __forceinline__ bool nonzero(double x, double y) {
+    return (((uint32_t)__double2hiint(x) | (uint32_t)__double2hiint(y)) << 1 | (uint32_t)(__double2loint(x) | __double2loint(y))) != 0;
+}
 // Pair t's j is t with zeros inserted: a thread's part (its index) and the
 // round's part, the same for all threads, are worked out apart, parities too.
+// (pairs is a multiple of 32, so that a warp's lanes take part together.)
 template <bool IMAG, bool BOTH>
-__device__ __forceinline__ void addPairs(const PairLoop& o, const int2* sr, const int2* si, Sums& s0, Sums& s1) {
+__device__ __forceinline__ void addPairs(const PairLoop& o, const double* sr, const double* si, double& s0, double& s1) {
     if (threadIdx.x >= o.pairs) return;
     const bool fixed = o.fix >= 0;
     const int b0 = fixed ? min(o.pair, o.fix) : o.pair, b1 = fixed ? max(o.pair, o.fix) : 31;
     const uint32_t jt = insert0(insert0(threadIdx.x, b0), b1);
     const uint32_t parT = __popc(jt & o.dl), sgnT = __popc(jt & o.ml);
     const uint32_t fixM = fixed && (o.ml >> o.fix & 1u);         // the fixed bit is one of ml's
-#pragma unroll 4
+#pragma unroll 2
     for (uint32_t u = 0; u < o.pairs; u += kThreads) {
         const uint32_t ju = insert0(insert0(u, b0), b1);
         const uint32_t parU = __popc(ju & o.dl) ^ o.outD, sgnU = __popc(ju & o.ml) ^ o.outM;
@@ -87,37 +97,28 @@ __device__ __forceinline__ void addPairs(const PairLoop& o, const int2* sr, cons
             sg ^= f & fixM;
         }
         const uint32_t k = j ^ o.xl;
-        const int sgn = 1 - 2 * (int)(sg & 1u);
-        int2 jr = sr[j], ji = si[j];
-        const int2 kr = sr[k], ki = si[k];
-        jr.x *= sgn; jr.y *= sgn;
-        const int sgi = IMAG ? -sgn : sgn;       // Im: jr ki - ji kr
-        ji.x *= sgi; ji.y *= sgi;
-        if (BOTH) {                              // (only where a step's terms do not cancel anywhere)
-            Sums v{0, 0, 0};
-            v.add(jr, IMAG ? ki : kr);
-            v.add(ji, IMAG ? kr : ki);
-            Sums& s = par ? s1 : s0;
-            s.hh += v.hh; s.x += v.x; s.ll += v.ll;
-        } else {
-            s0.add(jr, IMAG ? ki : kr);
-            s0.add(ji, IMAG ? kr : ki);
-        }
+        const double jr = sr[j], ji = si[j], kr = sr[k], ki = si[k];
+        // (a zero with an infinity or NaN is no zero)
+        if (o.skip && !__any_sync(0xffffffffu, nonzero(jr, ji) && nonzero(kr, ki))) continue;
+        sg &= 1u;
+        const double x = flip(jr, sg), y = flip(ji, IMAG ? sg ^ 1u : sg);      // Im: jr ki - ji kr
+        double& s = BOTH && par ? s1 : s0;
+        s = fma(y, IMAG ? kr : ki, fma(x, IMAG ? ki : kr, s));
     }
 }
 
 __global__ void __launch_bounds__(kThreads) kExpecTile(const double* re, const double* im,
                                                        uint64_t tiles, const __grid_constant__ ExpecPass p,
                                                        double* partials, unsigned* counter, double* result) {
-    extern __shared__ int2 sm[];
+    extern __shared__ double sm[];
     __shared__ int shE[kWarps];
     __shared__ float shS[kWarps];
     __shared__ double shD[kWarps];
     __shared__ bool amLast;
     const int b = p.b, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t size = 1u << b;
-    int2* sr = sm;
-    int2* si = sr + size;
+    double* sr = sm;
+    double* si = sr + size;
     uint64_t* high = reinterpret_cast<uint64_t*>(si + size);             // qubits of tile index bits >= kLow
     for (uint32_t h = tid; h < size >> kLow; h += kThreads) {
         uint64_t a = 0;
@@ -145,23 +146,11 @@ __global__ void __launch_bounds__(kThreads) kExpecTile(const double* re, const d
         if (lane == 0) shE[warp] = E;
         __syncthreads();
         for (int w = 0; w < kWarps; ++w) E = max(E, shE[w]);
-        if (E == 0x7FF) {                        // infinities or NaNs: so is the sum
-            acc = __longlong_as_double(0x7FF8000000000000ll);
-            continue;
-        }
-        // this thread converts what it loaded
-        for (uint32_t l = 2 * tid; l < size; l += 2 * kThreads) {
-            const double2 r = *reinterpret_cast<const double2*>(sr + l), i = *reinterpret_cast<const double2*>(si + l);
-            sr[l] = digits(r.x, E); sr[l + 1] = digits(r.y, E);
-            si[l] = digits(i.x, E); si[l + 1] = digits(i.y, E);
-        }
-        __syncthreads();
-        Sums s0{0, 0, 0}, s1{0, 0, 0};
-        const double unit = scalbn(1.0, 2 * E - 2098);               // of a high digits' product
+        double s0 = 0.0, s1 = 0.0;
         for (int o = 0; o < p.numOps; ++o) {
             const PairOp& op = p.op[o];
             PairLoop pl{op.xl, op.ml, op.dl, (uint32_t)__popcll(base & op.m) & 1u, (uint32_t)__popcll(base & op.d) & 1u, 0,
-                        op.pair, op.fix, op.c[0] != 0 && op.c[1] != 0 ? -1 : op.c[0] != 0 ? 0 : 1};
+                        op.pair, op.fix, op.c[0] != 0 && op.c[1] != 0 ? -1 : op.c[0] != 0 ? 0 : 1, E != 0x7FF};
             const int one = pl.one;
             pl.pairs = pl.dl == 0 && one >= 0 && (int)pl.outD != one ? 0 : pl.fix >= 0 ? size / 4 : size / 2;
             if (op.imag) {
@@ -172,20 +161,23 @@ __global__ void __launch_bounds__(kThreads) kExpecTile(const double* re, const d
                 else addPairs<false, false>(pl, sr, si, s0, s1);
             }
             if (op.flush) {
-                // products below 2^54: a sum ends (on the host's word) well before 2^8 of them
-                acc = s0.into(acc, (op.c[0] != 0 ? op.c[0] : op.c[1]) * unit);
-                if (one < 0) acc = s1.into(acc, op.c[1] * unit);
-                s0 = s1 = Sums{0, 0, 0};
+                acc = fma(op.c[0] != 0 ? op.c[0] : op.c[1], s0, acc);
+                if (one < 0) acc = fma(op.c[1], s1, acc);
+                s0 = s1 = 0.0;
             }
         }
         if (p.numDiag == 0) continue;
+        if (E == 0x7FF) {                        // infinities or NaNs: so is the sum
+            acc = __longlong_as_double(0x7FF8000000000000ll);
+            continue;
+        }
         __syncthreads();
         // |psi|^2 in units of 2^46 products, then scaled to the tile's sum
         int64_t* q = reinterpret_cast<int64_t*>(sr);
         float sum = 0.f;
         for (uint32_t l = tid; l < size; l += kThreads) {
-            const int2 r = sr[l], i = si[l];
-            const uint64_t x = (uint64_t)abs((int64_t)r.x * (1 << 27) + r.y) << 9, y = (uint64_t)abs((int64_t)i.x * (1 << 27) + i.y) << 9;
+            const int2 r = absDigits(sr[l], E), i = absDigits(si[l], E);
+            const uint64_t x = ((uint64_t)r.x << 36) | ((uint64_t)r.y << 9), y = ((uint64_t)i.x << 36) | ((uint64_t)i.y << 9);
             const int64_t v = (int64_t)(__umul64hi(x, x) + __umul64hi(y, y) + ((x * x) >> 63) + ((y * y) >> 63));
             sum += __ll2float_ru(v);
             __syncwarp();                        // place(l) is in this warp's sixteen
@@ -359,9 +351,11 @@ bool queueExpecTiles(SV s, const std::vector<PauliTermGroup>& groups, const Scra
         std::vector<Plan> p = deal(steps, (int)diag.size(), c);
         double us = 0;
         const double rounds = std::ceil(std::ldexp(1.0, s.n - c) / sms), amps = std::ldexp(1.0, c);
-        for (const Plan& q : p)
-            us += 4 + std::ldexp(1.0, s.n) * 16 / 6e6 + rounds * (q.steps.size() * std::max(0.3, amps * 0.25 * 45 / (90 * 1900)) +
-                                                                  (q.count ? 3 : 0) + amps * 40 / (90 * 1900));
+        for (const Plan& q : p) {
+            us += 4 + std::ldexp(1.0, s.n) * 16 / 6e6 + rounds * ((q.count ? 3 : 0) + amps * 40 / (90 * 1900));
+            for (const Step& a : q.steps)                            // 1.65 FP64 operations a clock
+                us += rounds * std::max(0.3, amps * ((a.c[0] == 0) != (a.c[1] == 0) && a.d ? 0.25 : 0.5) * 2 / (1.65 * 1900));
+        }
         if (b && us >= best) continue;
         b = c;
         best = us;
@@ -380,7 +374,7 @@ bool queueExpecTiles(SV s, const std::vector<PauliTermGroup>& groups, const Scra
         for (int q = 0; q < s.n && __builtin_popcountll(tile) < b; ++q) tile |= 1ull << q;
         for (int q = 0, k = 0; q < s.n; ++q)
             if (tile >> q & 1) p.pos[k++] = (unsigned char)q;
-        int run = 0;                             // products in this thread's sum
+        int run = 0;                             // products in this thread's sum, kept short
         for (size_t i = 0; i < pp.steps.size(); ++i) {
             const Step& a = pp.steps[i];
             PairOp& op = p.op[p.numOps++];

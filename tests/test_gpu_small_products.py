@@ -1,6 +1,7 @@
-"""Inner products whose products are all far smaller than the amplitudes that
-they are made of: every product has to keep FP64's precision relative to
-itself, not to the largest amplitude around it (csrc/fixed_sum.cuh)."""
+"""Inner products and Pauli expectation values whose products are all far
+smaller than the amplitudes that they are made of: every product has to keep
+FP64's precision relative to itself, not to the largest amplitude around it
+(csrc/fixed_sum.cuh, csrc/reduce.cu, csrc/expec_tile.cu)."""
 import math
 
 import numpy as np
@@ -66,3 +67,52 @@ def test_nearly_orthogonal_density_matrices(gpulib, eps):
         assert abs(L.lib.calcDensityInnerProduct(a, b) - math.fsum(p)) <= bound(2 * n, np.abs(p))
     L.destroy(a)
     L.destroy(b)
+
+
+def magnitude(psi, code):
+    """The products of an off-diagonal string's expectation value."""
+    n = len(code)
+    j = np.arange(psi.shape[0])
+    x = sum(1 << q for q in range(n) if code[q] in (1, 2))
+    yz = sum(1 << q for q in range(n) if code[q] in (2, 3))
+    ny = sum(1 for c in code if c == 2)
+    par = j & yz
+    for sh in (16, 8, 4, 2, 1):
+        par = par ^ (par >> sh)
+    sign = 1.0 - 2.0 * (par & 1)
+    k = j ^ x
+    if ny % 2 == 0:
+        p = np.concatenate([sign * psi.real * psi.real[k], sign * psi.imag * psi.imag[k]]) * (1 if ny % 4 == 0 else -1)
+    else:
+        p = np.concatenate([sign * psi.real * psi.imag[k], -sign * psi.imag * psi.real[k]]) * (1 if ny % 4 == 1 else -1)
+    return p
+
+
+@pytest.mark.parametrize("n", [2, 8, 10, 13, 16])
+@pytest.mark.parametrize("eps", EPS)
+def test_off_diagonal_strings(gpulib, n, eps):
+    L = gpulib
+    r = np.random.default_rng(n)
+    q, ws = L.create(n), L.create(n)
+    for seed in range(3):
+        codes = [[1 if k == t else 0 for k in range(n)] for t in (0, 1, n - 1)]
+        codes += [[2 if k == t else 0 for k in range(n)] for t in (0, n - 1)]
+        for _ in range(4):
+            c = [int(v) for v in r.choice((0, 0, 0, 1, 2, 3), n)]
+            c[int(r.integers(n))] = int(r.integers(1, 3))
+            codes.append(c)
+        states = [s for pair in near_basis(n, seed, eps) for s in pair][seed::6]
+        for psi in states[:8]:
+            # the partner of a large amplitude under some string is small
+            L.set_amps(q, psi)
+            for code in codes:
+                # and with a second string on the same X/Y mask, of another weight
+                two = [c if c in (1, 2) else int(v) for c, v in zip(code, r.choice((0, 3), n))]
+                co = np.array([0.7, -0.4])
+                h = L.pauli_hamil(np.array([code, two], dtype=np.int32), co)
+                got = L.lib.calcExpecPauliHamil(q, h, ws)
+                L.lib.destroyPauliHamil(h)
+                p = np.concatenate([w * magnitude(psi, c) for w, c in zip(co, (code, two))])
+                assert abs(got - math.fsum(p)) <= bound(n, np.abs(p)), (n, eps, code, two, got, math.fsum(p))
+    L.destroy(q)
+    L.destroy(ws)
