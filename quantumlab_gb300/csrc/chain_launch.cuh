@@ -21,6 +21,8 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
+#include <mutex>
 #include <utility>
 
 namespace qg {
@@ -36,15 +38,31 @@ __device__ __forceinline__ void chainStart() {
 // and its blocks then crowd where places are free first: 256 blocks (18 qubits)
 // of a gate bound by the FP64 pipe took 13.2 us, launched plainly 8.2.  Shared
 // memory that is not used keeps an SM to the even share.
+constexpr size_t kEvenShareBytes = 200 * 1024;
 inline size_t evenShare(unsigned blocks) {
     const unsigned sms = (unsigned)numSMs(), each = (blocks + sms - 1) / sms;
     // each + 1 such blocks do not fit 228 KB, and one leaves 27 KB for a kernel's own
-    return 2 * blocks > sms && each <= 4 ? 200 * 1024 / each : 0;
+    return 2 * blocks > sms && each <= 4 ? kEvenShareBytes / each : 0;
+}
+// Let a kernel's launches take up to `most` bytes of dynamic shared memory.  The
+// limit belongs to the process, and to set it while another thread launches the
+// kernel may fail that launch (or crash in the driver).  So it is set once, to
+// the most that any launch takes, before the kernel's first launch.
+template <auto kernel>
+inline cudaError_t allowShared(size_t most) {
+    static std::mutex mutex;
+    static std::atomic<bool> set{false};
+    if (set.load(std::memory_order_acquire)) return cudaSuccess;
+    std::lock_guard<std::mutex> lk(mutex);
+    if (set.load(std::memory_order_relaxed)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+    if (e == cudaSuccess) set.store(true, std::memory_order_release);
+    return e;
 }
 
 // `cluster`: blocks to a thread-block cluster (of consecutive blocks in x)
 template <class... Params, class... Args>
-inline void chainClusters(unsigned cluster, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+inline void launchChained(unsigned cluster, void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                           Args&&... args) {
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -55,17 +73,22 @@ inline void chainClusters(unsigned cluster, void (*kernel)(Params...), dim3 grid
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = grid;
     cfg.blockDim = block;
-    if (smem == 0 && (smem = evenShare(grid.x * grid.y)) > 48 * 1024)
-        (void)cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cfg.attrs = attr;
     cfg.numAttrs = cluster > 1 ? 2 : 1;
     (void)cudaLaunchKernelEx(&cfg, kernel, Params(std::forward<Args>(args))...);     // its error: launchFailed
 }
-template <class... Params, class... Args>
-inline void chain(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
-    chainClusters(1, kernel, grid, block, smem, st, std::forward<Args>(args)...);
+// A kernel without shared memory of its own takes the even share's.
+template <auto kernel, class... Args>
+inline void chain(dim3 grid, dim3 block, cudaStream_t st, Args&&... args) {
+    const bool allowed = allowShared<kernel>(kEvenShareBytes) == cudaSuccess;
+    launchChained(1, kernel, grid, block, allowed ? evenShare(grid.x * grid.y) : 0, st, std::forward<Args>(args)...);
+}
+// One with `smem` bytes, which allowShared has been asked for.
+template <auto kernel, class... Args>
+inline void chainShared(unsigned cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+    launchChained(cluster, kernel, grid, block, smem, st, std::forward<Args>(args)...);
 }
 
 }  // namespace qg

@@ -259,6 +259,9 @@ __global__ void __launch_bounds__(kThreads) kExpecTile(const double* re, const d
     }
 }
 
+// amplitudes, and the qubits of the tile index bits from kLow up
+size_t tileShared(int b) { return (size_t(16) << b) + (size_t(8) << (b - kLow)); }
+
 uint32_t localMask(uint64_t mask, const unsigned char* pos, int b) {
     uint32_t l = 0;
     for (int k = 0; k < b; ++k) l |= (uint32_t)(mask >> pos[k] & 1) << k;
@@ -363,8 +366,8 @@ bool queueExpecTiles(SV s, const std::vector<PauliTermGroup>& groups, const Scra
     }
     if (!b) return steps.empty() && diag.empty();
     cudaStream_t st = stream();
-    const size_t smem = (size_t(16) << b) + (size_t(8) << (b - kLow));
-    if (QG_CUDA(cudaFuncSetAttribute(kExpecTile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), caller)) return false;
+    const size_t smem = tileShared(b);
+    if (QG_CUDA(allowShared<kExpecTile>(tileShared(kMaxTileBits)), caller)) return false;
     const uint64_t tiles = 1ull << (s.n - b);
     const unsigned grid = (unsigned)std::min<uint64_t>(tiles, 3ull * (uint64_t)numSMs());
     for (const Plan& pp : plan) {
@@ -404,7 +407,7 @@ bool queueExpecTiles(SV s, const std::vector<PauliTermGroup>& groups, const Scra
         p.numDiag = pp.count;
         double* out = slot();
         if (!out) return false;
-        chain(kExpecTile, grid, kThreads, smem, st, s.re, s.im, tiles, p, w.partials, w.counter, out);
+        chainShared<kExpecTile>(1, grid, kThreads, smem, st, s.re, s.im, tiles, p, w.partials, w.counter, out);
         if (launchFailed(caller)) return false;
     }
     return true;

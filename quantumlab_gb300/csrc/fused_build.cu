@@ -288,10 +288,10 @@ bool queueBuild(const FusedPlan& plan, const std::vector<int>& which, const std:
     double2* products = reinterpret_cast<double2*>(dev + upload);
     unsigned long long* largest = reinterpret_cast<unsigned long long*>(dev + mAt);
     const dim3 grid((unsigned)passes.size(), kSlices);
-    chain(kProducts, grid, kThreads, 0, st, dp, reinterpret_cast<const DevGate*>(dev + gAt),
+    chain<kProducts>(grid, kThreads, st, dp, reinterpret_cast<const DevGate*>(dev + gAt),
           reinterpret_cast<const double2*>(dev + eAt), products, largest);
     if (launchFailed(caller)) return false;
-    chain(kImages, grid, kThreads, 0, st, dp, products, largest, out);
+    chain<kImages>(grid, kThreads, st, dp, products, largest, out);
     return !launchFailed(caller);
 }
 

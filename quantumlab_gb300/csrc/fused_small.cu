@@ -21,6 +21,7 @@
 //
 // Every wait on the barrier is bounded: a block that gives up sets the error
 // flag and ends.
+#include "chain_launch.cuh"
 #include "fused_build.h"
 #include "fused_small.h"
 #include "qg_internal.h"
@@ -351,6 +352,12 @@ struct PlanProgram {
 };
 constexpr size_t kCounterBytes = 2 * sizeof(unsigned);
 
+template <int GC>
+bool launchPasses(void** args, unsigned grid, cudaStream_t st, const char* caller) {
+    constexpr size_t smem = Shape<GC>::smem;
+    return !QG_CUDA(allowShared<kSmallPasses<GC>>(smem), caller) &&
+           !QG_CUDA(cudaLaunchCooperativeKernel((const void*)kSmallPasses<GC>, dim3(grid), dim3(kThreads), args, smem, st), caller);
+}
 bool launch(const PlanProgram& p, float* re, float* im, int step0, int step1, cudaStream_t st, const char* caller) {
     if (step0 >= step1) return true;
     const Seg* segs = p.segs;
@@ -359,13 +366,11 @@ bool launch(const PlanProgram& p, float* re, float* im, int step0, int step1, cu
     unsigned* counters = p.counters;
     int* errFlag = p.errFlag;
     void* args[] = {&re, &im, &mats, &segs, &chunks, &step0, &step1, &counters, &errFlag};
-    const void* fn = p.groups == 32 ? (const void*)kSmallPasses<32> : p.groups == 16 ? (const void*)kSmallPasses<16>
-                                                                                  : (const void*)kSmallPasses<8>;
-    const size_t smem = p.groups == 32 ? Shape<32>::smem : p.groups == 16 ? Shape<16>::smem : Shape<8>::smem;
     const unsigned grid = std::min((unsigned)numSMs(), chunks);
-    if (QG_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), caller)) return false;
-    if (QG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kThreads), args, smem, st), caller)) return false;
-    return !launchFailed(caller);
+    const bool ok = p.groups == 32   ? launchPasses<32>(args, grid, st, caller)
+                    : p.groups == 16 ? launchPasses<16>(args, grid, st, caller)
+                                     : launchPasses<8>(args, grid, st, caller);
+    return ok && !launchFailed(caller);
 }
 
 // the most of 8, 16, 32 groups a chunk that leaves at most half the SMs

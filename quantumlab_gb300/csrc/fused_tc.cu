@@ -1309,13 +1309,7 @@ bool launchTC(float* re, float* im, int n, const FusedPass& pass, const float* i
     constexpr int cols = (3 * K) <= 64 ? 64 : ((3 * K) <= 128 ? 128 : ((3 * K) <= 256 ? 256 : 512));
     constexpr int perSM = 512 / cols;
     const size_t smemReq = std::max(smem + 1024, (size_t)(220 * 1024 / perSM));
-    static bool configured[8] = {};
-    if (!configured[KQ]) {
-        if (QG_CUDA(cudaFuncSetAttribute(kApplyTC<KQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemReq),
-                    "applyPlanF32"))
-            return false;
-        configured[KQ] = true;
-    }
+    if (QG_CUDA(allowShared<kApplyTC<KQ>>(smemReq), "applyPlanF32")) return false;
     const uint64_t grid = std::min<uint64_t>(numTiles, (uint64_t)perSM * numSMs());
     kApplyTC<KQ><<<(unsigned)grid, kThreadsTC, smemReq, st>>>(re, im, img, numTiles, errFlag, nl, p);
     return !launchFailed("applyPlanF32");
@@ -1524,14 +1518,9 @@ bool launchTC2(float* re, float* im, int n, const FusedPass& pass, const float* 
     // groups shorten it: 300 passes over three 16-qubit states 1905 -> 1607 us,
     // split-FP16 passes on 16 qubits 7.6 -> 7.3 us, on 18 qubits 7.6 -> 7.2.
     p.pair = kPairs<KQ, LG, EG, LS> && p.ctasPerInst == numTiles && 4 * grid <= (uint64_t)numSMs();
-    static bool configured = false;
-    if (!configured) {
-        if (QG_CUDA(cudaFuncSetAttribute(kApplyTC2<KQ, LG, EG, LS, PR, CV, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                    "applyPlanF32"))
-            return false;
-        configured = true;
-    }
-    chainClusters(p.pair ? 2 : 1, kApplyTC2<KQ, LG, EG, LS, PR, CV, ST>, (unsigned)grid << p.pair, (4 * (LG + EG) + 1) * 32, smem, st, re, im, img, numTiles, errFlag, nl, p);
+    if (QG_CUDA((allowShared<kApplyTC2<KQ, LG, EG, LS, PR, CV, ST>>(smem)), "applyPlanF32")) return false;
+    chainShared<kApplyTC2<KQ, LG, EG, LS, PR, CV, ST>>(p.pair ? 2 : 1, (unsigned)grid << p.pair, (4 * (LG + EG) + 1) * 32, smem, st,
+                                                       re, im, img, numTiles, errFlag, nl, p);
     return !launchFailed("applyPlanF32");
 }
 

@@ -220,6 +220,9 @@ __global__ void __launch_bounds__(kThreads) kPauliTile(double* re, double* im,
     }
 }
 
+// amplitudes, and the qubits of the tile index bits from kLow up
+size_t tileShared(int b) { return (size_t(16) << b) + (size_t(8) << (b - kLow)); }
+
 // ------------------------------------------------------------------- planning
 struct Sum {                       // an angle as an unevaluated sum of two doubles
     double hi = 0.0, lo = 0.0;
@@ -469,9 +472,8 @@ void gatePauliSequence(SV s, const std::vector<PauliRotation>& seq, double* tabl
         return;
     }
     cudaStream_t st = stream();
-    const size_t smem = (size_t(16) << b) + (size_t(8) << (b - kLow));
-    // every call: the attribute belongs to the device that is current here
-    if (QG_CUDA(cudaFuncSetAttribute(kPauliTile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), caller)) return;
+    const size_t smem = tileShared(b);
+    if (QG_CUDA(allowShared<kPauliTile>(tileShared(kMaxTileBits)), caller)) return;
     // the scale of all the passes' rotations: with the first phase table, or
     // where there is none as the last pass writes
     double grow = 0;
@@ -558,11 +560,12 @@ void gatePauliSequence(SV s, const std::vector<PauliRotation>& seq, double* tabl
         if (ts.numWindows) {
             int bits = 0;
             for (int w = 0; w < ts.numWindows; ++w) bits = std::max(bits, ts.bits[w]);
-            chain(kPhaseTables, dim3(((1u << bits) + kThreads - 1) / kThreads, ts.numWindows), kThreads, 0, st, ts,
-                  reinterpret_cast<double2*>(tables));
+            chain<kPhaseTables>(dim3(((1u << bits) + kThreads - 1) / kThreads, ts.numWindows), kThreads, st, ts,
+                                reinterpret_cast<double2*>(tables));
             if (launchFailed(caller)) return;
         }
-        chain(kPauliTile, (unsigned)(1ull << (s.n - b)), kThreads, smem, st, s.re, s.im, p, reinterpret_cast<const double2*>(tables));
+        chainShared<kPauliTile>(1, (unsigned)(1ull << (s.n - b)), kThreads, smem, st, s.re, s.im, p,
+                                reinterpret_cast<const double2*>(tables));
         if (launchFailed(caller)) return;
     }
 }

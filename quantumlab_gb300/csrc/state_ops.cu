@@ -242,9 +242,9 @@ template <class Op>
 void launchChannel(SV s, int t, int N, const Op& op, const char* caller) {
     const uint64_t nGroups = 1ull << (s.n - 2);
     if (t >= 1 && nGroups >= 2)
-        chain(kChannelVec<Op>, blocksFor(nGroups / 2), kThreads, 0, stream(), s.re, s.im, t, N, nGroups / 2, op);
+        chain<kChannelVec<Op>>(blocksFor(nGroups / 2), kThreads, stream(), s.re, s.im, t, N, nGroups / 2, op);
     else
-        chain(kChannelT0<Op>, blocksFor(nGroups), kThreads, 0, stream(), s.re, s.im, N, nGroups, op);
+        chain<kChannelT0<Op>>(blocksFor(nGroups), kThreads, stream(), s.re, s.im, N, nGroups, op);
     launchFailed(caller);
 }
 
@@ -328,10 +328,10 @@ void launchTwoQubitChannel(SV s, int q1, int q2, int N, double retain, double di
     const TwoQubitBits tb{{q1, q2, q1 + N, q2 + N}};
     const uint64_t nGroups = 1ull << (s.n - 4);
     if (q1 >= 1)
-        chain(kTwoQubitChannel<2, MIX>, blocksFor(nGroups / 2), kThreads, 0, stream(), s.re, s.im, tb, nGroups / 2,
+        chain<kTwoQubitChannel<2, MIX>>(blocksFor(nGroups / 2), kThreads, stream(), s.re, s.im, tb, nGroups / 2,
                                                                                   retain, diagRetain, mix);
     else
-        chain(kTwoQubitChannel<1, MIX>, blocksFor(nGroups), kThreads, 0, stream(), s.re, s.im, tb, nGroups, retain,
+        chain<kTwoQubitChannel<1, MIX>>(blocksFor(nGroups), kThreads, stream(), s.re, s.im, tb, nGroups, retain,
                                                                                diagRetain, mix);
     launchFailed(caller);
 }

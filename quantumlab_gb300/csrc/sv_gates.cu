@@ -230,12 +230,12 @@ void launchPair(SV s, uint64_t ctrl, uint64_t setMask, uint64_t pmask, const Op&
     double* const lre = cross ? s.im : s.re;
     double* const lim = cross ? s.re : s.im;
     if (nPairs >= 2 && !(insMask & 1ull)) {
-        chain(kPairVec<Op>, blocksFor(nPairs / 2), kThreads, 0, st, s.re, s.im, lre, lim, ins, setMask, pmask, nPairs / 2, op);
+        chain<kPairVec<Op>>(blocksFor(nPairs / 2), kThreads, st, s.re, s.im, lre, lim, ins, setMask, pmask, nPairs / 2, op);
     } else if (nPairs >= 2 && pmask == 1ull) {
-        if (cross) chain(kPairAdj<true, Op>, blocksFor(nPairs / 2), kThreads, 0, st, s.re, s.im, ins, setMask, nPairs / 2, op);
-        else chain(kPairAdj<false, Op>, blocksFor(nPairs / 2), kThreads, 0, st, s.re, s.im, ins, setMask, nPairs / 2, op);
+        if (cross) chain<kPairAdj<true, Op>>(blocksFor(nPairs / 2), kThreads, st, s.re, s.im, ins, setMask, nPairs / 2, op);
+        else chain<kPairAdj<false, Op>>(blocksFor(nPairs / 2), kThreads, st, s.re, s.im, ins, setMask, nPairs / 2, op);
     } else {
-        chain(kPairScalar<Op>, blocksFor(nPairs), kThreads, 0, st, s.re, s.im, lre, lim, ins, setMask, pmask, nPairs, op);
+        chain<kPairScalar<Op>>(blocksFor(nPairs), kThreads, st, s.re, s.im, lre, lim, ins, setMask, pmask, nPairs, op);
     }
     launchFailed(caller);
 }
@@ -341,9 +341,9 @@ void launchDiag(SV s, uint64_t fixedMask, uint64_t setMask, const Op& op, const 
     const uint64_t nAmps = 1ull << free;
     cudaStream_t st = stream();
     if (nAmps >= 2 && !(fixedMask & 1ull))
-        chain(kDiagVec<Op>, blocksFor(nAmps / 2), kThreads, 0, st, s.re, s.im, ins, setMask, nAmps / 2, op);
+        chain<kDiagVec<Op>>(blocksFor(nAmps / 2), kThreads, st, s.re, s.im, ins, setMask, nAmps / 2, op);
     else
-        chain(kDiagScalar<Op>, blocksFor(nAmps), kThreads, 0, st, s.re, s.im, ins, setMask, nAmps, op);
+        chain<kDiagScalar<Op>>(blocksFor(nAmps), kThreads, st, s.re, s.im, ins, setMask, nAmps, op);
     launchFailed(caller);
 }
 
@@ -597,9 +597,9 @@ void gatePauliRotation(SV s, uint64_t ctrl, uint64_t xmask, uint64_t ymask, uint
     const uint64_t nPairs = 1ull << free;
     cudaStream_t st = stream();
     if (nPairs >= 2 && !(insMask & 1ull) && !(xmask & 1ull))
-        chain(kPauliRotVec, blocksFor(nPairs / 2), kThreads, 0, st, s.re, s.im, ins, ctrl, nPairs / 2, p);
+        chain<kPauliRotVec>(blocksFor(nPairs / 2), kThreads, st, s.re, s.im, ins, ctrl, nPairs / 2, p);
     else
-        chain(kPauliRotScalar, blocksFor(nPairs), kThreads, 0, st, s.re, s.im, ins, ctrl, nPairs, p);
+        chain<kPauliRotScalar>(blocksFor(nPairs), kThreads, st, s.re, s.im, ins, ctrl, nPairs, p);
     launchFailed("multiRotatePauli");
 }
 
@@ -607,7 +607,7 @@ void gateSwap(SV s, int q1, int q2) {
     if (s.cap && captureSwap(s, q1, q2)) return;
     const InsSpec ins = makeIns((1ull << q1) | (1ull << q2));
     const uint64_t n = 1ull << (s.n - 2);
-    chain(kSwap, blocksFor(n), kThreads, 0, stream(), s.re, s.im, ins, 1ull << q1, 1ull << q2, n);
+    chain<kSwap>(blocksFor(n), kThreads, stream(), s.re, s.im, ins, 1ull << q1, 1ull << q2, n);
     launchFailed("swapGate");
 }
 

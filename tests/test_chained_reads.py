@@ -28,7 +28,7 @@ def kernels():
                 yield pytest.param(signature, body, id=re.search(r"\b(k[A-Z]\w*)\s*\(", signature).group(1))
 
 
-@pytest.mark.parametrize("signature,body", kernels())
+@pytest.mark.parametrize("signature,body", list(kernels()))
 def test_chained_kernels_read_coherently(signature, body):
     assert "__restrict__" not in signature + body
     assert "__ldg(" not in body and "ld.global.nc" not in body
