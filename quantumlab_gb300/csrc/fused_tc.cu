@@ -1213,6 +1213,10 @@ struct DevicePlan {
     std::vector<const double*> target;
     int lastTC = -1;        // last tensor-core pass applied (its drift is corrected next)
     bool chain = false;     // the state is still lastTC's output up to unitary SIMT passes
+    // lastTC's input norm, output norm and squared scale were put behind the
+    // records (norms + 3 normPasses), because the range that has begun runs the
+    // passes that hold them again
+    bool carried = false;
     // sum |x|^2 of the state this range started from, when the caller measured
     // it (device; until a non-unitary SIMT pass): the bound of the first
     // tensor-core pass's split-FP16 scale
@@ -1669,7 +1673,7 @@ void* uploadPlanTC(const FusedPlan& plan, void* reuse) {
     dp->inNorm.clear();
     dp->target.clear();
     dp->lastTC = -1;
-    dp->chain = false;
+    dp->chain = dp->carried = false;
     dp->entryBound = nullptr;
     if (!dp->errFlag && cudaMalloc(&dp->errFlag, sizeof(int)) != cudaSuccess) {
         cudaGetLastError();
@@ -1681,7 +1685,7 @@ void* uploadPlanTC(const FusedPlan& plan, void* reuse) {
     if (dp->normPasses < std::max<size_t>(1, np)) {
         if (dp->norms) cudaFree(dp->norms);
         dp->normPasses = std::max<size_t>(1, np);
-        if (cudaMalloc(&dp->norms, 3 * dp->normPasses * sizeof(double)) != cudaSuccess) {
+        if (cudaMalloc(&dp->norms, 3 * (dp->normPasses + 1) * sizeof(double)) != cudaSuccess) {
             cudaGetLastError();
             dp->norms = nullptr;
             dp->normPasses = 0;
@@ -1856,7 +1860,7 @@ void tcBeginPlan(void* devPlan, size_t numPasses) {
     DevicePlan* dp = reinterpret_cast<DevicePlan*>(devPlan);
     if (!dp) return;
     dp->lastTC = -1;
-    dp->chain = false;
+    dp->chain = dp->carried = false;
     dp->inNorm.assign(numPasses, nullptr);
     dp->target.assign(numPasses, nullptr);
 }
@@ -1864,13 +1868,25 @@ void tcBeginPlan(void* devPlan, size_t numPasses) {
 // start of every applyPlanF32Range call: the caller may have changed the
 // state since the last call, so the next tensor-core pass measures its input;
 // entryBound: sum |x|^2 of the state now, on the device, or null; the norm
-// records of passes [first, last) are cleared
+// records of passes [first, last) are cleared, all at once (a memset before each
+// pass would keep it from starting as the one before ends); what the first of
+// them corrects by, the last pass's record, is kept
 void tcBeginRange(void* devPlan, const double* entryBound, size_t first, size_t last) {
     DevicePlan* dp = reinterpret_cast<DevicePlan*>(devPlan);
     if (!dp) return;
     dp->chain = false;
     dp->entryBound = entryBound;
-    if (dp->norms && last > first) cudaMemsetAsync(dp->norms + 3 * first, 0, 3 * (last - first) * sizeof(double), stream());
+    if (!dp->norms || last <= first) return;
+    auto cleared = [&](const double* p) { return p >= dp->norms + 3 * first && p < dp->norms + 3 * last; };
+    dp->carried = false;
+    if (dp->lastTC >= 0 && (size_t)dp->lastTC < dp->inNorm.size() && dp->inNorm[dp->lastTC]) {
+        const double *in = dp->inNorm[dp->lastTC], *record = dp->norms + 3 * dp->lastTC;
+        double* kept = dp->norms + 3 * dp->normPasses;
+        if (cleared(in) || cleared(record))
+            dp->carried = cudaMemcpyAsync(kept, in, sizeof(double), cudaMemcpyDeviceToDevice, stream()) == cudaSuccess &&
+                          cudaMemcpyAsync(kept + 1, record + 1, 2 * sizeof(double), cudaMemcpyDeviceToDevice, stream()) == cudaSuccess;
+    }
+    cudaMemsetAsync(dp->norms + 3 * first, 0, 3 * (last - first) * sizeof(double), stream());
 }
 
 // a pass ran on the SIMT applier: a non-unitary one changes the norm
@@ -2140,9 +2156,10 @@ int applyPassTCIndexed(QuregF32& q, const FusedPass& pass, const void* devPlan, 
         else if (dp->entryBound) nl.boundSq = dp->entryBound;
         const bool prevUnitary = dp->lastTC >= 0 && dp->unitary[dp->lastTC];
         if (prevUnitary) {
-            nl.corrIn = dp->inNorm[dp->lastTC];
-            nl.corrOut = dp->norms + 3 * dp->lastTC + 1;
-            nl.corrScaleSq = dp->norms + 3 * dp->lastTC + 2;
+            const double* kept = dp->norms + 3 * dp->normPasses;
+            nl.corrIn = dp->carried ? kept : dp->inNorm[dp->lastTC];
+            nl.corrOut = dp->carried ? kept + 1 : dp->norms + 3 * dp->lastTC + 1;
+            nl.corrScaleSq = dp->carried ? kept + 2 : dp->norms + 3 * dp->lastTC + 2;
         }
         // a chain of unitary passes keeps the norm its first pass started from
         const bool continues = chained && prevUnitary && dp->target[dp->lastTC];
@@ -2153,6 +2170,7 @@ int applyPassTCIndexed(QuregF32& q, const FusedPass& pass, const void* devPlan, 
     if (!ok) return -1;
     dp->lastTC = (int)index;
     dp->chain = true;
+    dp->carried = false;
     return 1;
 }
 
