@@ -36,6 +36,7 @@ namespace qg {
 bool tensorCoresEnabled();       // fused_tc.cu
 bool tcDefaultAppliers();
 void freePlanTC(void* devicePlan);
+size_t planBytesTC(const void* devicePlan);
 
 struct Capture {
     int n = 0;
@@ -43,7 +44,7 @@ struct Capture {
     bool tracePreserving = true;  // every queued op is a unitary gate or a channel
     std::vector<FusedGate> gates;
     void* q32 = nullptr;          // FP32 scratch register of the flushes (kept between flushes)
-    // device memory of the last flush's plan, for the next one's
+    // device memory of the last flush's plan, for the next one's (no more than keptBytes)
     void *spare = nullptr, *smallSpare = nullptr;
     long long flushes = 0, gatesApplied = 0, passesApplied = 0;
     double compileMs = 0.0;       // host time spent planning the flushes
@@ -162,6 +163,12 @@ void captureRegister(const double* re, int n, int dmQubits) {
     }
 }
 
+// Device memory a register keeps from one flush's plan to the next's: what some
+// hundred passes take (an 8-layer circuit on 20 qubits 4 MB), or a small part
+// of what the register itself takes.  A flush has no size limit; the memory of
+// a larger one is given back.
+static size_t keptBytes(int n) { return std::max<size_t>(size_t(16) << 20, (size_t(16) << n) / 64); }
+
 // apply and clear the queue of a capture record (caller holds no lock)
 static void flushRecord(Capture* c, double* re, double* im) {
     if (!c || c->gates.empty()) return;
@@ -226,6 +233,11 @@ static void flushRecord(Capture* c, double* re, double* im) {
     else copyToQuregAfterPlan(c->q32, view, plan);
     c->spare = plan->device ? plan->device : plan->spare;
     c->smallSpare = plan->small ? plan->small : plan->smallSpare;
+    if (planBytesTC(c->spare) + smallPlanBytes(c->smallSpare) > keptBytes(c->n)) {
+        freePlanTC(c->spare);
+        smallPlanFree(c->smallSpare);
+        c->spare = c->smallSpare = nullptr;
+    }
     plan->device = plan->small = plan->spare = plan->smallSpare = nullptr;
     c->gatesApplied += (long long)plan->gates.size();
     c->passesApplied += (long long)plan->passes.size();

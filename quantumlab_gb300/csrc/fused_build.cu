@@ -33,6 +33,7 @@ struct DevGate {
 struct DevPass {
     int k, gate, gates;
     int smallMask;
+    uint64_t product;                    // entries to its product
     uint64_t full, bf16, compact, f16, small;
 };
 
@@ -90,7 +91,7 @@ __device__ __forceinline__ void applyGate(double2* m, const double2* u, const De
     }
 }
 
-// products: D x D entries of pass p from p * 4096 on, row-major
+// products: D x D entries a pass, row-major
 __global__ void __launch_bounds__(kThreads) kProducts(const DevPass* passes, const DevGate* gates,
                                                       const double2* entries, double2* products, unsigned long long* largest) {
     constexpr int kMaxEntries = 1 << (2 * kMaxGateQubits);
@@ -109,7 +110,6 @@ __global__ void __launch_bounds__(kThreads) kProducts(const DevPass* passes, con
     for (int g = 0; g < p.gates; ++g) {
         __syncthreads();
         const DevGate dg = gate[g % 3];
-        const int G = 1 << dg.q;
         const double2* u = entry[g & 1];
         // the next gate's entries, the one after's description
         if (g + 1 < p.gates && tid < 1 << (2 * gate[(g + 1) % 3].q)) entry[(g + 1) & 1][tid] = entries[gate[(g + 1) % 3].m + tid];
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(kThreads) kProducts(const DevPass* passes, con
     unsigned long long big = 0;
     for (int i = threadIdx.x; i < D * W; i += kThreads) {
         const double2 v = m[i];
-        products[(size_t)blockIdx.x * 4096 + (i / W) * D + c0 + i % W] = v;
+        products[p.product + (i / W) * D + c0 + i % W] = v;
         const unsigned long long a = __double_as_longlong(fabs(v.x)), b = __double_as_longlong(fabs(v.y));
         big = max(big, max(a, b));
     }
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kThreads) kImages(const DevPass* passes, const
     chainStart();
     const DevPass p = passes[blockIdx.x];
     const int D = 1 << p.k, N = 2 * D;
-    const double2* M = products + (size_t)blockIdx.x * 4096;
+    const double2* M = products + p.product;
     const int first = blockIdx.y * kThreads + threadIdx.x, step = kSlices * kThreads;
     // entry (r, j) of the real form [[Re, -Im], [Im, Re]]
     auto real = [&](int r, int j) {
@@ -246,6 +246,7 @@ bool queueBuild(const FusedPlan& plan, const std::vector<int>& which, const std:
     std::vector<DevPass> passes;
     std::vector<DevGate> gates;
     std::vector<cplx> entries;
+    size_t product = 0;
     for (size_t w = 0; w < which.size(); ++w) {
         const FusedPass& pass = plan.passes[which[w]];
         const BuildOutput& o = outputs[w];
@@ -253,6 +254,8 @@ bool queueBuild(const FusedPlan& plan, const std::vector<int>& which, const std:
         d.k = (int)pass.targets.size();
         d.gate = (int)gates.size();
         d.smallMask = o.smallMask;
+        d.product = product;
+        product += (size_t)1 << (2 * d.k);
         d.full = o.full; d.bf16 = o.bf16; d.compact = o.compact; d.f16 = o.f16; d.small = o.small;
         for (int i : plan.passMembers[which[w]]) {
             const FusedGate& g = plan.gates[i];
@@ -271,7 +274,7 @@ bool queueBuild(const FusedPlan& plan, const std::vector<int>& which, const std:
     auto up16 = [](size_t b) { return (b + 15) / 16 * 16; };
     const size_t eAt = 0, pAt = up16(entries.size() * sizeof(cplx)), gAt = pAt + up16(passes.size() * sizeof(DevPass));
     const size_t mAt = gAt + up16(gates.size() * sizeof(DevGate)), upload = mAt + up16(passes.size() * 8);
-    const size_t need = upload + passes.size() * 4096 * sizeof(double2);
+    const size_t need = upload + product * sizeof(double2);
     if (scratch.bytes < need) {
         freeBuildScratch(scratch);
         if (QG_CUDA(cudaMalloc(&scratch.device, need), caller)) return false;

@@ -461,6 +461,11 @@ void smallPlanFree(void* h) {
     delete pp;
 }
 
+size_t smallPlanBytes(const void* h) {
+    const PlanProgram* pp = reinterpret_cast<const PlanProgram*>(h);
+    return pp ? pp->bytes + pp->scratch.bytes : 0;
+}
+
 // passes [first, last) of the plan; 0, a kernel's error code, or -1 when the launch failed
 int smallPlanApply(void* h, float* re, float* im, int first, int last) {
     PlanProgram* pp = reinterpret_cast<PlanProgram*>(h);

@@ -19,6 +19,7 @@ bool smallPlanFits(const FusedPlan& plan);
 // reuse: an earlier program, whose memory is taken over; null when it failed
 void* smallPlanUpload(const FusedPlan& plan, void* reuse);
 void smallPlanFree(void* program);
+size_t smallPlanBytes(const void* program);          // device memory it holds
 int smallPlanApply(void* program, float* re, float* im, int first, int last);
 
 }  // namespace qg

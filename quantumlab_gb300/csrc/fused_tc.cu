@@ -1855,6 +1855,12 @@ void freePlanTC(void* h) {
     delete dp;
 }
 
+// device memory of a plan's copy
+size_t planBytesTC(const void* devPlan) {
+    const DevicePlan* dp = reinterpret_cast<const DevicePlan*>(devPlan);
+    return dp ? dp->imageFloats * sizeof(float) + 3 * (dp->normPasses + 1) * sizeof(double) + dp->scratch.bytes : 0;
+}
+
 // start of a plan application (pass 0): no previous tensor-core pass
 void tcBeginPlan(void* devPlan, size_t numPasses) {
     DevicePlan* dp = reinterpret_cast<DevicePlan*>(devPlan);
