@@ -205,52 +205,60 @@ struct ExpecDiag1 {                              // SV, x = 0, one amplitude per
 };
 
 // ---- calcProbOfAllOutcomes ------------------------------------------------
-// The amplitude index is 8 low qubits, one per thread of a block, and the
-// rest, the items: (values of the measured high qubits, values of the others),
-// the others fastest.  A block takes a run of items; a thread sums its
+// The amplitude index is the low qubits, one value per thread of a unit, and
+// the rest, the items: (values of the measured high qubits, values of the
+// others), the others fastest.  A unit takes a run of items; a thread sums its
 // amplitudes while the measured high qubits stay, four at a time on the
-// integer pipes, and the block then adds its threads of equal outcome and
-// gives the sums to out.  An atomic addition in shared memory per amplitude,
-// as before, took 119 us at 24 qubits and 10 measured ones; 46 us so.
-constexpr int kLowQubits = 8;
+// integer pipes, and the unit then adds its threads of equal outcome and gives
+// the sums to out.  A unit is a block (8 low qubits); where a block's runs
+// would be short (most high qubits measured) and its adding, five FP64
+// additions by every thread a run, all the work, it is a warp (5 low qubits).
+// 24 qubits (HBM floor 39 us), 10 measured: 119 us with an atomic addition per
+// amplitude, 46 so; 16 measured, the highest (the whole call, with its copy to
+// the host): 270, by blocks 507, by warps 130.
+constexpr int kLowQubits = 8, kWarpQubits = 5;
 struct OutcomeSpec {
-    int low, high;                 // low qubits (8, or all of fewer), the other ones
-    uint64_t measured;             // high qubits that are measured (bit 0: qubit `low`)
-    int highBit[64];               // the outcome's bit of each measured high qubit, ascending
-    uint32_t lowMask;              // low qubits that are measured
-    int lowBit[kLowQubits];        // the outcome's bit of each low qubit
+    unsigned char low, high;            // low qubits (kLowQubits or kWarpQubits, or all of fewer), the other ones
+    unsigned char numMeasured;          // high qubits that are measured
+    unsigned char lowMask;              // low qubits that are measured
+    unsigned char lowBit[kLowQubits];   // the outcome's bit of each low qubit
+    uint64_t measured;                  // the measured high qubits (bit 0: qubit `low`)
+    unsigned char highQubit[40];        // ascending, likewise
+    unsigned char highBit[40];          // the outcome's bit of each
 };
-template <bool DM>
+template <bool DM, bool WARPS>
 __global__ void __launch_bounds__(1 << kLowQubits) kOutcomes(const double* __restrict__ re, const double* __restrict__ im,
                                                              uint64_t step, const __grid_constant__ OutcomeSpec s,
                                                              double* __restrict__ out) {
+    constexpr int kUnitQubits = WARPS ? kWarpQubits : kLowQubits, kPerBlock = 1 << (kLowQubits - kUnitQubits);
     __shared__ double part[1 << kLowQubits];
-    const uint32_t tid = threadIdx.x;
+    const uint32_t tid = threadIdx.x & ((1u << kUnitQubits) - 1u);
     const bool live = tid < 1u << s.low;
     const uint64_t others = ((1ull << s.high) - 1) & ~s.measured;
-    const int fast = __popcll(others);
+    const int fast = s.high - s.numMeasured;
     const uint64_t items = 1ull << s.high;
-    const uint64_t each = items / gridDim.x, more = items % gridDim.x;
-    uint64_t k = each * blockIdx.x + min((uint64_t)blockIdx.x, more);
-    const uint64_t end = k + each + (blockIdx.x < more ? 1 : 0);
-    uint32_t own = 0;
+    const uint64_t unit = (uint64_t)blockIdx.x * kPerBlock + (threadIdx.x >> kUnitQubits), units = (uint64_t)gridDim.x * kPerBlock;
+    const uint64_t each = items / units, more = items % units;
+    uint64_t k = each * unit + min(unit, more);
+    const uint64_t end = k + each + (unit < more ? 1 : 0);
+    // the first item's qubits and outcome
+    uint64_t set = 0, h = 0, v = k >> fast, r = k & ((1ull << fast) - 1);
+    uint32_t o = 0;
     for (int q = 0; q < s.low; ++q)
-        if (s.lowMask >> q & 1u) own |= ((tid >> q) & 1u) << s.lowBit[q];
+        if (s.lowMask >> q & 1u) o |= ((tid >> q) & 1u) << s.lowBit[q];
+    for (int m = 0; m < s.numMeasured; ++m) {
+        const uint32_t bit = (uint32_t)(v >> m) & 1u;
+        set |= (uint64_t)bit << s.highQubit[m];
+        o |= bit << s.highBit[m];
+    }
+    for (int q = 0; r; ++q) {
+        if (s.measured >> q & 1) continue;
+        h |= (r & 1) << q;
+        r >>= 1;
+    }
     while (k < end) {
         // a run with the same measured high qubits
         const uint64_t stop = min(end, ((k >> fast) + 1) << fast);
-        uint64_t set = 0, h = 0, v = k >> fast, r = k & ((1ull << fast) - 1);
-        uint32_t o = own;
-        for (int q = 0, m = 0; q < s.high; ++q) {
-            if (s.measured >> q & 1) {
-                set |= (v & 1) << q;
-                o |= (uint32_t)(v & 1) << s.highBit[m++];
-                v >>= 1;
-            } else {
-                h |= (r & 1) << q;
-                r >>= 1;
-            }
-        }
         double acc = 0.0;
         for (; k < stop; k += 4) {
             double x[4] = {0, 0, 0, 0}, y[4] = {0, 0, 0, 0};
@@ -264,21 +272,31 @@ __global__ void __launch_bounds__(1 << kLowQubits) kOutcomes(const double* __res
                 h = ((h | ~others) + 1) & others;
             }
             if (DM) acc += (x[0] + x[1]) + (x[2] + x[3]);
+            else if (stop - k == 1) acc = fma(x[0], x[0], fma(y[0], y[0], acc));        // one amplitude: FP64 is less work
             else acc = fsum::addSquares(acc, make_double2(x[0], x[1]), make_double2(x[2], x[3]), make_double2(y[0], y[1]), make_double2(y[2], y[3]));
         }
         k = stop;
-        // the threads that differ in unmeasured low qubits only: lanes, then warps
+        h = 0;
+        // the threads that differ in unmeasured low qubits only (those that a
+        // small register lacks too): lanes, then warps
+        const uint32_t skip = ~(uint32_t)s.lowMask & ((1u << kUnitQubits) - 1u);
 #pragma unroll
         for (int q = 0; q < 5; ++q)
-            if (!(s.lowMask >> q & 1u)) acc += __shfl_xor_sync(0xffffffffu, acc, 1 << q);
-        __syncthreads();
-        part[tid] = acc;
-        __syncthreads();
-        const uint32_t skip = ~s.lowMask & ((1u << kLowQubits) - 1u);          // (qubits a small register lacks too)
-        if (tid & skip) continue;
-        for (uint32_t w = 1; w < 8; ++w)
-            if (((w << 5) & ~skip) == 0) acc += part[tid | (w << 5)];
-        atomicAdd(out + o, acc);
+            if (skip >> q & 1u) acc += __shfl_xor_sync(0xffffffffu, acc, 1 << q);
+        if (!WARPS && skip >> 5) {
+            __syncthreads();
+            part[tid] = acc;
+            __syncthreads();
+            for (uint32_t w = 1; w < 8; ++w)
+                if (((w << 5) & ~skip) == 0 && (tid & skip) == 0) acc += part[tid | (w << 5)];
+        }
+        if ((tid & skip) == 0) atomicAdd(out + o, acc);
+        uint64_t changed = v ^ (v + 1);          // the next run's measured qubits
+        ++v;
+        for (int m = 0; changed && m < s.numMeasured; ++m, changed >>= 1) {
+            set ^= 1ull << s.highQubit[m];
+            o ^= 1u << s.highBit[m];
+        }
     }
 }
 
@@ -437,23 +455,34 @@ void reduceProbAllOutcomes(SV s, int isDM, int N, const int* qubits, int nq, dou
     cudaStream_t st = stream();
     if (QG_CUDA(cudaMemsetAsync(dOut, 0, (size_t)nOut * sizeof(double), st), "calcProbOfAllOutcomes")) return;
     const int n = isDM ? N : s.n;
-    OutcomeSpec sp{};
-    sp.low = std::min(n, kLowQubits);
-    sp.high = n - sp.low;
-    for (int q = 0, m = 0; q < n; ++q)
-        for (int b = 0; b < nq; ++b) {
-            if (qubits[b] != q) continue;
-            if (q < sp.low) {
-                sp.lowMask |= 1u << q;
-                sp.lowBit[q] = b;
-            } else {
-                sp.measured |= 1ull << (q - sp.low);
-                sp.highBit[m++] = b;
+    auto spec = [&](int lowest) {
+        OutcomeSpec sp{};
+        sp.low = (unsigned char)std::min(n, lowest);
+        sp.high = (unsigned char)(n - sp.low);
+        for (int q = 0; q < n; ++q)
+            for (int b = 0; b < nq; ++b) {
+                if (qubits[b] != q) continue;
+                if (q < sp.low) {
+                    sp.lowMask |= 1u << q;
+                    sp.lowBit[q] = (unsigned char)b;
+                } else {
+                    sp.measured |= 1ull << (q - sp.low);
+                    sp.highQubit[sp.numMeasured] = (unsigned char)(q - sp.low);
+                    sp.highBit[sp.numMeasured++] = (unsigned char)b;
+                }
             }
-        }
-    const unsigned grid = (unsigned)std::min<uint64_t>(1ull << sp.high, 8ull * (uint64_t)numSMs());
-    if (isDM) kOutcomes<true><<<grid, 1 << kLowQubits, 0, st>>>(s.re, s.im, (1ull << N) + 1, sp, dOut);
-    else kOutcomes<false><<<grid, 1 << kLowQubits, 0, st>>>(s.re, s.im, 1, sp, dOut);
+        return sp;
+    };
+    OutcomeSpec sp = spec(kLowQubits);
+    const bool warps = sp.numMeasured > 0 && sp.high - sp.numMeasured < 4;       // runs of fewer than 16 items
+    if (warps) sp = spec(kWarpQubits);
+    const uint64_t blocks = warps ? ((1ull << sp.high) + 7) / 8 : 1ull << sp.high;
+    const unsigned grid = (unsigned)std::min<uint64_t>(blocks, 8ull * (uint64_t)numSMs());
+    const uint64_t step = isDM ? (1ull << N) + 1 : 1;
+    if (isDM && warps) kOutcomes<true, true><<<grid, 1 << kLowQubits, 0, st>>>(s.re, s.im, step, sp, dOut);
+    else if (isDM) kOutcomes<true, false><<<grid, 1 << kLowQubits, 0, st>>>(s.re, s.im, step, sp, dOut);
+    else if (warps) kOutcomes<false, true><<<grid, 1 << kLowQubits, 0, st>>>(s.re, s.im, step, sp, dOut);
+    else kOutcomes<false, false><<<grid, 1 << kLowQubits, 0, st>>>(s.re, s.im, step, sp, dOut);
     if (launchFailed("calcProbOfAllOutcomes")) return;
     QG_CUDA(cudaMemcpyAsync(hostOut, dOut, (size_t)nOut * sizeof(double), cudaMemcpyDeviceToHost, st), "calcProbOfAllOutcomes");
     QG_CUDA(cudaStreamSynchronize(st), "calcProbOfAllOutcomes");
