@@ -337,6 +337,7 @@ bool queueExpecTiles(SV s, const std::vector<PauliTermGroup>& groups, const Scra
                 if (st.c[0] != 0 || st.c[1] != 0) steps.push_back(st);
             }
     }
+    if (steps.empty() && diag.empty()) return true;      // density matrices, small registers: no tile size fits them
     // equal weights next to one another
     std::stable_sort(steps.begin(), steps.end(), [](const Step& a, const Step& b) {
         return a.c[0] != b.c[0] ? a.c[0] < b.c[0] : a.c[1] < b.c[1];
@@ -364,7 +365,7 @@ bool queueExpecTiles(SV s, const std::vector<PauliTermGroup>& groups, const Scra
         best = us;
         plan.swap(p);
     }
-    if (!b) return steps.empty() && diag.empty();
+    if (!b) return false;
     cudaStream_t st = stream();
     const size_t smem = tileShared(b);
     if (QG_CUDA(allowShared<kExpecTile>(tileShared(kMaxTileBits)), caller)) return false;
