@@ -25,6 +25,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <atomic>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <sys/time.h>
@@ -1132,8 +1133,12 @@ static void expPauliHamil(const std::vector<qg::PauliRotation>& terms, double fa
         out.back().angle *= 2 * fac;
     }
 }
+// Appends a repetition's rotations to `out`; `full` takes them off where some
+// thousands have come together (a repetition of order 2 m has 5^(m - 1) times
+// those of order 2).
+constexpr size_t kTrotterRun = 4096;
 static void symTrotter(const std::vector<qg::PauliRotation>& terms, double time, int order,
-                       std::vector<qg::PauliRotation>& out) {
+                       std::vector<qg::PauliRotation>& out, const std::function<void()>& full) {
     if (order == 1) {
         expPauliHamil(terms, time, 0, out);
     } else if (order == 2) {
@@ -1142,12 +1147,14 @@ static void symTrotter(const std::vector<qg::PauliRotation>& terms, double time,
     } else {
         const double p = 1. / (4 - pow(4, 1. / (order - 1)));
         const int lo = order - 2;
-        symTrotter(terms, p * time, lo, out);
-        symTrotter(terms, p * time, lo, out);
-        symTrotter(terms, (1 - 4 * p) * time, lo, out);
-        symTrotter(terms, p * time, lo, out);
-        symTrotter(terms, p * time, lo, out);
+        symTrotter(terms, p * time, lo, out, full);
+        symTrotter(terms, p * time, lo, out, full);
+        symTrotter(terms, (1 - 4 * p) * time, lo, out, full);
+        symTrotter(terms, p * time, lo, out, full);
+        symTrotter(terms, p * time, lo, out, full);
+        return;
     }
+    if (out.size() >= kTrotterRun) full();
 }
 void applyTrotterCircuit(Qureg q, PauliHamil h, qreal time, int order, int reps) {
     const char* caller = "applyTrotterCircuit";
@@ -1165,13 +1172,11 @@ void applyTrotterCircuit(Qureg q, PauliHamil h, qreal time, int order, int reps)
         pauliMasks(ts.data(), h.pauliCodes + (idx_t)t * h.numQubits, h.numQubits, &r.x, &r.y, &r.z);
         if (r.x | r.z) terms.push_back(r);
     }
-    // The repetitions in runs of some thousand rotations.  A density matrix
-    // gets a run's rotations on its rows, then their conjugates on its
-    // columns: the two act on different qubits.
+    if (terms.empty()) return;
+    // A density matrix gets a run's rotations on its rows, then their
+    // conjugates on its columns: the two act on different qubits.
     const int s = q.isDensityMatrix ? q.numQubitsRepresented : 0;
-    for (int r = 0; r < reps; ++r) {
-        symTrotter(terms, time / reps, order, seq);
-        if (seq.size() < 4096 && r + 1 < reps) continue;
+    const std::function<void()> run = [&]() {
         const qg::SV state = svg(q);
         const size_t rows = seq.size();
         if (state.cap) {                     // queued one by one
@@ -1180,7 +1185,7 @@ void applyTrotterCircuit(Qureg q, PauliHamil h, qreal time, int order, int reps)
                 if (q.isDensityMatrix) qg::gatePauliRotation(state, 0, c.x << s, c.y << s, c.z << s, c.angle, 1);
             }
             seq.clear();
-            continue;
+            return;
         }
         if (q.isDensityMatrix)
             for (size_t i = 0; i < rows; ++i) {
@@ -1189,7 +1194,9 @@ void applyTrotterCircuit(Qureg q, PauliHamil h, qreal time, int order, int reps)
             }
         qg::gatePauliSequence(state, seq, q.firstLevelReduction + qg::kScratchDoubles);
         seq.clear();
-    }
+    };
+    for (int r = 0; r < reps; ++r) symTrotter(terms, time / reps, order, seq, run);
+    if (!seq.empty()) run();
 }
 
 // ---- measurement (QuEST.c:972-1016, QuEST_common.c:165-180, 361-375) ----
