@@ -240,6 +240,9 @@ struct Sum {                       // an angle as an unevaluated sum of two doub
 // A circuit repeats few angles, so that these last bits add up: over the 146
 // rotations of a 22-qubit Hubbard step the turns by the exact angles are
 // 3e-15 off the product of the rotations, with lo and grow 5e-16.
+// An angle of many turns is told by the same c and s as one within half a
+// turn, and that one is taken: the sums of merged angles then keep a lo so
+// small that its square is nothing.
 struct Turn {
     Sum phi;
     double grow;
@@ -248,8 +251,8 @@ Turn turnOf(double angle) {
     const double a = angle / 2, c = std::cos(a), s = std::sin(a);
     const long double lc = c, ls = s;
     Turn t;
-    t.phi.hi = a;
-    t.phi.lo = (double)(ls * std::cos((long double)a) - lc * std::sin((long double)a));
+    t.phi.hi = std::fabs(a) > 64 ? std::atan2(s, c) : a;
+    t.phi.lo = (double)(ls * std::cos((long double)t.phi.hi) - lc * std::sin((long double)t.phi.hi));
     t.grow = (double)((lc * lc + ls * ls - 1) / 2);
     return t;
 }
@@ -451,6 +454,12 @@ double cost(const std::vector<PassPlan>& plan, const std::vector<Step>& steps, c
 
 void gatePauliSequence(SV s, const std::vector<PauliRotation>& seq, double* tables) {
     const char* caller = "applyTrotterCircuit";
+    auto oneByOne = [&]() {
+        for (const PauliRotation& r : seq) gatePauliRotation(s, 0, r.x, r.y, r.z, r.angle, r.conj);
+    };
+    // angles that are not finite: the passes leave zeros as they are, where a
+    // rotation by NaN makes them NaN
+    if (!std::all_of(seq.begin(), seq.end(), [](const PauliRotation& r) { return std::isfinite(r.angle); })) return oneByOne();
     std::vector<Step> steps;
     merge(seq, steps);
     std::vector<Windows> win(steps.size());
@@ -468,7 +477,7 @@ void gatePauliSequence(SV s, const std::vector<PauliRotation>& seq, double* tabl
         plan.swap(p);
     }
     if (b < kLow + 1) {                            // registers of one to three qubits
-        for (const PauliRotation& r : seq) gatePauliRotation(s, 0, r.x, r.y, r.z, r.angle, r.conj);
+        oneByOne();
         return;
     }
     cudaStream_t st = stream();

@@ -1,5 +1,5 @@
 """applyTrotterCircuit at its edges: orders with millions of rotations, angles
-that are not finite, single rotations."""
+that are not finite or of many turns, single rotations."""
 import math
 import resource
 
@@ -42,3 +42,40 @@ def test_high_orders_in_bounded_memory(gpulib):
     e, v = np.linalg.eigh(H)
     want = v @ (np.exp(-0.1j * e) * (v.T @ psi))
     assert np.linalg.norm(got - want) <= 6 * 2.0 ** -53 * 4 * 5 ** 8
+
+
+@pytest.mark.parametrize("n", [2, 6, 9, 13])
+@pytest.mark.parametrize("time,weight", [(math.inf, 0.5), (math.nan, 0.5), (0.1, math.inf), (0.1, math.nan), (0.1, 1e200)])
+def test_angles_that_are_not_finite_show(gpulib, n, time, weight):
+    """Every amplitude that such a rotation acts on becomes NaN, zeros too."""
+    z = np.zeros(1 << n, complex)
+    z[0] = 1.0
+    for codes in ([[3] + [0] * (n - 1), [0, 3] + [0] * (n - 2)], [[1] + [0] * (n - 1), [3, 1] + [0] * (n - 2)]):
+        got = apply(gpulib, n, codes, [weight, 0.25], z, time, 1, 1)
+        if math.isfinite(time * weight):
+            assert np.isfinite(got).all() and abs(np.vdot(got, got) - 1) < 1e-12
+        else:
+            assert np.isnan(got.real).all() and np.isnan(got.imag).all()
+
+
+@pytest.mark.parametrize("n", [4, 9, 13])
+@pytest.mark.parametrize("scale", [50.0, 1e3, 1e7, 1e9, 1e15, 1e200])
+def test_angles_of_many_turns(gpulib, n, scale):
+    """Rotations of many turns next to ordinary ones that merge with them."""
+    r = np.random.default_rng(n)
+    codes, coeffs = [], []
+    for _ in range(4):
+        x = [int(v) for v in r.choice((0, 0, 1, 2), n)]
+        for w in (scale * r.uniform(0.5, 1), 0.3, -0.2 * scale):
+            codes.append([v if v else int(r.choice((0, 3))) for v in x])
+            coeffs.append(w)
+        for w in (scale * r.uniform(0.5, 1), 0.3):
+            codes.append([int(v) for v in r.choice((0, 3), n)])
+            coeffs.append(w)
+    psi = r.standard_normal(1 << n) + 1j * r.standard_normal(1 << n)
+    psi /= np.linalg.norm(psi)
+    got = apply(gpulib, n, codes, coeffs, psi, 1.0, 1, 1)
+    want = psi
+    for t, phi in rotations(coeffs, 1.0, 1, 1):
+        want = rotate(want, codes[t], phi)                  # by the cosine and sine of the whole angle
+    assert np.linalg.norm(got - want) <= 2 * 6 * 2.0 ** -53 * len(codes) * 2
