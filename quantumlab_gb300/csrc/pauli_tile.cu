@@ -252,7 +252,9 @@ Turn turnOf(double angle) {
     const long double lc = c, ls = s;
     Turn t;
     t.phi.hi = std::fabs(a) > 64 ? std::atan2(s, c) : a;
-    t.phi.lo = (double)(ls * std::cos((long double)t.phi.hi) - lc * std::sin((long double)t.phi.hi));
+    long double sh, ch;
+    ::sincosl(t.phi.hi, &sh, &ch);
+    t.phi.lo = (double)(ls * ch - lc * sh);
     t.grow = (double)((lc * lc + ls * ls - 1) / 2);
     return t;
 }
@@ -427,6 +429,7 @@ std::vector<PassPlan> cut(const std::vector<Step>& steps, const std::vector<Wind
     return out;
 }
 
+double aloneUs(const Step& s, int n) { return s.count * (3 + std::ldexp(1.0, n) * 8 / (numSMs() * 1.65 * 1900)); }
 // Expected microseconds: a launch, the state's traffic, and per SM the FP64
 // operations of its tiles (1.65 a clock at 1.9 GHz, as measured), a step not
 // under its latency.  Small registers take smaller tiles, so that every SM
@@ -437,13 +440,14 @@ double cost(const std::vector<PassPlan>& plan, const std::vector<Step>& steps, c
     double us = 0;
     for (const PassPlan& p : plan) {
         if (p.alone) {
-            for (int i : p.steps) us += steps[i].count * (3 + amps * 8 / (sms * 1.65 * 1900));
+            for (int i : p.steps) us += aloneUs(steps[i], n);
             continue;
         }
         us += 3 + (p.windows ? 3 : 0) + amps * 32 / 5e6;
         for (int i : p.steps) {
             const Step& s = steps[i];
-            const double ops = s.x ? (s.hasD ? 1.5 : 3) : 3.0 * win[i].alone.size() + 4.0 * win[i].bits.size();
+            const bool half = s.hasD && (s.even.hi == 0 || s.odd.hi == 0);       // only one parity turns
+            const double ops = s.x ? (half ? 1.5 : 3) : 3.0 * win[i].alone.size() + 4.0 * win[i].bits.size();
             us += std::max(0.35, ops * perAmp) * rounds;
         }
     }
@@ -460,26 +464,33 @@ void gatePauliSequence(SV s, const std::vector<PauliRotation>& seq, double* tabl
     // angles that are not finite: the passes leave zeros as they are, where a
     // rotation by NaN makes them NaN
     if (!std::all_of(seq.begin(), seq.end(), [](const PauliRotation& r) { return std::isfinite(r.angle); })) return oneByOne();
+    // one rotation of a small register is not worth a plan (8 qubits 12.3 us, as
+    // tiles 14.1; 16 qubits 13.8 and 14.8; 20 qubits 29.3 and 22.3)
+    if (seq.size() == 1 && s.n < 18) return oneByOne();
     std::vector<Step> steps;
     merge(seq, steps);
     std::vector<Windows> win(steps.size());
     for (size_t i = 0; i < steps.size(); ++i)
         if (!steps[i].x) win[i] = windowsOf(steps[i]);
+    // without tiles, if they come to more
     int b = 0;
     std::vector<PassPlan> plan;
     double best = 0;
+    for (const Step& a : steps) best += aloneUs(a, s.n);
+    const int low = std::min(kLow, s.n);
     for (int c = std::min(s.n, 7); c <= std::min(s.n, kMaxTileBits); ++c) {
+        // (no pass without a step that fits it)
+        if (std::none_of(steps.begin(), steps.end(), [&](const Step& a) { return !a.x || __builtin_popcountll(a.x >> low) <= c - low; }))
+            continue;
         std::vector<PassPlan> p = cut(steps, win, s.n, c);
         const double us = cost(p, steps, win, s.n, c);
-        if (b && us >= best) continue;
+        if (us >= best) continue;
         b = c;
         best = us;
         plan.swap(p);
     }
-    if (b < kLow + 1) {                            // registers of one to three qubits
-        oneByOne();
-        return;
-    }
+    // registers of one to three qubits, strings that fit no tile
+    if (b < kLow + 1 || std::all_of(plan.begin(), plan.end(), [](const PassPlan& p) { return p.alone; })) return oneByOne();
     cudaStream_t st = stream();
     const size_t smem = tileShared(b);
     if (QG_CUDA(allowShared<kPauliTile>(tileShared(kMaxTileBits)), caller)) return;

@@ -79,3 +79,26 @@ def test_angles_of_many_turns(gpulib, n, scale):
     for t, phi in rotations(coeffs, 1.0, 1, 1):
         want = rotate(want, codes[t], phi)                  # by the cosine and sine of the whole angle
     assert np.linalg.norm(got - want) <= 2 * 6 * 2.0 ** -53 * len(codes) * 2
+
+
+@pytest.mark.parametrize("n", [1, 2, 4, 9, 12, 13])
+def test_single_and_wide_rotations(gpulib, n):
+    """One rotation, and strings with more X/Y qubits than a tile: the same
+    kernels as multiRotatePauli, so the same bits."""
+    L = gpulib
+    r = np.random.default_rng(n)
+    psi = r.standard_normal(1 << n) + 1j * r.standard_normal(1 << n)
+    psi /= np.linalg.norm(psi)
+    wide = [[int(v) for v in r.integers(1, 3, n)] for _ in range(3)]
+    for codes, coeffs in (([wide[0]], [0.7]), ([[3] * n], [0.7]), (wide, [0.3, -1.1, 0.6])):
+        got = apply(L, n, codes, coeffs, psi, 0.4, 1, 1)
+        want = psi
+        for t, phi in rotations(coeffs, 0.4, 1, 1):
+            want = rotate(want, codes[t], phi)
+        assert np.linalg.norm(got - want) <= 12 * 2.0 ** -53 * len(codes) * 2
+        if len(codes) == 1:
+            q = L.create(n)
+            L.set_amps(q, psi)
+            L.multiRotatePauli(q, list(range(n)), codes[0], 2 * 0.4 * coeffs[0])
+            assert np.array_equal(got, L.amps(q))
+            L.destroy(q)
