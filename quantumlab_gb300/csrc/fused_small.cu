@@ -28,6 +28,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 namespace qg {
@@ -315,25 +316,28 @@ static Seg segOf(const FusedPass& pass, int n, int groups, size_t mat) {
     return s;
 }
 
-// the pass's matrix as the kernel reads it
+// the pass's matrix as the kernel reads it, into zeros
 static void smallMatrix(const FusedPass& pass, int n, float* out) {
     const std::vector<int> t = widened(pass.targets, n);
     const int Dk = 1 << pass.targets.size();
-    int old[kD], rest[kD];                    // a 6-qubit index's bits on the pass's own qubits, and the others
+    // 6-qubit indices by their bits on the other qubits and on the pass's own
+    int at[kD];
     for (int i = 0; i < kD; ++i) {
-        old[i] = rest[i] = 0;
-        for (int b = 0, ob = 0; b < 6; ++b) {
-            const bool own = std::find(pass.targets.begin(), pass.targets.end(), t[b]) != pass.targets.end();
-            if (own) old[i] |= (i >> b & 1) << ob++;
-            else rest[i] |= (i >> b & 1) << b;
+        int own = 0, rest = 0;
+        for (int b = 0, ob = 0, rb = 0; b < 6; ++b) {
+            if (std::binary_search(pass.targets.begin(), pass.targets.end(), t[b])) own |= (i >> b & 1) << ob++;
+            else rest |= (i >> b & 1) << rb++;
         }
+        at[rest * Dk + own] = i;
     }
-    for (int j = 0; j < kD; ++j)
-        for (int r = 0; r < kD; ++r) {
-            const cplx v = rest[r] == rest[j] ? pass.m[(size_t)old[r] * Dk + old[j]] : cplx(0, 0);
-            out[j * kD + r] = (float)v.real();
-            out[kD * kD + j * kD + r] = (float)v.imag();
-        }
+    for (int e = 0; e < kD; e += Dk)
+        for (int r = 0; r < Dk; ++r)
+            for (int j = 0; j < Dk; ++j) {
+                const cplx v = pass.m[(size_t)r * Dk + j];
+                float* o = out + at[e + j] * kD + at[e + r];
+                o[0] = (float)v.real();
+                o[kD * kD] = (float)v.imag();
+            }
 }
 
 // ------------------------------------------------------------ a plan on one register
@@ -381,7 +385,54 @@ int groupsFor(uint64_t amps) {
 }
 }  // namespace
 
+// Page-locked error words, given out by the page: a page-locked allocation and
+// its release for each plan took 150 us of a small plan's first application
+// (10 qubits, one layer: 296 us with the plan on passes of their own).  The
+// first page is kept for the process; when it is full, plans allocate a word of
+// their own.
+namespace {
+class ErrorWords {
+public:
+    int* take(const char* caller) {
+        std::lock_guard<std::mutex> lk(mutex_);
+        if (!page_) {
+            if (QG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&page_), kWords * sizeof(int), cudaHostAllocMapped), caller)) {
+                page_ = nullptr;
+                return nullptr;
+            }
+            for (int i = kWords; i-- > 0;) free_.push_back(i);
+        }
+        int* word = nullptr;
+        if (!free_.empty()) {
+            word = page_ + free_.back();
+            free_.pop_back();
+        } else if (QG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&word), sizeof(int), cudaHostAllocMapped), caller)) {
+            return nullptr;
+        }
+        *word = 0;
+        return word;
+    }
+    void give(int* word) {
+        std::lock_guard<std::mutex> lk(mutex_);
+        if (page_ && word >= page_ && word < page_ + kWords) free_.push_back((int)(word - page_));
+        else cudaFreeHost(word);
+    }
+
+private:
+    static constexpr int kWords = 1024;
+    std::mutex mutex_;
+    int* page_ = nullptr;
+    std::vector<int> free_;
+};
+ErrorWords& errorWords() {
+    static ErrorWords* words = new ErrorWords();     // (outlives every plan)
+    return *words;
+}
+}  // namespace
+
 bool smallPlanFits(const FusedPlan& plan) {
+    // a flush of one pass is not worth an upload (19 qubits 82 us, so 91)
+    if (plan.deferProducts && plan.passes.size() == 1) return false;
     if (plan.numQubits < 10 || plan.numQubits > kSmallMaxQubits || plan.passes.empty() || !tcDefaultAppliers()) return false;
     for (const FusedPass& pass : plan.passes)
         if (!pass.controls.empty() || pass.targets.empty() || pass.targets.size() > 6) return false;
@@ -424,7 +475,7 @@ void* smallPlanUpload(const FusedPlan& plan, void* reuse) {
     for (size_t i = 0; i < plan.passes.size(); ++i)
         if (!plan.passes[i].m.empty()) smallMatrix(plan.passes[i], n, reinterpret_cast<float*>(host) + i * 2 * kD * kD);
     memcpy(host + matHost, segs.data(), segs.size() * sizeof(Seg));
-    if (!pp->errFlag && QG_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&pp->errFlag), sizeof(int), cudaHostAllocMapped), caller)) {
+    if (!pp->errFlag && !(pp->errFlag = errorWords().take(caller))) {
         smallPlanFree(pp);
         return nullptr;
     }
@@ -457,7 +508,7 @@ void smallPlanFree(void* h) {
     pp->source.release();
     if (pp->buffer) cudaFree(pp->buffer);
     freeBuildScratch(pp->scratch);
-    if (pp->errFlag) cudaFreeHost(pp->errFlag);
+    if (pp->errFlag) errorWords().give(pp->errFlag);
     delete pp;
 }
 
