@@ -150,12 +150,16 @@ void quest_gb300_copyToQureg(void* qureg32, Qureg destination);
 int quest_gb300_applyPlanF32(void* qureg32, void* plan);
 /* Norm record of pass i of the plan's last application, if it ran on the
  * tensor cores: {sum |x|^2 in, sum |y|^2 out, square of the drift-correction
- * scale it applied}.  Returns 1, or 0 if there is no record. */
+ * scale it applied}.  Returns 1, or 0 if there is no record (a pass on FP32
+ * units has none: its sums are rounded to nearest and do not drift). */
 int quest_gb300_planPassNorms(void* plan, int i, double* inOutScaleSq);
 /* apply passes [firstPass, firstPass + numPasses) only (timing, stepping) */
 int quest_gb300_applyPlanF32Range(void* qureg32, void* plan, int firstPass, int numPasses);
-/* applier of pass i: 0 = SIMT, 1 = direct-load tensor-core kernel, 2..5 =
- * pipelined tensor-core kernel (as setTensorCoreKernel); -1 if invalid */
+/* applier of pass i: 0 = FP32 units, 1 = direct-load tensor-core kernel, 2..5 =
+ * pipelined tensor-core kernel (as setTensorCoreKernel); -1 if invalid.  Plans
+ * on 10 to 19 qubits without control qubits run in one launch on FP32 units
+ * when the appliers are the library's choice (setTensorCores 1,
+ * setTensorCoreKernel 0, no split-FP16, no per-pass timing). */
 int quest_gb300_planPassUsesTensorCores(void* plan, int i);
 /* passes on 4..6 qubits run on the tensor cores (split-TF32) unless disabled
  * here (1 = enabled, the default; 0 = FP32 SIMT applier for k <= 5) */

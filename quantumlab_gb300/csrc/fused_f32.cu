@@ -613,10 +613,12 @@ int quest_gb300_planPassNorms(void* plan, int i, double* inOutScaleSq) {
     return qg::tcPassNorms(p->device, (size_t)i, inOutScaleSq);
 }
 
-/* applier of pass i of the plan for registers of its size (tcKernelFor) */
+/* applier of pass i of the plan for registers of its size: none of its own where
+   the plan runs in one launch, else tcKernelFor */
 int quest_gb300_planPassUsesTensorCores(void* plan, int i) {
     qg::FusedPlan* p = reinterpret_cast<qg::FusedPlan*>(plan);
     if (!p || !p->compiled || i < 0 || i >= (int)p->passes.size()) return -1;
+    if (!g_passEvents && qg::smallPlanFits(*p)) return 0;
     return qg::tcKernelFor(p->passes[i], p->numQubits);
 }
 
