@@ -107,6 +107,9 @@ __device__ __forceinline__ void rotate(double& x, double& y, double t, double s,
     x = flip(fma(-t, y1, x1), neg);
     y = flip(y1, neg);
 }
+// The lanes of a warp that take part in a loop of the block's threads over
+// `count`, a power of two: all of its warps, or the first lanes of one.
+__device__ __forceinline__ uint32_t voters(uint32_t count) { return count >= 32 ? 0xffffffffu : (1u << count) - 1u; }
 __device__ __forceinline__ uint32_t insert0(uint32_t k, int b) { return ((k >> b) << (b + 1)) | (k & ((1u << b) - 1u)); }
 
 __global__ void __launch_bounds__(kThreads) kPauliTile(double* re, double* im,
@@ -114,7 +117,7 @@ __global__ void __launch_bounds__(kThreads) kPauliTile(double* re, double* im,
                                                        const double2* tables) {
     extern __shared__ double2 sm[];
     const int b = p.b;
-    const uint32_t size = 1u << b;
+    const uint32_t size = 1u << b, sizeVoters = voters(size);
     double* sr = reinterpret_cast<double*>(sm);
     double* si = sr + size;
     uint64_t* high = reinterpret_cast<uint64_t*>(si + size);           // qubits of tile index bits >= kLow
@@ -138,7 +141,7 @@ __global__ void __launch_bounds__(kThreads) kPauliTile(double* re, double* im,
         if (op.kind == kTablePhase) {
             for (uint32_t l = threadIdx.x; l < size; l += kThreads) {
                 const double x = sr[l], y = si[l];
-                if (!__any_sync(__activemask(), (bits(x) | bits(y)) != 0)) continue;
+                if (!__any_sync(sizeVoters, (bits(x) | bits(y)) != 0)) continue;
                 double fr = 1.0, fi = 0.0;
                 for (int w = op.w0; w < op.w1; ++w) {
                     const Window& win = p.win[w];
@@ -167,7 +170,7 @@ __global__ void __launch_bounds__(kThreads) kPauliTile(double* re, double* im,
             for (uint32_t l = threadIdx.x; l < size; l += kThreads) {
                 const uint32_t sgn = ((__popc(l & op.ml) & 1) ^ outM) << 31;
                 double x = sr[l], y = si[l];
-                if (!__any_sync(__activemask(), (bits(x) | bits(y)) != 0)) continue;
+                if (!__any_sync(sizeVoters, (bits(x) | bits(y)) != 0)) continue;
                 rotate(y, x, flip(op.t[0], sgn), flip(op.s[0], sgn), op.neg[0] ? 0x80000000u : 0u);
                 sr[l] = x;
                 si[l] = y;
@@ -179,7 +182,7 @@ __global__ void __launch_bounds__(kThreads) kPauliTile(double* re, double* im,
         const int one = op.act[0] && op.act[1] ? -1 : op.act[0] ? 0 : 1;
         if (op.dl == 0 && one >= 0 && (int)outD != one) continue;
         const int fix = op.fix;
-        const uint32_t pairs = fix >= 0 ? size / 4 : size / 2;
+        const uint32_t pairs = fix >= 0 ? size / 4 : size / 2, pairVoters = voters(pairs);
         for (uint32_t t = threadIdx.x; t < pairs; t += kThreads) {
             uint32_t j;
             if (fix >= 0) {
@@ -196,7 +199,7 @@ __global__ void __launch_bounds__(kThreads) kPauliTile(double* re, double* im,
             double jr = sr[j], ji = si[j], kr = sr[k], ki = si[k];
             // zeros stay zeros: a warp whose pairs hold nothing (particle-number
             // sectors leave most of a register zero) spends no FP64 on them
-            if (!__any_sync(__activemask(), (bits(jr) | bits(ji) | bits(kr) | bits(ki)) != 0)) continue;
+            if (!__any_sync(pairVoters, (bits(jr) | bits(ji) | bits(kr) | bits(ki)) != 0)) continue;
             if (op.kind == kCross) {
                 rotate(jr, ki, tt, ss, neg);
                 rotate(kr, ji, tt, ss, neg);
