@@ -38,12 +38,6 @@ __device__ __forceinline__ int2 absDigits(double x, int E) {
     t = (t + 1) >> 1;
     return make_int2((int)(t >> 27), (int)((uint32_t)t & 0x7FFFFFFu));
 }
-// the same with x's sign
-__device__ __forceinline__ int2 digits(double x, int E) {
-    const int s = (__double2hiint(x) >> 31) | 1;
-    const int2 d = absDigits(x, E);
-    return make_int2(d.x * s, d.y * s);
-}
 // x 2^(1082 - E) rounded to an integer below 2^60 in magnitude, as h 2^30 + l
 __device__ __forceinline__ int2 wideDigits(double x, int E) {
     const uint32_t hi = (uint32_t)__double2hiint(x);
@@ -56,17 +50,13 @@ __device__ __forceinline__ int2 wideDigits(double x, int E) {
 }
 __device__ __forceinline__ int64_t mad(int a, int b, int64_t c) { return c + (int64_t)a * b; }
 
-struct Sums {                                    // h h, h l + l h, l l; at most 2^8 products
+struct Sums {                                    // h h, h l + l h, l l
     int64_t hh, x, ll;
     __device__ __forceinline__ void add(int2 a, int2 b) {
         hh = mad(a.x, b.x, hh);
         x = mad(a.x, b.y, x);
         x = mad(a.y, b.x, x);
         ll = mad(a.y, b.y, ll);
-    }
-    // acc + c times the sum, in units of 2^54
-    __device__ __forceinline__ double into(double acc, double c) const {
-        return fma(c, (double)hh, fma(c * 0x1p-27, (double)(x + ((ll + (1 << 26)) >> 27)), acc));
     }
     // the sum of at most 16 products, rounded to units of 2^49
     __device__ __forceinline__ double few() const { return (double)((hh << 5) + ((x + (ll >> 27) + (1 << 21)) >> 22)); }
