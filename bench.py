@@ -378,21 +378,24 @@ def run_gpu(args, rank, world):
                     "one_minus_fidelity_vs_fp64": 1 - (ip.real ** 2 + ip.imag ** 2) / (n64 * ndf),
                     "total_prob": ndf, "total_prob_err_vs_fp64": abs(ndf - n64),
                     "mode": "quest_gb300_setPlainArithmetic(1): general 2x2 gates in double-float on the FP32 pipes"}
-        # one compactUnitary on qubit 10 of the 30-qubit state (no controls):
-        # 32 B per amplitude (read + write of the FP64 complex state)
+        # one gate on qubit 10 of the 30-qubit state (no controls): 32 B per
+        # amplitude (read + write of the FP64 complex state).  A general
+        # compactUnitary (all four real parts nonzero), a real one (rotateY),
+        # and the general one in double-float
         from quantumlab_gb300.quest import Complex
         gate_roof = {}
-        a_, b_ = Complex(0.6, 0.0), Complex(0.0, 0.8)
-        for mode, name in ((0, "fp64"), (1, "double_float")):
+        general = (lib.compactUnitary, Complex(0.5, 0.5), Complex(0.5, 0.5))
+        for mode, name, kernel, gate in ((0, "fp64", "OpFixed4", general), (0, "fp64_real_matrix", "OpFixed2", (lib.rotateY, 1.1)),
+                                         (1, "double_float", "OpMatrix2DF", general)):
             lib.quest_gb300_setPlainArithmetic(mode)
-            lib.compactUnitary(qdf, 10, a_, b_)
+            gate[0](qdf, 10, *gate[1:])
             lib.quest_gb300_eventRecord(12)
             for _ in range(8):
-                lib.compactUnitary(qdf, 10, a_, b_)
+                gate[0](qdf, 10, *gate[1:])
             lib.quest_gb300_eventRecord(13)
             gms = lib.quest_gb300_eventElapsedMs(12, 13) / 8
-            gate_roof[name] = {"kernel": "kPairVec<" + ("OpCompact" if mode == 0 else "OpMatrix2DF") + ">",
-                               "avg_launch_ms": round(gms, 4), "achieved_gbs": round((1 << n) * 32 / gms / 1e6, 1)}
+            gate_roof[name] = {"kernel": "kPairVec<" + kernel + ">", "avg_launch_ms": round(gms, 4),
+                               "achieved_gbs": round((1 << n) * 32 / gms / 1e6, 1)}
         lib.quest_gb300_setPlainArithmetic(0)
         L.destroy(qdf)
 

@@ -25,7 +25,7 @@
 // quarter (half) of the result's last place.  |c| <= 1 and row sums <= 2, as
 // the orthogonal maps of unitary gates have them, keep the sums in 64 bits.
 // Inputs whose largest exponent leaves no room for the result's exponent
-// (|x| < 2^-959 or > 2^1021, infinities, NaNs) are told by `apply`; they take
+// (|x| < 2^-959 or >= 2^958, infinities, NaNs) are told by `apply`; they take
 // FP64 arithmetic instead.
 //
 // The functions compile for the device and, for the CPU unit test, for the

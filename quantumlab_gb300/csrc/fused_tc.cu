@@ -38,7 +38,9 @@
 //
 // Every wait is bounded: on timeout the CTA records an error code in a
 // device flag, skips the rest of its tiles, frees its TMEM and returns; the
-// host reads the flag after the pass.
+// host reads the flag after the pass.  The one wait without a limit is the
+// barrier of a pair of CTAs (barrier.cluster.wait): every warp of both arrives
+// on it behind bounded waits only, whatever their outcome.
 #include "chain_launch.cuh"
 #include "fused_build.h"
 #include "fused_plan.h"
