@@ -715,10 +715,14 @@ bool compileBatch(TrotterBatch* b) {
 // The run's work: class after class, its states' initialisation, its passes
 // (one launch each over the class's states) and its reductions, then one copy
 // of every result to pinned host memory.  Queued on `st`; while `st` is being
-// captured into a graph each class goes to a branch of its own, so that the
-// classes run side by side (a pass over three 16-qubit states is 24 CTAs):
-// nine instances of 10, 20 and 100 steps 3.80 ms one class after the other,
-// 1.61 ms so, with the same bits.
+// captured into a graph the classes are dealt to branches, so that they run
+// side by side (a pass over three 16-qubit states is 24 CTAs): nine instances
+// of 10, 20 and 100 steps 3.80 ms one class after the other, 1.61 ms so, with
+// the same bits.  More classes gain more (one instance each, 16 qubits: 2
+// classes 0.19 -> 0.12 ms, 17 3.31 -> 0.65, 48 20.1 -> 3.2), also where a state
+// fills the chip (20 qubits, 17 classes 7.4 -> 6.8); a branch is a stream while
+// the graph is made, so their number has a limit.
+constexpr size_t kMaxBranches = 64;
 struct Branches {                    // (alive until the capture has ended)
     cudaEvent_t start = nullptr;
     std::vector<cudaStream_t> st;
@@ -746,12 +750,13 @@ struct Branches {                    // (alive until the capture has ended)
 bool queueRun(TrotterBatch* b, cudaStream_t st, Branches* branches) {
     if (QG_CUDA(cudaMemsetAsync(b->errFlag, 0, sizeof(int), st), kFn)) return false;
     const size_t C = b->classes.size();
-    const bool fork = branches && C > 1 && C <= 16;
-    if (fork && !branches->open(C, st)) return false;
+    const bool fork = branches && C > 1;
+    const size_t B = std::min(C, kMaxBranches);
+    if (fork && !branches->open(B, st)) return false;
     const cudaStream_t whole = st;
     for (size_t c = 0; c < b->classes.size(); ++c) {
         const TrotterClass& cl = b->classes[c];
-        const cudaStream_t st = fork ? branches->st[c] : whole;
+        const cudaStream_t st = fork ? branches->st[c % B] : whole;
         const int M = (int)cl.members.size();
         const uint64_t dim = 1ull << cl.n, all = dim * (uint64_t)M;
         float* re = b->re + cl.stateOffset;
@@ -771,7 +776,11 @@ bool queueRun(TrotterBatch* b, cudaStream_t st, Branches* branches) {
         unsigned int* counters = b->counters + cl.posBase;
         const int R = (int)cl.reds.size();
         bool reduced = false;
-        if (all <= 1ull << 20 && R <= 64) {
+        // In one launch while the class's states are small: two states of 20
+        // qubits 0.42 ms a reduction a launch, 0.31 so, 32 of 16 qubits 0.33 and
+        // 0.34; twice as many 0.56 and 0.53, but 0.50 and 0.64.  R: at least 32
+        // blocks for each reduction of an instance.
+        if (all <= 1ull << 21 && R <= 64) {
             // enough blocks for the widest reduction; an instance's partials hold R x bx
             const unsigned bx = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(kMaxBlocksPerInst / R, dim / 2 / (4 * red::kThreads)));
             kReduceAll<<<dim3(bx, (unsigned)M, (unsigned)R), red::kThreads, 0, st>>>(
@@ -803,9 +812,9 @@ bool queueRun(TrotterBatch* b, cudaStream_t st, Branches* branches) {
             if (launchFailed(kFn)) return false;
         }
     }
-    for (size_t c = 0; fork && c < C; ++c)
-        if (QG_CUDA(cudaEventRecord(branches->done[c], branches->st[c]), kFn) ||
-            QG_CUDA(cudaStreamWaitEvent(whole, branches->done[c], 0), kFn))
+    for (size_t k = 0; fork && k < B; ++k)
+        if (QG_CUDA(cudaEventRecord(branches->done[k], branches->st[k]), kFn) ||
+            QG_CUDA(cudaStreamWaitEvent(whole, branches->done[k], 0), kFn))
             return false;
     return !QG_CUDA(cudaMemcpyAsync(b->hResults, b->dResults, 2 * (size_t)b->numSlots * sizeof(double),
                                     cudaMemcpyDeviceToHost, st), kFn);
