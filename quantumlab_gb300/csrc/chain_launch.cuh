@@ -83,6 +83,7 @@ inline void launchChained(unsigned cluster, void (*kernel)(Params...), dim3 grid
 template <auto kernel, class... Args>
 inline void chain(dim3 grid, dim3 block, cudaStream_t st, Args&&... args) {
     const bool allowed = allowShared<kernel>(kEvenShareBytes) == cudaSuccess;
+    if (!allowed) (void)cudaGetLastError();          // it runs without the share
     launchChained(1, kernel, grid, block, allowed ? evenShare(grid.x * grid.y) : 0, st, std::forward<Args>(args)...);
 }
 // One with `smem` bytes, which allowShared has been asked for.

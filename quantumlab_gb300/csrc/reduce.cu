@@ -15,6 +15,7 @@
 #include "reduce_kernel.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace qg {
 namespace {
@@ -375,14 +376,18 @@ double reduceExpecPauliGroups(SV s, int isDM, int N, const std::vector<PauliTerm
     constexpr int kSlots = 32;                   // the scratch holds 64 result doubles
     const char* caller = "calcExpecPauliSum";
     cudaStream_t st = stream();
-    double total = 0.0;
+    double total = 0.0, low = 0.0;
     int used = 0;
     auto drain = [&]() -> bool {
         if (!used) return true;
         if (QG_CUDA(cudaMemcpyAsync(w.host, w.result, 2 * used * sizeof(double), cudaMemcpyDeviceToHost, st), caller) ||
             QG_CUDA(cudaStreamSynchronize(st), caller))
             return false;
-        for (int k = 0; k < used; ++k) total += w.host[2 * k];
+        for (int k = 0; k < used; ++k) {         // (TwoSum)
+            const double x = w.host[2 * k], s = total + x, z = s - total;
+            low += (total - (s - z)) + (x - z);
+            total = s;
+        }
         used = 0;
         return true;
     };
@@ -436,7 +441,7 @@ double reduceExpecPauliGroups(SV s, int isDM, int N, const std::vector<PauliTerm
         }
     }
     drain();
-    return total;
+    return std::isfinite(total) ? total + low : total;
 }
 
 void reduceProbAllOutcomes(SV s, int isDM, int N, const int* qubits, int nq, double* hostOut, const Scratch& w) {
