@@ -97,17 +97,19 @@ int quest_gb300_passTimesMs(double* out, int maxPasses);
 
 /* ---- arithmetic of the plain path ------------------------------------------
  * No counterpart in the reference.  GB300 runs FP64 fused multiply-adds at
- * about 1/70 of its FP32 rate, so the plain path's general 2 x 2 gates
- * (compactUnitary and the rotations, unitary and its controlled forms,
- * hadamard) are bound by the FP64 pipe, not by HBM.  Mode 1 computes them in
+ * about 1/70 of its FP32 rate.  Mode 0, the default, computes the plain path's
+ * general 2 x 2 gates (compactUnitary and the rotations, unitary and its
+ * controlled forms, hadamard) to FP64's precision, in fixed point on the integer
+ * pipes and in FP64 (all in FP64 for a matrix with a small coefficient).  Mode 1
+ * computes them in
  * double-float arithmetic on the FP32 and integer pipes: each double is split
  * into two floats by integer field operations (2^-47 relative), products are
  * exact through FMA, sums compensated (TwoSum), and the result is packed back
  * into the double's fields; the state stays FP64 in memory.  A gate's result
  * is then within a few 2^-47 of FP64, relative to its largest term.  Doubles
  * below 2^-126 in magnitude are flushed to 0 and those of 2^128 and above
- * are not representable.  Mode 0, exact FP64, is the default.  Returns 0, or
- * -1 for an unknown mode. */
+ * are not representable.  On the 30-qubit random circuit mode 1 takes 5.1 s
+ * and mode 0 5.7.  Returns 0, or -1 for an unknown mode. */
 int quest_gb300_setPlainArithmetic(int mode);
 int quest_gb300_getPlainArithmetic(void);
 

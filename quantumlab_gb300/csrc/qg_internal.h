@@ -114,7 +114,7 @@ void gatePauliRotation(SV s, uint64_t ctrl, uint64_t xmask, uint64_t ymask, uint
 struct PauliRotation { uint64_t x, y, z; double angle; int conj; };
 void gatePauliSequence(SV s, const std::vector<PauliRotation>& seq, double* tables);
 void gateSwap(SV s, int q1, int q2);
-// plain-path arithmetic of the general 2 x 2 gates: 0 FP64, 1 double-float
+// plain-path arithmetic of the general 2 x 2 gates: 0 FP64's precision, 1 double-float
 bool setPlainArithmetic(int mode);
 int plainArithmetic();
 // Dense 2^k x 2^k (k <= 6) on targets (targs[0] = least significant matrix bit).

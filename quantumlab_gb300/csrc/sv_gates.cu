@@ -152,7 +152,7 @@ OpMatrix2DF matrix2DF(const Mat2& m) {
         for (int j = 0; j < 4; ++j) op.coef[o][j] = df::splitConst(k[o][j]);
     return op;
 }
-// 0: exact FP64 (the default); 1: double-float for the general 2 x 2 gates
+// 0: FP64 and fixed point at its precision (the default); 1: double-float for the general 2 x 2 gates
 int g_plainArith = 0;
 
 struct OpSwap {
@@ -655,7 +655,7 @@ void gateMatrixN(SV s, uint64_t ctrl, const int* targs, int k, const double* mr,
 extern "C" {
 /* Arithmetic of the plain path's general 2 x 2 gates (compactUnitary and the
  * rotations built on it, unitary and its controlled forms, hadamard): 0 =
- * exact FP64 (the default), 1 = double-float on the FP32 and integer pipes
+ * FP64's precision (the default), 1 = double-float on the FP32 and integer pipes
  * (df64.cuh).  Returns 0, or -1 for an unknown mode. */
 int quest_gb300_setPlainArithmetic(int mode) { return qg::setPlainArithmetic(mode) ? 0 : -1; }
 int quest_gb300_getPlainArithmetic(void) { return qg::plainArithmetic(); }
